@@ -472,7 +472,11 @@ ns2d_status record(ns2d_handle* h, int nsteps, double dt, int every) {
         if (k % every == 0)
             ACK(h, cudaMemcpyAsync((char*)a->ckpt + (size_t)(k / every) * h->field_bytes, h->state, h->field_bytes,
                                    cudaMemcpyDeviceToDevice, h->stream));
-        if ((s = internal::rk4_step_loop(h, dt))) return s;
+        // the reverse sweep recomputes these steps bit for bit with the pass kernels
+        h->use_passes = true;
+        s = internal::rk4_step_loop(h, dt);
+        h->use_passes = false;
+        if (s) return s;
     }
     ACK(h, cudaEventRecord(a->t[1], h->stream));
     if ((s = internal::check_status(h))) return s;

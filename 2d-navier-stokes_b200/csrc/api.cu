@@ -17,6 +17,7 @@
 #include "engine.cuh"
 #include "handle.h"
 #include "host_common.h"
+#include "resident.h"
 
 using namespace ns2d;
 
@@ -44,6 +45,8 @@ ns2d_status fail(ns2d_handle* h, ns2d_status s, const std::string& msg) {
         cudaError_t e_ = cudaGetLastError();                                                          \
         if (e_ != cudaSuccess) return fail((h), NS2D_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e_)); \
     } while (0)
+
+#define DISPATCH(h, fn, ...) ((h)->fp32 ? fn<float>(__VA_ARGS__) : fn<double>(__VA_ARGS__))
 
 // Branch of the linear operator for this evaluation (see host_common.h).
 int resolve_branch(ns2d_handle* h, bool latch) { return ns2d::resolve_branch(h->hyper_flag, h->p.ekmn_drag_flag, latch); }
@@ -210,6 +213,58 @@ void launch_row(ns2d_handle* h, int stage = 0) {
     with_size<Real>(h->nx, [&](auto L) { decltype(L)::row(r, h->stream); });
 }
 
+// First ky column the 2/3 rule empties (every kx there has k2 >= kmax_sqr), nyf
+// for the Hou-Li filter, which empties none.
+int kept_columns(const ns2d_handle* h) {
+    if (h->p.dealias != 0) return h->nyf;
+    const int m = (int)(h->nx / 3.0), lim = m * m + h->p.dealias_edge;
+    int kc = 0;
+    while (kc < h->nyf && kc * kc < lim) ++kc;
+    return kc;
+}
+
+// Whether this handle's steps and evaluations run in the resident kernel: a
+// small grid, and neither the adjoint (whose recomputation captures the stage
+// fields of the passes, so its recorded run takes them too), the per-pass timing
+// nor the ZERO forcing's rewrite of the state before each step.
+bool resident_ok(const ns2d_handle* h) {
+    return h->resident && !h->use_passes && !h->timing && !h->cap_step && h->p.forcing != NS2D_FORCING_ZERO;
+}
+
+template <typename Real>
+void fill_resident(ns2d_handle* h, ResArgs<Real>& r, int branch) {
+    ColArgs<Real> a;
+    fill_common<Real>(h, a, branch);
+    std::memset(&r, 0, sizeof(r));
+    r.state = a.state;
+    r.tw = a.tw;
+    r.force_field = a.force_field;
+    r.ldc = a.ldc;
+    r.nyf = a.nyf;
+    r.kmax_sqr = a.kmax_sqr;
+    r.kc = kept_columns(h);
+    r.dealias = a.dealias;
+    r.houli_int = a.houli_int;
+    r.kolm = a.kolm;
+    r.has_force = a.has_force;
+    r.force_i = a.force_i;
+    r.force_j = a.force_j;
+    r.force_val = a.force_val;
+    r.wide = (a.has_force && a.force_j >= r.kc) || a.force_field ? 1 : 0;
+    r.phase_only = a.phase_only;
+    r.norm2 = a.norm2;
+    r.inv_nxny = a.inv_nxny;
+    r.lin = a.lin;
+    r.status = a.status;
+}
+
+template <typename Real>
+ns2d_status launch_resident(ns2d_handle* h, int scheme, const ResArgs<Real>& r) {
+    CK(h, resident_launch<Real>(h->nx, scheme, r, h->stream));
+    h->launches += r.nsteps;  // counted per step (ns2d_launch_count)
+    return NS2D_OK;
+}
+
 // Forcing values for this step (ComputeForcing, Solver/src/force.c:516-581);
 // ZERO forcing kills its modes of the state instead.
 void compute_forcing(ns2d_handle* h, double dt) {
@@ -239,11 +294,15 @@ ns2d_status ensure_cn(ns2d_handle* h, double dt, int branch) {
     return NS2D_OK;
 }
 
+template <typename Real>
+ns2d_status resident_rk4(ns2d_handle* h, int nsteps, double dt, void* rk1_out);
+
 // One RK4 / RK4CN step (RK4Step, Solver/src/solver.c:625-873).  If rk1_out is
 // non-null the stage-1 RHS is stored there (AB4 start-up, solver.c:283).
 template <typename Real>
 ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
     using C = Cplx<Real>;
+    if (resident_ok(h)) return resident_rk4<Real>(h, 1, dt, rk1_out);
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const bool explicit_rk4 = euler || h->p.integrator == NS2D_RK4;
@@ -298,10 +357,72 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
     return NS2D_OK;
 }
 
+// Steps per launch of the resident kernel: the launch and the load and store of
+// the state cost about one step, and a launch stays well under a millisecond or
+// two, so other work on the device gets its turn.
+constexpr int kResidentSteps = 128;
+
+// nsteps RK4 / RK4CN steps of a small grid in the resident kernel; rk1_out as in
+// rk4_step_impl (then nsteps is 1).
+template <typename Real>
+ns2d_status resident_rk4(ns2d_handle* h, int nsteps, double dt, void* rk1_out) {
+    using C = Cplx<Real>;
+    compute_forcing(h, dt);
+    const bool euler = h->p.system == NS2D_EULER;
+    const bool explicit_rk4 = euler || h->p.integrator == NS2D_RK4;
+    const bool rk4_lin = !euler && h->p.integrator == NS2D_RK4;
+    const int branch = euler ? 4 : resolve_branch(h, quirk(h, NS2D_QUIRK_HYPER_LATCH));
+    ResArgs<Real> r;
+    fill_resident<Real>(h, r, branch);
+    r.dt = dt;
+    r.lin_stage = rk4_lin ? (quirk(h, NS2D_QUIRK_RK4_LINEAR) ? 1 : 2) : 0;
+    r.conj_quirk = quirk(h, NS2D_QUIRK_CONJ_STATE) ? 1 : 0;
+    r.rhs = (C*)rk1_out;
+    if (!explicit_rk4) {
+        ns2d_status s = ensure_cn(h, dt, branch);
+        if (s) return s;
+        r.cn = h->cn;
+    }
+    for (int k = 0; k < nsteps; k += r.nsteps) {
+        r.nsteps = std::min(kResidentSteps, nsteps - k);
+        ns2d_status s = launch_resident(h, explicit_rk4 ? RES_EXPLICIT : RES_CN, r);
+        if (s) return s;
+    }
+    return NS2D_OK;
+}
+
+// nsteps AB4 steps past the start-up in the resident kernel.
+template <typename Real>
+ns2d_status resident_ab4(ns2d_handle* h, int nsteps, double dt) {
+    using C = Cplx<Real>;
+    compute_forcing(h, dt);
+    const bool euler = h->p.system == NS2D_EULER;
+    const int branch = euler ? 4 : resolve_branch(h, false);
+    ResArgs<Real> r;
+    fill_resident<Real>(h, r, branch);
+    r.dt = dt;
+    r.euler = euler ? 1 : 0;
+    r.conj_quirk = 1;
+    if (!euler) {
+        ns2d_status s = ensure_cn(h, dt, branch);
+        if (s) return s;
+        r.cn = h->cn;
+    }
+    for (int k = 0; k < nsteps; k += r.nsteps) {
+        r.nsteps = std::min(kResidentSteps, nsteps - k);
+        for (int j = 0; j < 4; ++j) r.h[j] = (C*)h->ab[j];
+        ns2d_status s = launch_resident(h, RES_AB4, r);
+        if (s) return s;
+        std::rotate(h->ab, h->ab + r.nsteps % 4, h->ab + 4);  // the kernel's rotation, one place per step
+    }
+    return NS2D_OK;
+}
+
 // AB4Step past the start-up (Solver/src/solver.c:286-349).
 template <typename Real>
 ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
     using C = Cplx<Real>;
+    if (resident_ok(h)) return resident_ab4<Real>(h, 1, dt);
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
@@ -341,6 +462,15 @@ ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
 template <typename Real>
 ns2d_status rhs_impl(ns2d_handle* h, const void* src, bool src_is_state) {
     using C = Cplx<Real>;
+    if (resident_ok(h)) {
+        ResArgs<Real> r;
+        fill_resident<Real>(h, r, 4);
+        r.src = (const C*)src;
+        r.rhs = (C*)h->rhsbuf;
+        r.nsteps = 1;
+        r.conj_quirk = (quirk(h, NS2D_QUIRK_CONJ_STATE) || src_is_state) ? 1 : 0;
+        return launch_resident(h, RES_RHS, r);
+    }
     ColArgs<Real> a;
     fill_common<Real>(h, a, 4);
     a.src = (const C*)src;
@@ -667,6 +797,7 @@ ns2d_status create_impl(ns2d_handle* h) {
     CK(h, cudaMalloc(&h->dpart, sizeof(double) * 4096));
     CK(h, cudaMalloc(&h->cn, sizeof(double2) * (size_t)h->nx * h->ldc));
     build_col_maps<Real>(h);
+    h->resident = resident_setup(h->nx, h->fp32);
     CK(h, cudaFuncSetAttribute((const void*)diag_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(sizeof(double) * (8 * (size_t)h->n_spect + DG_N * 8))));
     std::vector<C> tw;
@@ -694,8 +825,6 @@ ns2d_status unpack_out(ns2d_handle* h, const void* src, double2* d_dst) {
     CKL(h);
     return NS2D_OK;
 }
-
-#define DISPATCH(h, fn, ...) ((h)->fp32 ? fn<float>(__VA_ARGS__) : fn<double>(__VA_ARGS__))
 
 void drop_graph(ns2d_handle* h) {
     if (h->step_graph) cudaGraphExecDestroy(h->step_graph);
@@ -738,7 +867,7 @@ ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out) {
 // every launch and is read back after each replay.  Stage capture for the
 // adjoint uses the eager form.
 ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
-    if (h->cap_step) return DISPATCH(h, rk4_step_impl, h, dt, nullptr);
+    if (h->cap_step || resident_ok(h)) return DISPATCH(h, rk4_step_impl, h, dt, nullptr);
     int hf = h->hyper_flag;
     const int branch = (h->p.system == NS2D_EULER && h->p.integrator != NS2D_RK4)
                            ? 4
@@ -779,11 +908,39 @@ ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
     return NS2D_OK;
 }
 
+// nsteps fixed-dt steps of the configured integrator, queued on the handle's
+// stream.
+ns2d_status queue_steps(ns2d_handle* h, int nsteps, double dt) {
+    ns2d_status s = NS2D_OK;
+    for (int k = 0; k < nsteps && s == NS2D_OK;) {
+        int n = 1;
+        if (h->p.integrator == NS2D_AB4 && h->ab_count < 3) {
+            const int it = h->ab_count + 1;
+            ns2d_params saved = h->p;
+            h->p.integrator = NS2D_RK4CN;
+            s = DISPATCH(h, rk4_step_impl, h, dt, h->ab[it - 1]);
+            h->p = saved;
+            h->ab_count = it;
+        } else if (resident_ok(h)) {
+            n = nsteps - k;
+            if (h->p.integrator == NS2D_AB4) s = DISPATCH(h, resident_ab4, h, n, dt);
+            else s = DISPATCH(h, resident_rk4, h, n, dt, nullptr);
+        } else if (h->p.integrator == NS2D_AB4) {
+            s = DISPATCH(h, ab4_update_impl, h, dt);
+        } else {
+            s = rk4_step_loop(h, dt);
+        }
+        k += n;
+    }
+    return s;
+}
+
 // One step for the per-call entry points (ns2d_rk4_step, ns2d_rk4_step_host):
 // eager when dt differs from the previous call's (adaptive stepping would
 // recapture every step), the graph-replayed step of the time loops when the
 // same dt comes again.  Both run the same kernels on the same arguments.
 ns2d_status single_step(ns2d_handle* h, double dt) {
+    if (resident_ok(h)) return DISPATCH(h, resident_rk4, h, 1, dt, nullptr);
     const bool again = (h->last_call_dt == dt);
     h->last_call_dt = dt;
     if (again) return rk4_step_loop(h, dt);
@@ -1199,21 +1356,7 @@ ns2d_status ns2d_step_n(ns2d_handle* h, int32_t nsteps, double dt) {
             if ((s = check_status(h))) return s;
             continue;
         }
-        for (int k = done; k < nsteps; ++k) {
-            if (h->p.integrator == NS2D_AB4 && h->ab_count < 3) {
-                const int it = h->ab_count + 1;
-                ns2d_params saved = h->p;
-                h->p.integrator = NS2D_RK4CN;
-                s = DISPATCH(h, rk4_step_impl, h, dt, h->ab[it - 1]);
-                h->p = saved;
-                h->ab_count = it;
-            } else if (h->p.integrator == NS2D_AB4) {
-                s = DISPATCH(h, ab4_update_impl, h, dt);
-            } else {
-                s = rk4_step_loop(h, dt);
-            }
-            if (s) return s;
-        }
+        if ((s = queue_steps(h, nsteps - done, dt))) return s;
         if ((s = read_status(h, &bits, &steps1))) return s;
         done += steps1 - steps0;
         if (bits && (s = check_status(h))) return s;  // a false alarm is cleared and the loop resumes
@@ -1391,23 +1534,7 @@ ns2d_status ns2d_step_async(ns2d_handle* h, int32_t nsteps, double dt) {
     if (!h || nsteps < 0) return NS2D_ERR_INVALID;
     if (h->p.integrator == NS2D_DP5) return fail(h, NS2D_ERR_UNSUPPORTED, "DP5 is advanced by its own entry point");
     cudaSetDevice(h->p.device);
-    for (int k = 0; k < nsteps; ++k) {
-        ns2d_status s;
-        if (h->p.integrator == NS2D_AB4 && h->ab_count < 3) {
-            const int it = h->ab_count + 1;
-            ns2d_params saved = h->p;
-            h->p.integrator = NS2D_RK4CN;
-            s = DISPATCH(h, rk4_step_impl, h, dt, h->ab[it - 1]);
-            h->p = saved;
-            h->ab_count = it;
-        } else if (h->p.integrator == NS2D_AB4) {
-            s = DISPATCH(h, ab4_update_impl, h, dt);
-        } else {
-            s = rk4_step_loop(h, dt);
-        }
-        if (s) return s;
-    }
-    return NS2D_OK;
+    return queue_steps(h, nsteps, dt);
 }
 
 ns2d_status ns2d_set_forcing_modes(ns2d_handle* h, int32_t n, const int32_t* idx, const double* values) {

@@ -38,8 +38,18 @@ template <typename C>
 __device__ __forceinline__ C cadd(C a, C b) { return cmake<C>(a.x + b.x, a.y + b.y); }
 template <typename C>
 __device__ __forceinline__ C csub(C a, C b) { return cmake<C>(a.x - b.x, a.y - b.y); }
+// Products with their roundings written out.  Left to the compiler, which of
+// two products a multiply-add absorbs can differ from one kernel to the next;
+// the transforms of every kernel round alike, so kernels that share a plan give
+// the same bits.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 template <typename C>
-__device__ __forceinline__ C cmul(C a, C b) { return cmake<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+__device__ __forceinline__ C cmul(C a, C b) {
+    return cmake<C>(fma_rn(a.x, b.x, -mul_rn(a.y, b.y)), fma_rn(a.x, b.y, mul_rn(a.y, b.x)));
+}
 template <typename C>
 __device__ __forceinline__ C cconj(C a) { return cmake<C>(a.x, -a.y); }
 template <typename C>
@@ -80,13 +90,33 @@ __device__ __forceinline__ C ctw(C a) {
         constexpr Real s1 = (Real)0.38268343236508977173;  // sin(pi/8)
         constexpr int q = k % 4;                           // 1 or 3 within the quadrant
         constexpr Real cr = (q == 1) ? c1 : s1;
-        constexpr Real si = (q == 1) ? s1 : c1;
-        C b = cmake<C>(a.x * cr - a.y * (SIGN * si), a.x * (SIGN * si) + a.y * cr);
+        constexpr Real si = (Real)SIGN * ((q == 1) ? s1 : c1);
+        C b = cmake<C>(fma_rn(a.x, cr, -mul_rn(a.y, si)), fma_rn(a.x, si, mul_rn(a.y, cr)));
         constexpr int quad = k / 4;
         if constexpr (quad == 0) return b;
         else if constexpr (quad == 1) return cmul_i<SIGN>(b);
         else if constexpr (quad == 2) return cmake<C>(-b.x, -b.y);
         else return cmul_i<-SIGN>(b);
+    }
+}
+
+// Butterfly p = e + W o, q = e - W o with W = exp(SIGN * 2 pi i K / R), K < R/2;
+// the scale 1/sqrt2 of the 45-degree twiddles goes into the multiply-adds.
+template <int R, int K, int SIGN, typename C>
+__device__ __forceinline__ void butterfly(C e, C o, C& p, C& q) {
+    using Real = decltype(C::x);
+    if constexpr (8 * K == R || 8 * K == 3 * R) {
+        constexpr Real h = (Real)0.70710678118654752440;
+        // W o = h d
+        C d;
+        if constexpr (8 * K == R) d = SIGN > 0 ? cmake<C>(o.x - o.y, o.x + o.y) : cmake<C>(o.x + o.y, o.y - o.x);
+        else d = SIGN > 0 ? cmake<C>(-(o.x + o.y), o.x - o.y) : cmake<C>(o.y - o.x, -(o.x + o.y));
+        p = cmake<C>(fma_rn(h, d.x, e.x), fma_rn(h, d.y, e.y));
+        q = cmake<C>(fma_rn(-h, d.x, e.x), fma_rn(-h, d.y, e.y));
+    } else {
+        const C w = ctw<R, K, SIGN>(o);
+        p = cadd(e, w);
+        q = csub(e, w);
     }
 }
 
@@ -106,10 +136,7 @@ struct SmallDFT {
     template <int K>
     __device__ __forceinline__ static void combine(const C* tmp, C* v) {
         if constexpr (K < R / 2) {
-            C e = tmp[2 * K];
-            C o = ctw<R, K, SIGN>(tmp[2 * K + 1]);
-            v[K * S] = cadd(e, o);
-            v[(K + R / 2) * S] = csub(e, o);
+            butterfly<R, K, SIGN>(tmp[2 * K], tmp[2 * K + 1], v[K * S], v[(K + R / 2) * S]);
             combine<K + 1>(tmp, v);
         }
     }

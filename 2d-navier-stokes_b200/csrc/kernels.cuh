@@ -294,8 +294,10 @@ __device__ __forceinline__ Real kx_of(int m, int t, Real tr) {
 // Derived spectra of the stage input X at (kx, ky) (solver.c:904-957), two at a
 // time: pair 0 gives u = i ky/k^2 X and v = -i kx/k^2 X (one reciprocal), pair 2
 // gives w_x = i kx X and w_y = i ky X.  Zero at the mean mode.  kx and ky are
-// integers held as reals.
-template <typename C>
+// integers held as reals.  RN: the products rounded before the transform's first
+// additions (the sizes that the resident kernel serves too; see mul_rn), which
+// costs the multiply-adds of that stage.
+template <bool RN, typename C>
 __device__ __forceinline__ void derived_pair(int fp, decltype(C::x) kx, decltype(C::x) ky, C X, C& a, C& b) {
     using Real = decltype(C::x);
     if (kx == (Real)0 && ky == (Real)0) {
@@ -313,8 +315,19 @@ __device__ __forceinline__ void derived_pair(int fp, decltype(C::x) kx, decltype
         sb = ky;
     }
     // i s X = (-s X.y, s X.x)
-    a = cmake<C>(-sa * X.y, sa * X.x);
-    b = cmake<C>(-sb * X.y, sb * X.x);
+    if constexpr (RN) {
+        a = cmake<C>(mul_rn(-sa, X.y), mul_rn(sa, X.x));
+        b = cmake<C>(mul_rn(-sb, X.y), mul_rn(sb, X.x));
+    } else {
+        a = cmake<C>(-sa * X.y, sa * X.x);
+        b = cmake<C>(-sb * X.y, sb * X.x);
+    }
+}
+
+// Crank-Nicolson update f w + g tot (solver.c:853).
+template <typename C>
+__device__ __forceinline__ C cn_update(C w, C tot, decltype(C::x) f, decltype(C::x) g) {
+    return cmake<C>(fma_rn(tot.x, g, mul_rn(w.x, f)), fma_rn(tot.y, g, mul_rn(w.y, f)));
 }
 
 // Derived spectra of the stage input X (pre0, [N][TC] in shared memory) and
@@ -336,7 +349,7 @@ __device__ __forceinline__ void derived_ifft(const typename Cx<Real>::T* pre0, t
 #pragma unroll
         for (int m = 0; m < E; ++m) {
             const int i = t + T * m;
-            derived_pair(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+            derived_pair<(N <= 128)>(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
         }
         fft_batched<N, +1, 2>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
         if (valid) {
@@ -383,7 +396,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const int i = t + T * m;
-                derived_pair(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+                derived_pair<(N <= 128)>(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
             }
             // first pair: the accumulator store (if any) must have read B1;
             // second pair: the first pair's first field must have left B0 (at
@@ -418,7 +431,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const int i = t + T * m;
-                derived_pair(0, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+                derived_pair<(N <= 128)>(0, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
             }
             if (pending) {  // the accumulator store must have read B1
                 if (threadIdx.x == 0) bulk_wait_read_all();
@@ -443,7 +456,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 #pragma unroll
         for (int m = 0; m < E; ++m) {
             const int i = t + T * m;
-            derived_pair(2, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+            derived_pair<(N <= 128)>(2, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
         }
         __syncthreads();  // every thread has read B2
 #pragma unroll 1
@@ -711,7 +724,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
                     } else {
                         // Crank-Nicolson factors (solver.c:853), from the table
                         const double2 f = a.cn[(size_t)i * ldc + kyc];
-                        wn = cadd(cscale(w, (Real)f.x), cscale(tot, (Real)f.y));
+                        wn = cn_update<C>(w, tot, (Real)f.x, (Real)f.y);
                     }
                     if (!FAST && a.phase_only && (kx != 0 || ky != 0)) {
                         // amplitude reset of the phase-only model (solver.c:822-824, 855-857):
@@ -915,7 +928,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, int rblock, uns
     // n = 1.0 * (u w_x + v w_y)  (solver.c:979-981), parked for the packing
     Real* nl_own = reinterpret_cast<Real*>(region + TL::ROWS);
 #pragma unroll
-    for (int m = 0; m < E; ++m) nl_own[t + T * m] = v[0][m].x * v[1][m].x + v[0][m].y * v[1][m].y;
+    for (int m = 0; m < E; ++m) nl_own[t + T * m] = fma_rn(v[0][m].x, v[1][m].x, mul_rn(v[0][m].y, v[1][m].y));
     // HALF: each team transforms its own row's real product as an N/2-point
     // complex sequence z[j] = n[2j] + i n[2j+1] and splits the result,
     //   X[k] = (Z[k] + conj Z[N/2-k])/2 + W^k (Z[k] - conj Z[N/2-k])/(2i),
