@@ -53,6 +53,7 @@ struct AdjointState {
     void* mu = nullptr;                                 // adjoint column-pass output
     void* w_final = nullptr;
     double* dpart = nullptr;  // per-block partial sums
+    int* band = nullptr;      // the recorded run's band_narrow word of the state
     bool ready = false;       // kernel attributes set
     cudaStream_t stream = nullptr;  // adjoint stream
     cudaEvent_t rec_done[2] = {nullptr, nullptr}, adj_done[2] = {nullptr, nullptr}, join = nullptr;
@@ -86,7 +87,7 @@ const double kA[3] = {0.5, 0.5, 1.0};
 
 template <typename Real, int N>
 struct AdjLaunch {
-    using S = Shape<N>;
+    using S = Shape<Real, N>;
     static constexpr size_t col_smem() { return ColSmem<Real, N, S::TC>::bytes(); }
     static constexpr size_t row_smem() { return RowSmem<Real, N, 2 * S::PAIRS>::bytes(); }
     static cudaError_t setup() {
@@ -138,7 +139,7 @@ void drop_graphs(AdjointState* a) {
 void free_state(AdjointState* a) {
     drop_graphs(a);
     void* ptrs[] = {a->ckpt, a->cap[0], a->cap[1], a->lam[0], a->lam[1], a->P[0], a->P[1],
-                    a->P[2], a->P[3], a->mu, a->w_final, a->dpart};
+                    a->P[2], a->P[3], a->mu, a->w_final, a->dpart, a->band};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     cudaEvent_t evs[] = {a->rec_done[0], a->rec_done[1], a->adj_done[0], a->adj_done[1], a->join,
@@ -183,6 +184,7 @@ ns2d_status ensure_buffers(ns2d_handle* h, int nsteps, int every) {
             ACK(h, cudaMalloc(f, h->field_bytes));
             ACK(h, cudaMemsetAsync(*f, 0, h->field_bytes, h->stream));
         }
+    if (!a->band) ACK(h, cudaMalloc(&a->band, sizeof(int)));
     if (!a->dpart) ACK(h, cudaMalloc(&a->dpart, sizeof(double) * kRedBlocks));
     if (!a->stream) {
         ACK(h, cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking));
@@ -403,6 +405,10 @@ ns2d_status backward_impl(ns2d_handle* h) {
     // the CN table of the recorded dt, before any launch reads it
     ns2d_status s0 = internal::ensure_cn(h, a->dt, a->branch);
     if (s0) return s0;
+    // the state becomes the recorded run's again, which the caller may have
+    // replaced since
+    ACK(h, cudaMemcpyAsync(h->dband, a->band, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+    h->band_known = true;
     ACK(h, cudaEventRecord(a->t[2], h->stream));
     ACK(h, cudaStreamWaitEvent(a->stream, a->t[2], 0));  // lambda(T) is written on the handle's stream
     ns2d_status st = recompute_segment(h, nck - 1, (nck - 1) & 1);
@@ -467,6 +473,8 @@ ns2d_status record(ns2d_handle* h, int nsteps, double dt, int every) {
     if ((s = ensure_buffers(h, nsteps, every))) return s;
     AdjointState* a = h->adj;
     a->recorded = false;
+    if ((s = internal::ensure_band(h))) return s;
+    ACK(h, cudaMemcpyAsync(a->band, h->dband, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
     ACK(h, cudaEventRecord(a->t[0], h->stream));
     for (int k = 0; k < nsteps; ++k) {
         if (k % every == 0)

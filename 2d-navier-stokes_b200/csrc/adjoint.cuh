@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(Plan<N>::T * TC) adj_col_kernel(AdjColArgs<Rea
     const bool valid = ky < a.nyf;
     const int kyc = valid ? ky : 0;
     const int ldc = a.ldc;
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N>(a.tw, t);
 
     if constexpr (MODE != ADJ_START) {
         // L = conj(m_u) P0 + conj(m_v) P1 + conj(m_x) P2 + conj(m_y) P3
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) adj_row_kernel(AdjRowA
     const int t = threadIdx.x % T;
     const int x = blockIdx.x * TC + g;
     C* region = reinterpret_cast<C*>(smraw) + (size_t)g * RS::TEAM;
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N>(a.tw, t);
     const TeamPolicy<N, C> pol{region, 1 + g};
     // mu = c2r(mu_x) along y: Hermitian extension, real parts at ky = 0 and N/2
     C z[1][E];

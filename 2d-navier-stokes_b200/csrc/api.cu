@@ -55,9 +55,10 @@ LinOp make_lin(const ns2d_handle* h, int branch) { return make_lin_params(h->p, 
 
 bool quirk(const ns2d_handle* h, int bit) { return (h->p.quirks & bit) != 0; }
 
+template <typename Real>
 int col_tc(int n) {
     int tc = 0;
-    with_size<double>(n, [&](auto L) { tc = decltype(L)::S::TC; });
+    with_size<Real>(n, [&](auto L) { tc = decltype(L)::S::TC; });
     return tc;
 }
 
@@ -79,6 +80,8 @@ void fill_common(ns2d_handle* h, ColArgs<Real>& a, int branch) {
     a.nyf = h->nyf;
     const int m = (int)(h->nx / 3.0);
     a.kmax_sqr = m * m + h->p.dealias_edge;
+    a.kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
+    a.band = h->dband;
     a.dealias = h->p.dealias;
     a.houli_int = quirk(h, NS2D_QUIRK_HOU_LI_INT) ? 1 : 0;
     a.kolm = (h->p.forcing == NS2D_FORCING_KOLM) ? 1 : 0;
@@ -93,7 +96,7 @@ void fill_common(ns2d_handle* h, ColArgs<Real>& a, int branch) {
     a.status = h->dstatus;
     a.final_tail = 1;
     a.force_field = h->ffield_on ? (const C*)h->ffield : nullptr;
-    a.ntiles = (h->nyf + col_tc(h->nx) - 1) / col_tc(h->nx);
+    a.ntiles = (h->nyf + col_tc<Real>(h->nx) - 1) / col_tc<Real>(h->nx);
     a.lin = make_lin(h, branch);
     a.phase_only = h->p.model == NS2D_MODEL_PHASE_ONLY ? 1 : 0;
 }
@@ -110,6 +113,8 @@ RowArgs<Real> row_args(ns2d_handle* h) {
     r.tw = (const C*)h->tw;
     r.ldc = h->ldc;
     r.nrows = h->nx;
+    r.kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
+    r.band = h->dband;
     r.status = h->dstatus;
     return r;
 }
@@ -169,7 +174,7 @@ struct TimedLaunch {
 template <typename Real>
 void build_col_maps(ns2d_handle* h) {
     if (!tma_copies_enabled()) return;
-    const int tc = col_tc(h->nx);
+    const int tc = col_tc<Real>(h->nx);
     auto* m = new (std::nothrow) ColMaps;
     if (!m) return;
     void* const bases[7] = {h->f[0], h->f[1], h->f[2], h->f[3], h->acc, h->state, h->nl};
@@ -202,25 +207,16 @@ void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a) {
 // Row pass of stage `stage` (1..4); with a capture target set, the stage's real
 // fields go to planes 2(stage-1) and 2(stage-1)+1 of it.
 template <typename Real>
-void launch_row(ns2d_handle* h, int stage = 0) {
+void launch_row(ns2d_handle* h, int stage = 0, bool use_band = true) {
     TimedLaunch t(h, 3);
     RowArgs<Real> r = row_args<Real>(h);
+    if (!use_band) r.band = nullptr;
     if (h->cap_step && stage >= 1) {
         const size_t plane = (size_t)h->nx * h->ny;
         r.cap_uv = (Cplx<Real>*)h->cap_step + (size_t)(2 * (stage - 1)) * plane;
         r.cap_w = r.cap_uv + plane;
     }
     with_size<Real>(h->nx, [&](auto L) { decltype(L)::row(r, h->stream); });
-}
-
-// First ky column the 2/3 rule empties (every kx there has k2 >= kmax_sqr), nyf
-// for the Hou-Li filter, which empties none.
-int kept_columns(const ns2d_handle* h) {
-    if (h->p.dealias != 0) return h->nyf;
-    const int m = (int)(h->nx / 3.0), lim = m * m + h->p.dealias_edge;
-    int kc = 0;
-    while (kc < h->nyf && kc * kc < lim) ++kc;
-    return kc;
 }
 
 // Whether this handle's steps and evaluations run in the resident kernel: a
@@ -242,7 +238,7 @@ void fill_resident(ns2d_handle* h, ResArgs<Real>& r, int branch) {
     r.ldc = a.ldc;
     r.nyf = a.nyf;
     r.kmax_sqr = a.kmax_sqr;
-    r.kc = kept_columns(h);
+    r.kc = a.kc;
     r.dealias = a.dealias;
     r.houli_int = a.houli_int;
     r.kolm = a.kolm;
@@ -283,10 +279,43 @@ void compute_forcing(ns2d_handle* h, double dt) {
     }
 }
 
+// Whether the pass kernels may leave out the columns the 2/3 rule empties
+// (band_narrow): after the state was written from outside, one scan of those
+// columns on the device; the passes read its answer there, so nothing waits for
+// it.  Steps keep zeros there zero, except with a forced mode among them (the
+// column stays in use until the state is set again).
+ns2d_status ensure_band(ns2d_handle* h) {
+    if (h->band_known) return NS2D_OK;
+    const int kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
+    if (h->band_forced || (h->forced && h->force_j >= kc)) {
+        CK(h, cudaMemsetAsync(h->dband, 1, sizeof(int), h->stream));
+    } else {
+        CK(h, cudaMemsetAsync(h->dband, 0, sizeof(int), h->stream));
+        if (kc < h->nyf) {
+            if (h->fp32)
+                band_scan_kernel<float><<<148, 256, 0, h->stream>>>((const float2*)h->state, h->nx, h->nyf, h->ldc, kc, h->dband);
+            else
+                band_scan_kernel<double><<<148, 256, 0, h->stream>>>((const double2*)h->state, h->nx, h->nyf, h->ldc, kc, h->dband);
+            h->launches++;
+            CKL(h);
+        }
+    }
+    h->band_known = true;
+    return NS2D_OK;
+}
+
+// The state was written from outside (set_w_hat and the host-resident step).
+void state_replaced(ns2d_handle* h) {
+    h->band_known = false;
+    h->band_forced = h->ffield_on && h->ffield_band;
+}
+
 // Rebuild the Crank-Nicolson factor table when dt or the operator branch changed.
 ns2d_status ensure_cn(ns2d_handle* h, double dt, int branch) {
     if (h->cn_dt == dt && h->cn_branch == branch) return NS2D_OK;
-    cn_table_kernel<<<296, 256, 0, h->stream>>>(h->cn, h->nx, h->nyf, h->ldc, dt, make_lin(h, branch));
+    CK(h, cudaMemsetAsync(h->dband + 1, 0, sizeof(int), h->stream));
+    cn_table_kernel<<<296, 256, 0, h->stream>>>(h->cn, h->nx, h->nyf, h->ldc, dt, make_lin(h, branch),
+                                                kept_columns(h->nx, h->p.dealias, h->p.dealias_edge), h->dband + 1);
     h->launches++;
     CKL(h);
     h->cn_dt = dt;
@@ -303,6 +332,7 @@ template <typename Real>
 ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
     using C = Cplx<Real>;
     if (resident_ok(h)) return resident_rk4<Real>(h, 1, dt, rk1_out);
+    if (ns2d_status sb = ensure_band(h)) return sb;
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const bool explicit_rk4 = euler || h->p.integrator == NS2D_RK4;
@@ -423,6 +453,7 @@ template <typename Real>
 ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
     using C = Cplx<Real>;
     if (resident_ok(h)) return resident_ab4<Real>(h, 1, dt);
+    if (ns2d_status sb = ensure_band(h)) return sb;
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
@@ -471,11 +502,16 @@ ns2d_status rhs_impl(ns2d_handle* h, const void* src, bool src_is_state) {
         r.conj_quirk = (quirk(h, NS2D_QUIRK_CONJ_STATE) || src_is_state) ? 1 : 0;
         return launch_resident(h, RES_RHS, r);
     }
+    // of an input other than the state nothing is known
+    if (src_is_state) {
+        if (ns2d_status sb = ensure_band(h)) return sb;
+    }
     ColArgs<Real> a;
     fill_common<Real>(h, a, 4);
     a.src = (const C*)src;
+    if (!src_is_state) a.band = nullptr;
     launch_col<Real>(h, COL_P1, a);
-    launch_row<Real>(h);
+    launch_row<Real>(h, 0, src_is_state);
     fill_common<Real>(h, a, 4);
     a.src = (const C*)h->nl;
     a.rhs_store = (C*)h->rhsbuf;
@@ -511,6 +547,7 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
         CK(h, cudaMalloc((void**)&h->dp_kptr, sizeof(void*) * 7));
         CK(h, cudaMemcpy((void*)h->dp_kptr, h->dp, sizeof(void*) * 7, cudaMemcpyHostToDevice));
     }
+    if (ns2d_status sb = ensure_band(h)) return sb;
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
@@ -595,6 +632,7 @@ ns2d_status rk5dp_step_impl(ns2d_handle* h, double dt, int iters, double* err) {
         CK(h, cudaMalloc(&h->dp_last, h->field_bytes));
         CK(h, cudaMemsetAsync(h->dp_last, 0, h->field_bytes, h->stream));
     }
+    if (ns2d_status sb = ensure_band(h)) return sb;
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
@@ -756,7 +794,7 @@ void fill_twiddles(std::vector<Cplx<Real>>& tw, int n) {
 void free_all(ns2d_handle* h) {
     void* ptrs[] = {h->state, h->acc, h->nl, h->f[0], h->f[1], h->f[2], h->f[3], h->tmpfull, h->col0[0], h->col0[1],
                     h->tw, h->rhsbuf, h->ab[0], h->ab[1], h->ab[2], h->ab[3], h->uhat_ref, h->dreal, h->dscal, h->dmax,
-                    h->dstatus, h->dio, h->ddiag, h->dpart, h->cn, h->dp_last};
+                    h->dstatus, h->dband, h->dio, h->ddiag, h->dpart, h->cn, h->dp_last};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (void* p : h->dp)
@@ -792,6 +830,8 @@ ns2d_status create_impl(ns2d_handle* h) {
     CK(h, cudaMalloc(&h->dmax, sizeof(unsigned long long) * 2));
     CK(h, cudaMalloc(&h->dstatus, sizeof(int) * 4));
     CK(h, cudaMemsetAsync(h->dstatus, 0, sizeof(int) * 4, h->stream));
+    CK(h, cudaMalloc(&h->dband, sizeof(int) * 2));
+    CK(h, cudaMemsetAsync(h->dband, 0, sizeof(int) * 2, h->stream));
     CK(h, cudaMalloc(&h->dio, sizeof(double2) * (size_t)h->nx * h->nyf));
     CK(h, cudaMalloc(&h->ddiag, sizeof(double) * (DG_N + 8 * (size_t)h->n_spect)));
     CK(h, cudaMalloc(&h->dpart, sizeof(double) * 4096));
@@ -868,6 +908,7 @@ ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out) {
 // adjoint uses the eager form.
 ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
     if (h->cap_step || resident_ok(h)) return DISPATCH(h, rk4_step_impl, h, dt, nullptr);
+    if (ns2d_status sb = ensure_band(h)) return sb;
     int hf = h->hyper_flag;
     const int branch = (h->p.system == NS2D_EULER && h->p.integrator != NS2D_RK4)
                            ? 4
@@ -1127,6 +1168,7 @@ ns2d_status fail(ns2d_handle* h, ns2d_status s, const std::string& msg) { return
 ns2d_status rk4_step(ns2d_handle* h, double dt) { return DISPATCH(h, rk4_step_impl, h, dt, nullptr); }
 ns2d_status rk4_step_loop(ns2d_handle* h, double dt) { return ::rk4_step_loop(h, dt); }
 ns2d_status ensure_cn(ns2d_handle* h, double dt, int branch) { return ::ensure_cn(h, dt, branch); }
+ns2d_status ensure_band(ns2d_handle* h) { return ::ensure_band(h); }
 ns2d_status check_status(ns2d_handle* h) { return ::check_status(h); }
 ns2d_status pack_in(ns2d_handle* h, const double2* d_src, void* dst) { return DISPATCH(h, ::pack_in, h, d_src, dst); }
 ns2d_status unpack_out(ns2d_handle* h, const void* src, double2* d_dst) {
@@ -1262,6 +1304,7 @@ ns2d_status ns2d_dims(const ns2d_handle* h, int32_t* nx, int32_t* ny, int32_t* n
 ns2d_status ns2d_set_w_hat(ns2d_handle* h, const double* w_hat) {
     if (!h || !w_hat) return NS2D_ERR_INVALID;
     cudaSetDevice(h->p.device);
+    state_replaced(h);
     ns2d_status s = host_to_state(h, w_hat, h->state);
     if (s) return s;
     s = clear_status(h);
@@ -1280,6 +1323,7 @@ ns2d_status ns2d_get_w_hat(ns2d_handle* h, double* w_hat) {
 ns2d_status ns2d_set_w_hat_device(ns2d_handle* h, const double* d_w_hat) {
     if (!h || !d_w_hat) return NS2D_ERR_INVALID;
     cudaSetDevice(h->p.device);
+    state_replaced(h);
     ns2d_status s = DISPATCH(h, pack_in, h, (const double2*)d_w_hat, h->state);
     if (s) return s;
     s = clear_status(h);
@@ -1523,6 +1567,7 @@ ns2d_status ns2d_mean_flow(ns2d_handle* h, double* mean_x, double* mean_y) {
 ns2d_status ns2d_rk4_step_host(ns2d_handle* h, double* w_hat, double dt) {
     if (!h || !w_hat) return NS2D_ERR_INVALID;
     cudaSetDevice(h->p.device);
+    state_replaced(h);
     ns2d_status s = host_to_state(h, w_hat, h->state);
     if (s) return s;
     if ((s = single_step(h, dt))) return s;
@@ -1547,8 +1592,12 @@ ns2d_status ns2d_set_forcing_modes(ns2d_handle* h, int32_t n, const int32_t* idx
         return NS2D_OK;
     }
     const int64_t total = (int64_t)h->nx * h->nyf;
-    for (int32_t m = 0; m < n; ++m)
+    const int kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
+    bool past_kc = false;  // a forced mode in the columns the dealiasing empties
+    for (int32_t m = 0; m < n; ++m) {
         if (idx[m] < 0 || idx[m] >= total) return fail(h, NS2D_ERR_INVALID, "forcing index outside the half spectrum");
+        past_kc |= idx[m] % h->nyf >= kc;
+    }
     if (!h->ffield) CK(h, cudaMalloc(&h->ffield, h->field_bytes));
     if (h->fcap < n) {
         if (h->fidx) cudaFree(h->fidx);
@@ -1572,6 +1621,11 @@ ns2d_status ns2d_set_forcing_modes(ns2d_handle* h, int32_t n, const int32_t* idx
     CKL(h);
     CK(h, cudaStreamSynchronize(h->stream));  // the caller's arrays may go away on return
     h->ffield_on = true;
+    h->ffield_band = past_kc;
+    if (past_kc) {
+        h->band_forced = true;
+        h->band_known = false;
+    }
     if (!was_on) drop_graph(h);  // captured steps carry the field pointer only when it is on
     return NS2D_OK;
 }

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(Plan<N>::T * TC) col_inv_kernel(InvArgs<Real> 
     const int ky = blockIdx.x * TC + c;
     const bool valid = ky < a.nyf;
     const int kyc = valid ? ky : 0;
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N>(a.tw, t);
     for (int f = 0; f < a.nf; ++f) {
         const InvField<Real> F = a.f[f];
         C v[E];
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) row_c2r_kernel(RowC2RA
     const int x = blockIdx.x * TC + g;
     const C* rA = a.A + (size_t)x * a.ldc;
     const C* rB = a.B ? a.B + (size_t)x * a.ldc : nullptr;
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N>(a.tw, t);
     C z[E];
 #pragma unroll
     for (int m = 0; m < E; ++m) {
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(Plan<N>::T * TC) fwd_kernel(const double* __re
     const int line = blockIdx.x * TC + c;
     const bool valid = line < nlines;
     const int lc = valid ? line : 0;
-    const TwSeed<C> seed = twiddle_seeds<N>(tw, t);
+    const auto seed = twiddle_seeds<N>(tw, t);
     C v[E];
 #pragma unroll
     for (int m = 0; m < E; ++m) {

@@ -10,7 +10,7 @@ namespace ns2d {
 // accesses fetch TC * 16 B per row, so wider tiles use each row's cache line
 // better; at 512 and 1024 four columns per block measured faster than two
 // (even with fewer blocks than SMs at 1024), so they get TC = 4.
-template <int N>
+template <typename Real, int N>
 struct Shape {
     static constexpr int T = Plan<N>::T;
     static constexpr int TC_RAW = 128 / T < 2 ? 2 : 128 / T;
@@ -22,7 +22,7 @@ struct Shape {
 template <typename Real, int N>
 struct Launch {
     using C = typename Cx<Real>::T;
-    using S = Shape<N>;
+    using S = Shape<Real, N>;
     static constexpr int SIZE = N;
     static constexpr size_t col_smem() { return ColSmem<Real, N, S::TC>::bytes(); }
     static constexpr size_t col_tma_smem() { return ColSmem<Real, N, S::TC>::bytes_tma() + 1024; }

@@ -53,6 +53,7 @@ struct ns2d_ensemble {
     std::vector<void*> state, nl, acc, tw;
     std::vector<double2*> cn;
     std::vector<int> ldc;
+    int* band = nullptr;          // [n][2]: band_narrow words of each member
     double2* io = nullptr;        // staging for host I/O, largest member
     int col_grid = 0, row_grid = 0;
     // CN tables and graph for the current dt
@@ -217,6 +218,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
     e->tw.resize(e->n);
     e->cn.resize(e->n);
     e->ldc.resize(e->n);
+    ECK(e, alloc(sizeof(int) * 2 * (size_t)e->n, (void**)&e->band));
     for (int m = 0; m < e->n; ++m) {
         const int n = e->sizes[m];
         const int nyf = n / 2 + 1;
@@ -260,6 +262,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
         a.nyf = nyf;
         const int km = (int)(n / 3.0);
         a.kmax_sqr = km * km;
+        a.kc = kept_columns(n, e->p.dealias, 0);
         a.dealias = e->p.dealias;
         a.houli_int = (e->p.quirks & NS2D_QUIRK_HOU_LI_INT) ? 1 : 0;
         a.kolm = (e->p.forcing == NS2D_FORCING_KOLM) ? 1 : 0;
@@ -270,6 +273,8 @@ ns2d_status create_t(ns2d_ensemble* e) {
             a.force_val.x = (Real)(-0.5 * e->p.force_scale * (double)e->p.force_k);
             a.force_val.y = (Real)0;
         }
+        // a forced mode among the emptied columns keeps them in the transforms
+        if (!(a.has_force && a.force_j >= a.kc)) a.band = e->band + 2 * m;
         a.norm2 = (Real)std::pow(1.0 / (double)(n * n), 2.0);
         a.inv_nxny = 1.0 / (double)(n * n);
         a.cn = (const double2*)cn;
@@ -282,6 +287,8 @@ ns2d_status create_t(ns2d_ensemble* e) {
         mb.row.tw = (const C*)tw;
         mb.row.ldc = ldc;
         mb.row.nrows = n;
+        mb.row.kc = a.kc;
+        mb.row.band = a.band;
         mb.row.status = nullptr;
         mb.col0[0] = (C*)c0[0];
         mb.col0[1] = (C*)c0[1];
@@ -397,7 +404,10 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
         const LinOp L = make_lin_params(e->p, branch);
         for (int m = 0; m < e->n; ++m) {
             const int n = e->sizes[m];
-            cn_table_kernel<<<148, 256, 0, e->stream>>>(e->cn[m], n, n / 2 + 1, e->ldc[m], dt, L);
+            int* const odd = e->band + 2 * m + 1;
+            ECK(e, cudaMemsetAsync(odd, 0, sizeof(int), e->stream));
+            cn_table_kernel<<<148, 256, 0, e->stream>>>(e->cn[m], n, n / 2 + 1, e->ldc[m], dt, L,
+                                                        kept_columns(n, e->p.dealias, 0), odd);
             e->launches++;
         }
         e->cn_dt = dt;
@@ -547,9 +557,13 @@ ns2d_status check_impl(ns2d_ensemble* e) {
 template <typename Real>
 ns2d_status set_t(ns2d_ensemble* e, int m, const double* host) {
     const int n = e->sizes[m], nyf = n / 2 + 1;
+    using C = typename Cx<Real>::T;
     ECK(e, cudaMemcpyAsync(e->io, host, sizeof(double2) * (size_t)n * nyf, cudaMemcpyHostToDevice, e->stream));
-    pack_kernel<Real><<<148, 256, 0, e->stream>>>(e->io, (typename Cx<Real>::T*)e->state[m], n, nyf, e->ldc[m]);
-    e->launches++;
+    ECK(e, cudaMemsetAsync(e->band + 2 * m, 0, sizeof(int), e->stream));
+    pack_kernel<Real><<<148, 256, 0, e->stream>>>(e->io, (C*)e->state[m], n, nyf, e->ldc[m]);
+    band_scan_kernel<Real><<<32, 256, 0, e->stream>>>((const C*)e->state[m], n, nyf, e->ldc[m],
+                                                      kept_columns(n, e->p.dealias, 0), e->band + 2 * m);
+    e->launches += 2;
     ECK(e, cudaGetLastError());
     ECK(e, cudaStreamSynchronize(e->stream));
     return NS2D_OK;

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
                                                       const EnsItem* __restrict__ items, int nitems, EnsStage st,
                                                       const ColMaps* __restrict__ maps) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    if (block_should_exit(st.status)) return;
+    if (block_begin(st.status, nullptr).exit) return;
     unsigned char* sm = smraw;
     if constexpr (TMA) sm = smraw + ((1024u - ((unsigned)__cvta_generic_to_shared(smraw) & 1023u)) & 1023u);
     constexpr int VI = THREADS == kEnsThreadChoices[0] ? 0 : 1;
@@ -102,11 +102,16 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
         ColArgs<Real> a = mb.col;
         ens_apply_stage(a, mb, st);
         const ColMaps* mp = TMA ? maps + 2 * item.member + VI : nullptr;
+        const bool narrow = band_narrow(a.band);
+        const auto begin = [&] {
+            __syncthreads();
+            return BlockBegin{false, narrow};
+        };
         bool go = true;
         switch (mb.n) {
 #define NS2D_ENS_COL(NN)                                                                           \
     case NN:                                                                                       \
-        go = col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE, FAST, TMA>(a, item.tile, sm, mp); \
+        go = col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE, FAST, TMA>(a, begin, item.tile, sm, mp); \
         break;
             NS2D_ENS_SIZES(NS2D_ENS_COL)
 #undef NS2D_ENS_COL
@@ -120,14 +125,15 @@ template <typename Real, int THREADS>
 __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value)) ens_row_kernel(const EnsMember<Real>* __restrict__ members,
                                                       const EnsItem* __restrict__ items, int nitems, int* status) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    if (block_should_exit(status)) return;
+    if (block_begin(status, nullptr).exit) return;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const EnsItem item = items[it];
         const EnsMember<Real>& mb = members[item.member];
+        const bool narrow = band_narrow(mb.row.band);
         switch (mb.n) {
 #define NS2D_ENS_ROW(NN)                                                                  \
     case NN:                                                                              \
-        row_body<Real, NN, EnsShape<NN, THREADS>::PAIRS, false>(mb.row, item.tile, smraw); \
+        row_body<Real, NN, EnsShape<NN, THREADS>::PAIRS, false>(mb.row, narrow, item.tile, smraw); \
         break;
             NS2D_ENS_SIZES(NS2D_ENS_ROW)
 #undef NS2D_ENS_ROW
@@ -180,7 +186,7 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
                      EnsStage st, EnsSync sy) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_task, s_ok;
-    if (block_should_exit(st.status)) return;
+    if (block_begin(st.status, nullptr).exit) return;
     for (;;) {
         if (threadIdx.x == 0) s_task = atomicAdd(sy.head + (st.stage - 1), 1);
         __syncthreads();
@@ -188,6 +194,7 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
         if (it >= ntasks) return;
         const EnsTask task = tasks[it];
         const EnsMember<Real>& mb = members[task.member];
+        const bool narrow = band_narrow(mb.row.band);
         // inputs of this task produced earlier in this launch
         if (threadIdx.x == 0) {
             bool ok = true;
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
             switch (mb.n) {
 #define NS2D_ENS_SROW(NN)                                                                 \
     case NN:                                                                              \
-        row_body<Real, NN, EnsShape<NN, THREADS>::PAIRS, false>(mb.row, task.tile, smraw); \
+        row_body<Real, NN, EnsShape<NN, THREADS>::PAIRS, false>(mb.row, narrow, task.tile, smraw); \
         break;
                 NS2D_ENS_SIZES(NS2D_ENS_SROW)
 #undef NS2D_ENS_SROW
@@ -215,13 +222,14 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
             EnsStage sc = st;
             if (task.kind == 0) sc.stage = 0;
             ens_apply_stage(a, mb, sc);
+            const auto begin = [&] { return BlockBegin{false, narrow}; };
             switch (mb.n) {
 #define NS2D_ENS_SCOL(NN)                                                                          \
     case NN:                                                                                       \
         if (task.kind == 0) {                                                                      \
-            col_body<Real, NN, EnsShape<NN, THREADS>::TC, COL_P1>(a, task.tile, smraw);            \
+            col_body<Real, NN, EnsShape<NN, THREADS>::TC, COL_P1>(a, begin, task.tile, smraw);            \
         } else {                                                                                   \
-            col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE>(a, task.tile, smraw);              \
+            col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE>(a, begin, task.tile, smraw);              \
         }                                                                                          \
         break;
                 NS2D_ENS_SIZES(NS2D_ENS_SCOL)

@@ -39,6 +39,10 @@ struct ns2d_handle {
     double* dscal = nullptr;   // [0] bound accumulator, [1] ticket
     unsigned long long* dmax = nullptr;
     int* dstatus = nullptr;    // [0] bits, [1] completed steps
+    int* dband = nullptr;      // band_narrow words: [0] the state, [1] the update factors
+    bool band_known = false;   // dband[0] describes the state
+    bool ffield_band = false;  // the listed forcing has modes in the columns dealiasing empties
+    bool band_forced = false;  // and the state may hold their trace
     double2* dio = nullptr;    // staging [nx][nyf] complex128
     double* ddiag = nullptr;   // measurables: DG_N totals + 8 * n_spect spectra
     double* dpart = nullptr;   // per-block partial bounds of the final column pass
@@ -108,6 +112,8 @@ ns2d_status rk4_step(ns2d_handle* h, double dt);
 ns2d_status rk4_step_loop(ns2d_handle* h, double dt);
 // Crank-Nicolson factor table for (dt, operator branch).
 ns2d_status ensure_cn(ns2d_handle* h, double dt, int branch);
+// The pass kernels' knowledge of the state's emptied columns (band_narrow).
+ns2d_status ensure_band(ns2d_handle* h);
 // Status read-back and SystemCheck after a batch of steps.
 ns2d_status check_status(ns2d_handle* h);
 // complex128 [nx][nyf] device array <-> internal [nx][ldc] field.

@@ -43,6 +43,17 @@ inline LinOp make_lin_params(const ns2d_params& p, int branch) {
     return L;
 }
 
+// First ky column the 2/3 rule empties (every kx there has k2 >= kmax_sqr); n/2+1
+// for the Hou-Li filter, which empties none.
+inline int kept_columns(int n, int dealias, int dealias_edge) {
+    const int nyf = n / 2 + 1;
+    if (dealias != 0) return nyf;
+    const int m = (int)(n / 3.0), lim = m * m + dealias_edge;
+    int kc = 0;
+    while (kc < nyf && kc * kc < lim) ++kc;
+    return kc;
+}
+
 inline bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
 // Whether the column passes may move their tiles by TMA copies: yes unless the

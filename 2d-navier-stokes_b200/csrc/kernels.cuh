@@ -9,12 +9,18 @@
 //   column pass (x direction, tiles of TC ky-columns, all kx rows):
 //     [forward x-FFT of the previous product + normalise/dealias/force/
 //      conjugacy + RK stage combine]  ->  derived spectra of the next stage
-//     input (i ky/k^2 X, -i kx/k^2 X, i kx X, i ky X)  ->  four inverse x-FFTs
+//     input  ->  four inverse x-FFTs
 //   row pass (y direction, pairs of x rows):
-//     Z1 = U + iV, Z2 = WX + iWY (Hermitian extension in y) -> two inverse
-//     y-FFTs give u, v, w_x, w_y in real space; n = u w_x + v w_y; the two
-//     rows' products are packed into one forward y-FFT and split into the two
-//     half spectra.
+//     Z1 = U + iV, Z2 = WX + iWY over all ky -> two inverse y-FFTs give u, v,
+//     w_x, w_y in real space; n = u w_x + v w_y; the rows' products go through
+//     forward y-FFTs into their half spectra.
+//
+// Z1 and Z2 are what the row pass transforms, so the column pass forms them: the
+// x-transform is linear, and with U, V Hermitian in y the negative wavenumbers
+// are Z1(x, -ky) = conj(U - iV)(x, ky).  Its four x-space fields are therefore
+//   f0 = U + iV, f1 = U - iV, f2 = WX + iWY, f3 = WX - iWY   at ky >= 0,
+// four transforms as before, and a row element is one load instead of two (row
+// pass at 1024^2 / 2048^2 FP64 19.9 / 69.3 -> 17.9 / 61.8 us with the event nodes).
 //
 // Spectral arrays are [nx][ldc] complex (row = kx index as in the reference,
 // ldc >= ny/2+1); the intermediate "x-space" arrays use the same shape with
@@ -71,7 +77,7 @@ struct ColArgs {
     C* acc;              // RK accumulator
     C* out;              // COL_STAGE: full next-stage input (explicit RK4 only), may be null
     C* rhs_store;        // any non-P1 mode: this evaluation's RHS, may be null
-    C* f0;               // COL_P1/STAGE outputs (x-space): U, V, WX, WY
+    C* f0;               // COL_P1/STAGE outputs (x-space): U+iV, U-iV, WX+iWY, WX-iWY
     C* f1;
     C* f2;
     C* f3;
@@ -82,6 +88,8 @@ struct ColArgs {
     const C* xin;        // RK4 explicit: stage input for the +D X term (stride ldc), may be null
     int ldc, nyf;
     int kmax_sqr;        // (int)(N/3)^2 for the 2/3 rule
+    int kc;              // columns ky >= kc are emptied by the dealiasing (nyf: none)
+    const int* band;     // see band_narrow
     int dealias;         // 0: 2/3, 1: Hou-Li
     int houli_int;       // integer k/(N/2) (reference quirk)
     int kolm;            // zero the kx = 0 row (2/3 + KOLM)
@@ -110,16 +118,34 @@ struct ColArgs {
     int* status;         // [0] status bits (kernels return early when set), [1] completed steps
 };
 
-// Early exit once the device status word is set (a failed SystemCheck).  One
-// thread reads the word and the block agrees on it through shared memory, so
-// every thread of a block takes the same path past the barriers that follow.
-__device__ __forceinline__ bool block_should_exit(const int* status) {
-    __shared__ int flag;
-    if (threadIdx.x == 0) flag = status ? *(volatile const int*)status : 0;
+// Whether the evaluation's input is known to be zero in the columns ky >= kc
+// that the 2/3 rule empties: band[0] is set when the state holds something there
+// (it may: the caller sets it), band[1] when an update factor there is not finite
+// (0 times it is not 0).  The x-space fields of those columns are then zero too,
+// so the passes neither form, store nor read them: a third of the columns, and a
+// third of every pass's x-space traffic.  null: not known.  Per step, FP64 / FP32:
+// 2048^2 678 / 400 -> 542 / 329 us, the 64-member FP32 ensemble 421 -> 328 us;
+// 1024^2, where the tiles fill one wave either way, 149 / 97 -> 144 / 94 us.
+__device__ __forceinline__ bool band_narrow(const int* band) { return band && (band[0] | band[1]) == 0; }
+
+// Start of a pass block: early exit once the device status word is set (a failed
+// SystemCheck), and band_narrow of the evaluation.  One thread reads the words
+// (independent loads) and the block agrees on them through shared memory, so
+// every thread takes the same path past the barriers that follow.  Once per kernel.
+struct BlockBegin {
+    bool exit, narrow;
+};
+__device__ __forceinline__ BlockBegin block_begin(const int* status, const int* band) {
+    __shared__ int flags;
+    if (threadIdx.x == 0) {
+        const int st = status ? *(volatile const int*)status : 0;
+        const int b0 = band ? band[0] : 1;
+        const int b1 = band ? band[1] : 1;
+        flags = (st != 0 ? 1 : 0) | ((b0 | b1) == 0 ? 2 : 0);
+    }
     __syncthreads();
-    const bool out = flag != 0;
-    __syncthreads();
-    return out;
+    const int f = flags;
+    return {(f & 1) != 0, (f & 2) != 0};
 }
 
 template <typename Real>
@@ -292,42 +318,35 @@ __device__ __forceinline__ Real kx_of(int m, int t, Real tr) {
 }
 
 // Derived spectra of the stage input X at (kx, ky) (solver.c:904-957), two at a
-// time: pair 0 gives u = i ky/k^2 X and v = -i kx/k^2 X (one reciprocal), pair 2
-// gives w_x = i kx X and w_y = i ky X.  Zero at the mean mode.  kx and ky are
-// integers held as reals.  RN: the products rounded before the transform's first
-// additions (the sizes that the resident kernel serves too; see mul_rn), which
-// costs the multiply-adds of that stage.
-template <bool RN, typename C>
-__device__ __forceinline__ void derived_pair(int fp, decltype(C::x) kx, decltype(C::x) ky, C X, C& a, C& b) {
+// time.  With u = i ky/k^2 X, v = -i kx/k^2 X, w_x = i kx X, w_y = i ky X and
+// q = kx + i ky:
+//   pair 0: u + i v = q (X/k^2)  and  u - i v = -conj(q) (X/k^2),
+//   pair 1: w_x + i w_y = i q X  and  w_x - i w_y = i conj(q) X.
+// Zero at the mean mode.  kx and ky are integers held as reals.
+template <typename C>
+__device__ __forceinline__ void derived_pair(int pair, decltype(C::x) kx, decltype(C::x) ky, C X, C& a, C& b) {
     using Real = decltype(C::x);
     if (kx == (Real)0 && ky == (Real)0) {
         a = cmake<C>(0, 0);
         b = a;
         return;
     }
-    Real sa, sb;
-    if (fp == 0) {
+    if (pair == 0) {
         const Real inv = inv_k2<Real>(kx * kx + ky * ky);
-        sa = ky * inv;
-        sb = -kx * inv;
-    } else {
-        sa = kx;
-        sb = ky;
+        X = cmake<C>(mul_rn(inv, X.x), mul_rn(inv, X.y));
     }
-    // i s X = (-s X.y, s X.x)
-    if constexpr (RN) {
-        a = cmake<C>(mul_rn(-sa, X.y), mul_rn(sa, X.x));
-        b = cmake<C>(mul_rn(-sb, X.y), mul_rn(sb, X.x));
-    } else {
-        a = cmake<C>(-sa * X.y, sa * X.x);
-        b = cmake<C>(-sb * X.y, sb * X.x);
-    }
+    const Real tx = mul_rn(ky, X.x), ty = mul_rn(ky, X.y);
+    const C p = cmake<C>(fma_rn(kx, X.x, -ty), fma_rn(kx, X.y, tx));  // q X
+    const C m = cmake<C>(fma_rn(kx, X.x, ty), fma_rn(kx, X.y, -tx));  // conj(q) X
+    a = pair == 0 ? p : cmake<C>(-p.y, p.x);
+    b = pair == 0 ? cmake<C>(-m.x, -m.y) : cmake<C>(-m.y, m.x);
 }
 
-// Crank-Nicolson update f w + g tot (solver.c:853).
+// Crank-Nicolson update f w + g tot (solver.c:853); the larger product is the one
+// that goes into the sum unrounded.
 template <typename C>
 __device__ __forceinline__ C cn_update(C w, C tot, decltype(C::x) f, decltype(C::x) g) {
-    return cmake<C>(fma_rn(tot.x, g, mul_rn(w.x, f)), fma_rn(tot.y, g, mul_rn(w.y, f)));
+    return cmake<C>(fma_rn(w.x, f, mul_rn(tot.x, g)), fma_rn(w.y, f, mul_rn(tot.y, g)));
 }
 
 // Derived spectra of the stage input X (pre0, [N][TC] in shared memory) and
@@ -337,24 +356,24 @@ template <typename Real, int N, int TC>
 __device__ __forceinline__ void derived_ifft(const typename Cx<Real>::T* pre0, typename Cx<Real>::T* sm,
                                           typename Cx<Real>::T* f0, typename Cx<Real>::T* f1,
                                           typename Cx<Real>::T* f2, typename Cx<Real>::T* f3, int ldc, int ky,
-                                          bool valid, int t, int c, TwSeed<typename Cx<Real>::T> seed) {
+                                          bool valid, int t, int c, const TwSeed<typename Cx<Real>::T>& seed) {
     using C = typename Cx<Real>::T;
     constexpr int T = Plan<N>::T;
     constexpr int E = N / T;
     C* outs[4] = {f0, f1, f2, f3};
     const Real tr = (Real)t, kyr = (Real)ky;
 #pragma unroll 1
-    for (int fp = 0; fp < 4; fp += 2) {
+    for (int fp = 0; fp < 2; ++fp) {
         C v[2][E];
 #pragma unroll
         for (int m = 0; m < E; ++m) {
             const int i = t + T * m;
-            derived_pair<(N <= 128)>(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+            derived_pair(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
         }
         fft_batched<N, +1, 2>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
         if (valid) {
-            C* __restrict__ o0 = outs[fp];
-            C* __restrict__ o1 = outs[fp + 1];
+            C* __restrict__ o0 = outs[2 * fp];
+            C* __restrict__ o1 = outs[2 * fp + 1];
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 o0[(size_t)(t + T * m) * ldc + ky] = v[0][m];
@@ -366,11 +385,11 @@ __device__ __forceinline__ void derived_ifft(const typename Cx<Real>::T* pre0, t
 
 // derived_ifft with TMA stores.  The three shared regions B0 = sm, B1 = sm +
 // STRIDE and B2 = pre0 (sized as an exchange buffer in this form) rotate.  The
-// first pair (U, V) transforms batched in (B0, B1) and is staged there, each
-// field stored by its own bulk-async group.  The second pair (WX, WY) runs as
-// two single transforms: WX in B2 (the stage input, free once both spectra are
-// formed), WY in B0 as soon as the U store has read it; so the first pair's
-// stores drain under the second pair's transforms and only WY's store is left
+// first pair (f0, f1) transforms batched in (B0, B1) and is staged there, each
+// field stored by its own bulk-async group.  The second pair (f2, f3) runs as
+// two single transforms: f2 in B2 (the stage input, free once both spectra are
+// formed), f3 in B0 as soon as the f0 store has read it; so the first pair's
+// stores drain under the second pair's transforms and only f3's store is left
 // to drain at the end.  Without SPLIT the second pair transforms batched in
 // (B2, B0) instead (a persistent caller's next tile overlaps the drain, and the
 // batched pair keeps the transforms' ILP).  pending: a store issued before
@@ -379,7 +398,7 @@ __device__ __forceinline__ void derived_ifft(const typename Cx<Real>::T* pre0, t
 template <typename Real, int N, int TC, bool SPLIT>
 __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typename Cx<Real>::T* sm,
                                                  const ColMaps* maps, int tile, int ky, int t, int c,
-                                                 TwSeed<typename Cx<Real>::T> seed, bool pending) {
+                                                 const TwSeed<typename Cx<Real>::T>& seed, bool pending) {
     using C = typename Cx<Real>::T;
     constexpr int T = Plan<N>::T;
     constexpr int E = N / T;
@@ -391,12 +410,12 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
     if constexpr (!SPLIT) {
         // both pairs batched, one copy of the transform code: (B0, B1), then (B2, B0)
 #pragma unroll 1
-        for (int fp = 0; fp < 4; fp += 2) {
+        for (int fp = 0; fp < 2; ++fp) {
             C v[2][E];
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const int i = t + T * m;
-                derived_pair<(N <= 128)>(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+                derived_pair(fp, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
             }
             // first pair: the accumulator store (if any) must have read B1;
             // second pair: the first pair's first field must have left B0 (at
@@ -419,9 +438,9 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
             fence_async_smem();
             __syncthreads();
             if (threadIdx.x == 0) {
-                tma_store_tile<C, N, TC>(&maps->f[fp], tile, Pa);
+                tma_store_tile<C, N, TC>(&maps->f[2 * fp], tile, Pa);
                 bulk_commit();
-                tma_store_tile<C, N, TC>(&maps->f[fp + 1], tile, Pb);
+                tma_store_tile<C, N, TC>(&maps->f[2 * fp + 1], tile, Pb);
                 bulk_commit();
             }
         }
@@ -431,7 +450,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const int i = t + T * m;
-                derived_pair<(N <= 128)>(0, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+                derived_pair(0, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
             }
             if (pending) {  // the accumulator store must have read B1
                 if (threadIdx.x == 0) bulk_wait_read_all();
@@ -456,13 +475,13 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 #pragma unroll
         for (int m = 0; m < E; ++m) {
             const int i = t + T * m;
-            derived_pair<(N <= 128)>(2, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
+            derived_pair(1, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
         }
         __syncthreads();  // every thread has read B2
 #pragma unroll 1
         for (int b = 0; b < 2; ++b) {
             C* const P = b == 0 ? B2 : B0;
-            if (b == 1) {  // the U store (the oldest group) must have read B0
+            if (b == 1) {  // the f0 store (the oldest group) must have read B0
                 if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 2;\n" ::: "memory");
                 __syncthreads();
             }
@@ -496,8 +515,13 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 // caller can run the body again on the same shared memory.  A load that does
 // not land within its bound sets status bit 8 and the body returns false (the
 // block must stop); otherwise it returns true.
-template <typename Real, int N, int TC, int MODE, bool FAST = false, bool TMA = false, bool SPLIT = false>
-__device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsigned char* smraw,
+// A tile of emptied columns (all ky >= kc) needs no
+// forward transform (its RHS is zero) and, when narrow, no inverse ones; in the
+// FAST modes there is then nothing left to do (state and accumulator stay zero).
+// begin(): the block's flags (BlockBegin) and a block barrier; called once the
+// TMA tile loads are under way, so the flags' latency runs under theirs.
+template <typename Real, int N, int TC, int MODE, bool FAST = false, bool TMA = false, bool SPLIT = false, typename Begin>
+__device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& begin, int tile, unsigned char* smraw,
                                          const ColMaps* maps = nullptr) {
     static_assert(!TMA || (FAST && MODE != COL_RHS), "TMA copies: FAST P1, STAGE and FINAL only");
     using C = typename Cx<Real>::T;
@@ -514,26 +538,67 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
     const bool valid = ky < a.nyf;
     const int kyc = valid ? ky : 0;
     const int ldc = a.ldc;
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const bool dead = tile * TC >= a.kc;
+    const auto seed = twiddle_seeds<N>(a.tw, t);
+    constexpr bool need_state = (MODE == COL_STAGE || MODE == COL_FINAL);
+    const bool need_acc = (MODE == COL_STAGE && !a.first) || (MODE == COL_FINAL && a.scheme < 2);
+    // TMA: [0] the input, [1] state and accumulator (P1: the input alone)
+    __shared__ __align__(8) unsigned long long bar_tile[2];
+    auto issue = [&] {
+        if constexpr (TMA) {
+            if (threadIdx.x == 0) {
+                constexpr unsigned tile_bytes = (unsigned)(sizeof(C) * N * TC);
+                mbar_init(&bar_tile[0]);
+                if constexpr (MODE != COL_P1) mbar_init(&bar_tile[1]);
+                mbar_expect_tx(&bar_tile[0], tile_bytes);
+                if constexpr (MODE == COL_P1) {
+                    tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_tile[0]);
+                } else {
+                    tma_load_tile<C, N, TC>(&maps->nl, tile, sm, &bar_tile[0]);
+                    mbar_expect_tx(&bar_tile[1], need_acc ? 2 * tile_bytes : tile_bytes);
+                    tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_tile[1]);
+                    if (need_acc) tma_load_tile<C, N, TC>(&maps->acc, tile, pre1, &bar_tile[1]);
+                }
+            }
+        }
+    };
+    // Waits for the loads of `bar`; false (status bit 8 set, and every copy still
+    // in flight waited for once more, bounded) when they do not land.  A block
+    // barrier after the wait: it also orders the reads before it.
+    auto landed = [&](bool late) {
+        if (__syncthreads_or(late)) {
+            if (threadIdx.x == 0) {
+                atomicOr(a.status, 8);
+                mbar_wait0(&bar_tile[0]);
+                if constexpr (MODE != COL_P1) mbar_wait0(&bar_tile[1]);
+            }
+            return false;
+        }
+        return true;
+    };
+    if (!dead) issue();
+    const BlockBegin b = begin();
+    const bool narrow = b.narrow;
+    if (b.exit) {
+        // nothing is computed, but the copies must not outlive the block
+        if constexpr (TMA) {
+            if (!dead && threadIdx.x == 0) {
+                mbar_wait0(&bar_tile[0]);
+                if constexpr (MODE != COL_P1) mbar_wait0(&bar_tile[1]);
+            }
+        }
+        return false;
+    }
+    if (dead) {
+        if ((FAST || MODE == COL_P1) && narrow) return true;
+        issue();
+        if constexpr (TMA) __syncthreads();
+    }
 
     if constexpr (MODE == COL_P1) {
         if constexpr (TMA) {
-            __shared__ __align__(8) unsigned long long bar_in;
-            if (threadIdx.x == 0) {
-                mbar_init(&bar_in);
-                mbar_expect_tx(&bar_in, (unsigned)(sizeof(C) * N * TC));
-                tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_in);
-            }
-            __syncthreads();
-            const bool late = !mbar_wait0(&bar_in);
-            if (__syncthreads_or(late)) {
-                if (threadIdx.x == 0) {
-                    atomicOr(a.status, 8);
-                    mbar_wait0(&bar_in);
-                }
-                return false;
-            }
-            if (threadIdx.x == 0) mbar_inval(&bar_in);
+            if (!landed(!mbar_wait0(&bar_tile[0]))) return false;
+            if (threadIdx.x == 0) mbar_inval(&bar_tile[0]);
         } else {
             const C* __restrict__ src = a.src;
 #pragma unroll
@@ -554,40 +619,18 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
     } else {
         const C* __restrict__ src = a.src;
         C v[1][E];
-        constexpr bool need_state = (MODE == COL_STAGE || MODE == COL_FINAL);
-        const bool need_acc = (MODE == COL_STAGE && !a.first) || (MODE == COL_FINAL && a.scheme < 2);
-        __shared__ __align__(8) unsigned long long bar_tile[2];  // TMA: [0] the input, [1] state and accumulator
         if constexpr (TMA) {
-            if (threadIdx.x == 0) {
-                mbar_init(&bar_tile[0]);
-                mbar_init(&bar_tile[1]);
-                constexpr unsigned tile_bytes = (unsigned)(sizeof(C) * N * TC);
-                mbar_expect_tx(&bar_tile[0], tile_bytes);
-                tma_load_tile<C, N, TC>(&maps->nl, tile, sm, &bar_tile[0]);
-                mbar_expect_tx(&bar_tile[1], need_acc ? 2 * tile_bytes : tile_bytes);
-                tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_tile[1]);
-                if (need_acc) tma_load_tile<C, N, TC>(&maps->acc, tile, pre1, &bar_tile[1]);
-            }
-            __syncthreads();
             const bool late = !mbar_wait0(&bar_tile[0]);
 #pragma unroll
             for (int m = 0; m < E; ++m) v[0][m] = sm[(t + T * m) * TC + c];
             // every thread has its input before the transform reuses the buffer
-            if (__syncthreads_or(late)) {
-                if (threadIdx.x == 0) {
-                    // once more, bounded, for the copies still in flight
-                    atomicOr(a.status, 8);
-                    mbar_wait0(&bar_tile[0]);
-                    mbar_wait0(&bar_tile[1]);
-                }
-                return false;
-            }
+            if (!landed(late)) return false;
             if (threadIdx.x == 0) mbar_inval(&bar_tile[0]);
         } else {
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const int i = t + T * m;
-                v[0][m] = valid ? src[(size_t)i * ldc + kyc] : cmake<C>(0, 0);
+                v[0][m] = valid && !dead ? src[(size_t)i * ldc + kyc] : cmake<C>(0, 0);
             }
         }
         // prefetch the epilogue operands while the forward transform runs
@@ -613,30 +656,103 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
                 for (int m = 0; m < E; ++m) prefetch_l2(a.cn + (size_t)(t + T * m) * ldc + ky);
             }
         }
-        fft_batched<N, -1, 1>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
+        if (FAST || !dead) fft_batched<N, -1, 1>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
+        double bsum = 0.0;
+        bool bad = false;
+        if constexpr (FAST) {
+            // The common step's epilogue, straight from the transform's registers.
+            // Operands come in batches that are read before any result of the batch
+            // is written (a load after a store to shared memory would wait for it).
+            // Stage pass at 1024^2 FP64, transform to transform: 4,540 -> 3,200 cycles;
+            // final pass at 256^2 13.8 -> 9.6 us.
+            if constexpr (TMA) {
+                if (!landed(!mbar_wait0(&bar_tile[1]))) return false;
+                if (threadIdx.x == 0) mbar_inval(&bar_tile[1]);
+            } else {
+                cp_async_wait_all();
+            }
+#pragma unroll
+            for (int m = 0; m < E; ++m) {
+                const int i = t + T * m;
+                const int kx = (i <= N / 2) ? i : i - N;
+                // normalisation and zero mean (solver.c:998-1013), 2/3 mask (solver.c:1039-1099)
+                const bool zero = (m == 0 && i == 0 && ky == 0) || kx * kx + ky * ky >= a.kmax_sqr || (a.kolm && kx == 0);
+                v[0][m] = zero ? cmake<C>(0, 0) : cscale(v[0][m], a.norm2);
+            }
+            // forcing (solver.c:1022-1027)
+            if (a.has_force && ky == a.force_j) {
+#pragma unroll
+                for (int m = 0; m < E; ++m)
+                    if (t + T * m == a.force_i) v[0][m] = cadd(v[0][m], a.force_val);
+            }
+            // ForceConjugacy side effect on the state (solver.c:1031, 2096-2103)
+            if (a.conj_mode && ky == 0) {
+#pragma unroll
+                for (int m = E / 2; m < E; ++m) {
+                    const int i = t + T * m;
+                    if (i > N / 2) {
+                        const C w = cconj(a.conj_src[(size_t)(N - i) * a.conj_stride]);
+                        pre0[i * TC + c] = w;
+                        // (the TMA final pass stores this element's update through the tile copy)
+                        if constexpr (!(TMA && MODE == COL_FINAL)) a.state[(size_t)i * ldc] = w;
+                    }
+                }
+            }
+            constexpr int EB = E < 4 ? E : (MODE == COL_FINAL && E >= 8) ? 8 : 4;
+            const Real bc = (Real)a.b_cur;
+            const Real adt = (Real)(a.dt * a.a_next);
+#pragma unroll
+            for (int m0 = 0; m0 < E; m0 += EB) {
+                C w[EB], acc[EB];
+                double2 f[MODE == COL_FINAL ? EB : 1];
+                if constexpr (MODE == COL_FINAL) {
+                    // Crank-Nicolson factors (solver.c:853), from the table
+#pragma unroll
+                    for (int m = 0; m < EB; ++m) f[m] = a.cn[(size_t)(t + T * (m0 + m)) * ldc + kyc];
+                }
+#pragma unroll
+                for (int m = 0; m < EB; ++m) {
+                    const int q = (t + T * (m0 + m)) * TC + c;
+                    w[m] = pre0[q];
+                    if (MODE == COL_FINAL || !a.first) acc[m] = pre1[q];
+                }
+#pragma unroll
+                for (int m = 0; m < EB; ++m) {
+                    const int i = t + T * (m0 + m);
+                    const int q = i * TC + c;
+                    const C r = v[0][m0 + m];
+                    if constexpr (MODE == COL_STAGE) {
+                        const C ac = a.first ? cscale(r, bc) : cadd(acc[m], cscale(r, bc));
+                        if constexpr (TMA) pre1[q] = ac;  // staged for the tile store
+                        else if (valid) a.acc[(size_t)i * ldc + ky] = ac;
+                        pre0[q] = cadd(w[m], cscale(r, adt));
+                    } else {
+                        C wn = cn_update<C>(w[m], cadd(acc[m], cscale(r, bc)), (Real)f[m].x, (Real)f[m].y);
+                        if (m0 + m == 0 && i == 0 && ky == 0) wn = cmake<C>(0, 0);
+                        if constexpr (TMA) pre0[q] = wn;  // staged for the tile store
+                        else if (valid) a.state[(size_t)i * ldc + ky] = wn;
+                        if (valid) {
+                            const double mag = fabs((double)wn.x) + fabs((double)wn.y);
+                            bad |= !isfinite(mag);
+                            bsum += (ky == 0 || 2 * ky == N) ? mag : 2.0 * mag;
+                        }
+                    }
+                }
+            }
+            if constexpr (MODE == COL_STAGE) {
+                if (ky == 0) {
+#pragma unroll
+                    for (int m = 0; m < E; ++m) a.col0_out[t + T * m] = pre0[(t + T * m) * TC + c];
+                }
+            }
+        } else {
         // The epilogue runs as a rolled loop over this thread's elements (one
         // copy of its code): the transform output is parked in the exchange
         // buffer, in slots only this thread touches.
 #pragma unroll
         for (int m = 0; m < E; ++m) sm[(t + T * m) * TC + c] = v[0][m];
-        if constexpr (TMA) {
-            const bool late = !mbar_wait0(&bar_tile[1]);
-            if (__syncthreads_or(late)) {
-                if (threadIdx.x == 0) {
-                    atomicOr(a.status, 8);
-                    mbar_wait0(&bar_tile[1]);  // once more, bounded, for the copies still in flight
-                }
-                return false;
-            }
-            if (threadIdx.x == 0) mbar_inval(&bar_tile[1]);
-        } else if constexpr (need_state) {
-            cp_async_wait_all();
-        }
-        double bsum = 0.0;
-        bool bad = false;
-        // FAST: fully unrolled (its epilogue is short enough); else four at a time
-        constexpr int EU = FAST ? E : 4;
-#pragma unroll EU
+        if constexpr (need_state) cp_async_wait_all();
+#pragma unroll 4
         for (int m = 0; m < E; ++m) {
             const int i = t + T * m;
             const int q = i * TC + c;
@@ -745,6 +861,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
                 }
             }
         }
+        }
         // the next transform's first stage writes other threads' parked slots
         if constexpr (TMA) fence_async_smem();
         __syncthreads();
@@ -802,6 +919,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
         if constexpr (MODE == COL_RHS) return true;
     }
 
+    if (!FAST && dead && narrow) return true;
     if constexpr (TMA) derived_ifft_tma<Real, N, TC, SPLIT>(pre0, sm, maps, tile, ky, t, c, seed, MODE == COL_STAGE);
     else derived_ifft<Real, N, TC>(pre0, sm, a.f0, a.f1, a.f2, a.f3, ldc, ky, valid, t, c, seed);
     return true;
@@ -814,8 +932,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, int tile, unsig
 template <typename Real, int N, int TC, int MODE, bool FAST = false>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_kernel(ColArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    if (block_should_exit(a.status)) return;
-    col_body<Real, N, TC, MODE, FAST>(a, blockIdx.x, smraw);
+    col_body<Real, N, TC, MODE, FAST>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, smraw);
 }
 
 // Column pass with TMA tile loads and stores (FAST P1, STAGE and FINAL).  Shared
@@ -823,9 +940,8 @@ __global__ void __launch_bounds__(Plan<N>::T * TC) col_kernel(ColArgs<Real> a) {
 template <typename Real, int N, int TC, int MODE>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_tma_kernel(ColArgs<Real> a, const __grid_constant__ ColMaps maps) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    if (block_should_exit(a.status)) return;
     unsigned char* sm = smraw + ((1024u - ((unsigned)__cvta_generic_to_shared(smraw) & 1023u)) & 1023u);
-    col_body<Real, N, TC, MODE, true, true, true>(a, blockIdx.x, sm, &maps);
+    col_body<Real, N, TC, MODE, true, true, true>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, sm, &maps);
 }
 
 // Whether a stage or final column pass can run the FAST epilogue.
@@ -838,14 +954,16 @@ inline bool col_fast_ok(const ColArgs<Real>& a) {
 template <typename Real>
 struct RowArgs {
     using C = typename Cx<Real>::T;
-    const C* f0;  // U(x, ky)
-    const C* f1;  // V
-    const C* f2;  // WX
-    const C* f3;  // WY
+    const C* f0;  // (U + iV)(x, ky)
+    const C* f1;  // U - iV
+    const C* f2;  // WX + iWY
+    const C* f3;  // WX - iWY
     C* nl;        // product spectrum n(x, ky)
     const C* tw;
     int ldc;
     int nrows;
+    int kc;           // columns of the product that survive dealiasing (only they are stored)
+    const int* band;  // see band_narrow
     int* status;
     C* cap_uv;    // optional capture of the real fields: (u, v) and (w_x, w_y) as
     C* cap_w;     // complex pairs, [x][y] (adjoint stage recomputation); null = off
@@ -874,8 +992,9 @@ constexpr int half_plan_width() {
 // transforms together; rows 2p and 2p+1 then share one packed forward
 // transform, done by team 2p alone when teams are whole warps (team 2p+1
 // leaves) and by both teams, each keeping its half, below a warp.
+// narrow: band_narrow(a.band), the fields are zero (and not stored) from ky = kc on.
 template <typename Real, int N, int PAIRS, bool CAP = true>
-__device__ __forceinline__ void row_body(const RowArgs<Real>& a, int rblock, unsigned char* smraw) {
+__device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, int rblock, unsigned char* smraw) {
     using C = typename Cx<Real>::T;
     using P = Plan<N>;
     constexpr int T = P::T;
@@ -887,31 +1006,43 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, int rblock, uns
     const int t = threadIdx.x % T;
     const int x = rblock * TC + g;
     C* region = reinterpret_cast<C*>(smraw) + (size_t)g * RS::TEAM;
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N>(a.tw, t);
     const TeamPolicy<N, C> pol{region, 1 + g};
 
-    // Z1 = U + i V and Z2 = WX + i WY over the full y range (Hermitian
-    // extension; DC and Nyquist use the real parts only, as FFTW's c2r does)
+    // Z1 = U + i V and Z2 = WX + i WY over the full y range; at DC and Nyquist
+    // from the real parts of U, V, WX and WY only, as FFTW's c2r reads them
     C v[2][E];
     {
-        const C* __restrict__ U = a.f0 + (size_t)x * a.ldc;
-        const C* __restrict__ V = a.f1 + (size_t)x * a.ldc;
-        const C* __restrict__ WX = a.f2 + (size_t)x * a.ldc;
-        const C* __restrict__ WY = a.f3 + (size_t)x * a.ldc;
+        const int cols = narrow ? a.kc : N / 2 + 1;
+        const C* __restrict__ P1 = a.f0 + (size_t)x * a.ldc;
+        const C* __restrict__ M1 = a.f1 + (size_t)x * a.ldc;
+        const C* __restrict__ P2 = a.f2 + (size_t)x * a.ldc;
+        const C* __restrict__ M2 = a.f3 + (size_t)x * a.ldc;
 #pragma unroll
         for (int m = 0; m < E; ++m) {
             const int y = t + T * m;
             const int yy = (y <= N / 2) ? y : N - y;
-            const C p0 = U[yy], q0 = V[yy], p1 = WX[yy], q1 = WY[yy];
-            if (y == 0 || y == N / 2) {
-                v[0][m] = cmake<C>(p0.x, q0.x);
-                v[1][m] = cmake<C>(p1.x, q1.x);
-            } else if (y < N / 2) {
-                v[0][m] = cmake<C>(p0.x - q0.y, p0.y + q0.x);
-                v[1][m] = cmake<C>(p1.x - q1.y, p1.y + q1.x);
-            } else {
-                v[0][m] = cmake<C>(p0.x + q0.y, q0.x - p0.y);
-                v[1][m] = cmake<C>(p1.x + q1.y, q1.x - p1.y);
+            v[0][m] = v[1][m] = cmake<C>(0, 0);
+            if (yy < cols) {
+                if (y <= N / 2) {
+                    v[0][m] = P1[yy];
+                    v[1][m] = P2[yy];
+                } else {
+                    v[0][m] = cconj(M1[yy]);
+                    v[1][m] = cconj(M2[yy]);
+                }
+            }
+        }
+        if (t == 0) {
+            static_assert((N / 2) % T == 0, "DC and Nyquist belong to thread 0");
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int m = h * (N / 2 / T);
+                if (h * (N / 2) < cols) {
+                    const C m1 = M1[h * (N / 2)], m2 = M2[h * (N / 2)];
+                    v[0][m] = cmake<C>((Real)0.5 * (v[0][m].x + m1.x), (Real)0.5 * (v[0][m].y - m1.y));
+                    v[1][m] = cmake<C>((Real)0.5 * (v[1][m].x + m2.x), (Real)0.5 * (v[1][m].y - m2.y));
+                }
             }
         }
     }
@@ -957,12 +1088,13 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, int rblock, uns
 #pragma unroll
         for (int m = 0; m < EH; ++m) {
             const int k = t + T * m;
+            if (k >= a.kc) continue;
             const C zk = z[0][m];
             const C zm = region[TLH::slot((NH - k) & (NH - 1))];
             const C ev = cmake<C>((Real)0.5 * (zk.x + zm.x), (Real)0.5 * (zk.y - zm.y));
             const C od = cmake<C>((Real)0.5 * (zk.y + zm.y), (Real)0.5 * (zm.x - zk.x));
             dst[k] = cadd(ev, cmul(__ldg(a.tw + k), od));
-            if (k == 0) dst[NH] = cmake<C>(zk.x - zk.y, (Real)0);  // W^(N/2) = -1
+            if (k == 0 && NH < a.kc) dst[NH] = cmake<C>(zk.x - zk.y, (Real)0);  // W^(N/2) = -1
         }
     } else {
     __syncthreads();
@@ -988,7 +1120,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, int rblock, uns
 #pragma unroll
     for (int m = 0; m < E; ++m) {
         const int k = t + T * m;
-        if (k <= N / 2) {
+        if (k < a.kc) {  // kc <= N/2 + 1
             const C zk = region[TL::slot(k)];
             const C zm = region[TL::slot((N - k) & (N - 1))];
             const C ra = cmake<C>((Real)0.5 * (zk.x + zm.x), (Real)0.5 * (zk.y - zm.y));
@@ -1012,13 +1144,16 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, int rblock, uns
 template <typename Real, int N, int PAIRS, bool CAP = true>
 __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) row_kernel(RowArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    if (block_should_exit(a.status)) return;
-    row_body<Real, N, PAIRS, CAP>(a, blockIdx.x, smraw);
+    const BlockBegin b = block_begin(a.status, a.band);
+    if (b.exit) return;
+    row_body<Real, N, PAIRS, CAP>(a, b.narrow, blockIdx.x, smraw);
 }
 
 // Crank-Nicolson factors per mode for the current dt and operator branch:
 // cn = ((2 - D)/(2 + D), 2 dt/(2 + D)), D = dt * bracket(|k|^2) (solver.c:839-853).
-static __global__ void cn_table_kernel(double2* cn, int nx, int nyf, int ldc, double dt, LinOp lin) {
+// *odd (cleared by the caller) is set when a factor in the columns ky >= kc is
+// not finite.
+static __global__ void cn_table_kernel(double2* cn, int nx, int nyf, int ldc, double dt, LinOp lin, int kc, int* odd) {
     const long long n = (long long)nx * nyf;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(q / nyf), ky = (int)(q % nyf);
@@ -1028,9 +1163,25 @@ static __global__ void cn_table_kernel(double2* cn, int nx, int nyf, int ldc, do
         if (kx != 0 || ky != 0) {
             const double D = dt * lin_bracket(lin, k2);
             f = make_double2((2.0 - D) / (2.0 + D), (2.0 * dt) / (2.0 + D));
+            if (ky >= kc && !(isfinite(f.x) && isfinite(f.y))) atomicOr(odd, 1);
         }
         cn[(size_t)i * ldc + ky] = f;
     }
+}
+
+// *flag (cleared by the caller) is set when the state holds anything but zeros in
+// the columns ky >= kc.
+template <typename Real>
+__global__ void __launch_bounds__(256) band_scan_kernel(const typename Cx<Real>::T* __restrict__ state, int nx, int nyf,
+                                                        int ldc, int kc, int* flag) {
+    const int w = nyf - kc;
+    const long long n = (long long)nx * w;
+    bool any = false;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const auto z = state[(size_t)(q / w) * ldc + kc + (size_t)(q % w)];
+        any |= !(z.x == 0 && z.y == 0);
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(flag, 1);
 }
 
 }  // namespace ns2d

@@ -21,6 +21,7 @@
 
 #include "../../include/ns2d.h"
 #include "engine.cuh"
+#include "host_common.h"
 
 using namespace ns2d;
 
@@ -146,6 +147,7 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
     a.nyf = nyf;
     const int m = (int)(n / 3.0);
     a.kmax_sqr = m * m + (p->dealias_edge ? 1 : 0);
+    a.kc = kept_columns(n, p->dealias, p->dealias_edge);
     a.dealias = p->dealias;
     a.houli_int = (p->quirks & NS2D_QUIRK_HOU_LI_INT) ? 1 : 0;
     a.kolm = (p->forcing == NS2D_FORCING_KOLM) ? 1 : 0;
@@ -168,6 +170,7 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
     r.tw = tw;
     r.ldc = nyf;
     r.nrows = n;
+    r.kc = a.kc;
     r.status = nullptr;
     with_small_size(n, [&](auto L) { decltype(L)::row(r, st); });
 

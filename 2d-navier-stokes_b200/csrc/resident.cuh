@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
     const int t = threadIdx.x % T;
     const int team = threadIdx.x / T;
     const int warp_team = (threadIdx.x & ~31) / T;  // first team of this warp
-    const TwSeed<C> seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N>(a.tw, t);
     const TeamPolicy<N, C> pol{sm + L::REG + team * TeamLayout<N>::ROWS, 0};
     constexpr bool rhs_only = SCHEME == RES_RHS;
     constexpr bool ab4 = SCHEME == RES_AB4;
@@ -249,18 +249,20 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
                 const bool on = u < 4 * slots;
                 const int slot = on ? u >> 2 : 0, f = u & 3;
                 const int ky = rank + CL * slot;
-                // the field's multiplier i sc (derived_pair): ky/k^2, -kx/k^2, kx, ky
-                const Real tr = (Real)t, kyr = (Real)ky;
+                // the field's derived spectrum (derived_pair): f & 1 the conj(q) ones
+                const Real tr = (Real)t;
+                const Real kys = (f & 1) ? -(Real)ky : (Real)ky;
                 C v[1][E];
 #pragma unroll
                 for (int m = 0; m < E; ++m) {
                     const int q = slot * N + t + T * m;
-                    const C X = sX[q];
                     const Real kx = kx_of<Real, N, T>(m, t, tr);
-                    const Real num = (f == 0 || f == 3) ? kyr : f == 1 ? -kx : kx;
-                    const Real sc = f < 2 ? num * sI[q] : num;
-                    const bool mean = m == 0 && t == 0 && ky == 0;
-                    v[0][m] = mean ? cmake<C>(0, 0) : cmake<C>(mul_rn(-sc, X.y), mul_rn(sc, X.x));
+                    const Real sc = f < 2 ? sI[q] : (Real)1;
+                    C X = sX[q];
+                    X = cmake<C>(mul_rn(sc, X.x), mul_rn(sc, X.y));
+                    const C d = cmake<C>(fma_rn(kx, X.x, -mul_rn(kys, X.y)), fma_rn(kx, X.y, mul_rn(kys, X.x)));
+                    v[0][m] = f >= 2 ? cmake<C>(-d.y, d.x) : f == 1 ? cmake<C>(-d.x, -d.y) : d;
+                    if (m == 0 && t == 0 && ky == 0) v[0][m] = cmake<C>(0, 0);
                 }
                 fft_batched<N, +1, 1>(v, pol, seed, t);
                 if (on) {
@@ -280,7 +282,7 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
                 for (int r = 0; r < CL; ++r) stop |= s_stop[r] != 0;
                 if (stop) break;  // the same in every block
             }
-            // --- rows: inverse y-FFTs of Z1 = U + iV and Z2 = WX + iWY
+            // --- rows: inverse y-FFTs of Z1 = U + iV and Z2 = WX + iWY (fields as the passes')
             for (int u0 = 0; u0 + warp_team < 2 * RPC; u0 += L::TEAMS) {
                 const int u = u0 + team;
                 const bool on = u < 2 * RPC;
@@ -290,14 +292,16 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
                 for (int m = 0; m < E; ++m) {
                     const int y = t + T * m;
                     const int yy = (y <= N / 2) ? y : N - y;
-                    C p = cmake<C>(0, 0), q = p;
+                    const C* const plus = sF + (size_t)yy * L::KS + (2 * b) * RPC + g;
+                    C p = cmake<C>(0, 0);
                     if (yy < kx_cols) {
-                        p = sF[(size_t)yy * L::KS + (2 * b) * RPC + g];
-                        q = sF[(size_t)yy * L::KS + (2 * b + 1) * RPC + g];
+                        p = y <= N / 2 ? plus[0] : cconj(plus[RPC]);
+                        if (y == 0 || y == N / 2) {
+                            const C q = plus[RPC];
+                            p = cmake<C>((Real)0.5 * (p.x + q.x), (Real)0.5 * (p.y - q.y));
+                        }
                     }
-                    if (y == 0 || y == N / 2) v[0][m] = cmake<C>(p.x, q.x);
-                    else if (y < N / 2) v[0][m] = cmake<C>(p.x - q.y, p.y + q.x);
-                    else v[0][m] = cmake<C>(p.x + q.y, q.x - p.y);
+                    v[0][m] = p;
                 }
                 fft_batched<N, +1, 1>(v, pol, seed, t);
                 // n = u w_x + v w_y: the row's two teams (neighbours in the warp)

@@ -1,0 +1,120 @@
+"""The pass kernels leave out the columns that the 2/3 rule empties when the
+state holds nothing there, and must take them back in when it does: states set
+from outside with content past the circle (a whole spectrum, or one mode in the
+first emptied column), a forced mode there, changes from one kind to the other
+on one handle, ensembles of both kinds, and a reverse sweep after the state was
+replaced.  Against the oracle, FP64, to the parity tests' 1e-12 of max|w_hat|."""
+import numpy as np
+import pytest
+
+from _util import rel_err
+from ns2d import Ensemble, Solver, abi, initial
+from pyoracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(n, kind, seed=3):
+    w = initial.decaying(n, seed=seed, k0=n / 16.0, dealias="2/3")
+    top = np.abs(w).max()
+    if kind == "wide":
+        w = w + initial.hermitian(np.full_like(w, 1e-3 * top))
+    elif kind == "edge":  # ky = int(n/3), the first column with no kept mode
+        w[5, int(n / 3.0)] = 0.05 * top * (1 + 2j)
+    return w
+
+
+def _oracle(p, w0, steps, dt):
+    o = Oracle(p, threads=8)
+    o.set_w_hat(w0)
+    for k in range(steps):
+        if p.integrator == abi.AB4:
+            o.ab4_step(dt, k + 1)
+        else:
+            o.compute_forcing(dt)
+            o.rk4_step(dt)
+    return o.get_w_hat()
+
+
+@pytest.mark.parametrize("kind", ["narrow", "edge", "wide"])
+@pytest.mark.parametrize("integ", [abi.RK4CN, abi.RK4, abi.AB4])
+@pytest.mark.parametrize("n", [256, 512, 1024])
+def test_steps_match_oracle(n, integ, kind):
+    dt, steps = 1e-4, 5
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, ekmn_drag_flag=1, integrator=integ, dt=dt)
+    w0 = _state(n, kind)
+    s = Solver(p)
+    s.set_w_hat(w0)
+    s.step_n(steps, dt)
+    assert rel_err(s.get_w_hat(), _oracle(p, w0, steps, dt)) <= 1e-12
+    assert rel_err(s.nonlinear_rhs(w0), _rhs(p, w0)) <= 1e-12
+    s.close()
+
+
+def _rhs(p, w):
+    o = Oracle(p, threads=8)
+    o.set_w_hat(w)
+    return o.nonlinear_rhs(w)
+
+
+def test_one_handle_changes_kind():
+    n, dt = 256, 2e-4
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, ekmn_drag_flag=1, dt=dt)
+    s = Solver(p)
+    for k, kind in enumerate(["narrow", "edge", "narrow", "wide", "narrow"]):
+        w0 = _state(n, kind, seed=20 + k)
+        s.set_w_hat(w0)
+        s.step_n(4, dt)  # the step graph stays captured across the changes
+        assert rel_err(s.get_w_hat(), _oracle(p, w0, 4, dt)) <= 1e-12, (k, kind)
+    for k, kind in enumerate(["edge", "narrow", "wide"]):
+        w0 = _state(n, kind, seed=30 + k)
+        w = w0.copy()
+        for _ in range(3):
+            s.rk4_step_host(w, dt)
+        assert rel_err(w, _oracle(p, w0, 3, dt)) <= 1e-12, (k, kind)
+    s.close()
+
+
+def test_forced_mode_past_the_circle():
+    n, dt = 256, 1e-3
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, ekmn_drag_flag=1, dt=dt, forcing=abi.FORCING_KOLM, force_k=n // 2 - 3,
+                           force_scale=50.0)
+    w0 = _state(n, "narrow")
+    s = Solver(p)
+    s.set_w_hat(w0)
+    s.step_n(6, dt)
+    assert rel_err(s.get_w_hat(), _oracle(p, w0, 6, dt)) <= 1e-12
+
+
+def test_ensemble_of_both_kinds():
+    sizes, kinds, dt = [256, 512, 64, 256, 128], ["edge", "narrow", "wide", "narrow", "edge"], 2e-4
+    p = abi.default_params(nu=1e-3, ekmn_drag_flag=1, dt=dt)
+    w0 = [_state(n, k, seed=m) for m, (n, k) in enumerate(zip(sizes, kinds))]
+    e = Ensemble(p, sizes)
+    for stage_launch in (0, 1):
+        e.set_shape(stage_launch=stage_launch)
+        for m, w in enumerate(w0):
+            e.set_w_hat(m, w)
+        e.step_n(4, dt)
+        for m, n in enumerate(sizes):
+            q = p.copy()
+            q.nx = q.ny = n
+            assert rel_err(e.get_w_hat(m), _oracle(q, w0[m], 4, dt)) <= 1e-12, (stage_launch, m)
+    e.close()
+
+
+def test_reverse_sweep_after_the_state_was_replaced():
+    n, dt = 256, 1e-3
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, quirks=0, dt=dt)
+    lam = initial.decaying(n, 8, k0=5.0, dealias="2/3")
+    grads = []
+    for replace in (False, True):
+        s = Solver(p)
+        s.set_w_hat(_state(n, "edge"))
+        s.adjoint_record(6, dt, 3)
+        if replace:
+            s.set_w_hat(_state(n, "narrow"))
+            s.step_n(2, dt)
+        grads.append(s.adjoint_backward(lam))
+        s.close()
+    assert np.array_equal(grads[0], grads[1])
