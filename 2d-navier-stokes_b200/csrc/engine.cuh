@@ -7,15 +7,19 @@
 namespace ns2d {
 
 // Column-tile width (ky columns per block) and row pairs per block.  Column
-// accesses fetch TC * 16 B per row, so wider tiles use each row's cache line
-// better; at 512 and 1024 four columns per block measured faster than two
-// (even with fewer blocks than SMs at 1024), so they get TC = 4.
+// accesses fetch TC * 16 B per row in FP64, so wider tiles use each row's lines
+// better, while narrower ones spread a pass over more SMs.  With the emptied
+// columns left out a pass at 256 has 86 columns and at 512 171: two to a block
+// there (a step at 512^2 FP64 57.4 us against 68.2 with four; one: 57.5; at 256^2
+// 43.2 against 47.2 with four), four at 1024 (three: 153.6 us against 144.2, the
+// six warps weigh on the four schedulers as eight do and the 48-byte rows break
+// sectors; two: 141.8, but 4 us more for the final pass).
 template <typename Real, int N>
 struct Shape {
     static constexpr int T = Plan<N>::T;
     static constexpr int TC_RAW = 128 / T < 2 ? 2 : 128 / T;
-    static constexpr int TC = (N == 16) ? 8 : (N == 512 || N == 1024) ? 4 : TC_RAW;
-    static constexpr int PAIRS_RAW = (128 / T) / 2 < 1 ? 1 : (128 / T) / 2;
+    static constexpr int TC = (N == 16) ? 8 : (N == 1024) ? 4 : (N == 256) ? 2 : TC_RAW;
+    static constexpr int PAIRS_RAW = (N == 256) ? 1 : (128 / T) / 2 < 1 ? 1 : (128 / T) / 2;
     static constexpr int PAIRS = PAIRS_RAW > N / 2 ? N / 2 : PAIRS_RAW;
 };
 

@@ -150,13 +150,16 @@ template <int R, int SIGN, typename C>
 __device__ __forceinline__ void small_dft(C* v) { SmallDFT<R, SIGN, 1, C>::run(v); }
 
 // Plans: first and last radix equal, one butterfly per thread at both ends.
+// 256 as 8 x 4 x 8 by a warp (a step at 256^2 FP64 43 us) rather than 16 x 16 by 16
+// threads (60 us): the passes of one such grid fill few SMs, so what counts is
+// how long a thread's own instruction stream is.
 template <int N>
 struct Plan;
 template <> struct Plan<16>   { static constexpr int T = 4,   S = 2, R0 = 4,  R1 = 4,  R2 = 1; };
 template <> struct Plan<32>   { static constexpr int T = 8,   S = 3, R0 = 4,  R1 = 2,  R2 = 4; };
 template <> struct Plan<64>   { static constexpr int T = 8,   S = 2, R0 = 8,  R1 = 8,  R2 = 1; };
 template <> struct Plan<128>  { static constexpr int T = 16,  S = 3, R0 = 8,  R1 = 2,  R2 = 8; };
-template <> struct Plan<256>  { static constexpr int T = 16,  S = 2, R0 = 16, R1 = 16, R2 = 1; };
+template <> struct Plan<256>  { static constexpr int T = 32,  S = 3, R0 = 8,  R1 = 4,  R2 = 8; };
 template <> struct Plan<512>  { static constexpr int T = 64,  S = 3, R0 = 8,  R1 = 8,  R2 = 8; };
 template <> struct Plan<1024> { static constexpr int T = 64,  S = 3, R0 = 16, R1 = 4,  R2 = 16; };
 template <> struct Plan<2048> { static constexpr int T = 128, S = 3, R0 = 16, R1 = 8,  R2 = 16; };
@@ -298,7 +301,7 @@ struct TeamLayout {
 
 template <int T>
 __device__ __forceinline__ void team_sync(int bar) {
-    if constexpr (T >= 32) {
+    if constexpr (T > 32) {
         asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "r"(T) : "memory");
     } else {
         __syncwarp();
