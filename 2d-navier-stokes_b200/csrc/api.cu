@@ -56,13 +56,6 @@ LinOp make_lin(const ns2d_handle* h, int branch) { return make_lin_params(h->p, 
 bool quirk(const ns2d_handle* h, int bit) { return (h->p.quirks & bit) != 0; }
 
 template <typename Real>
-int col_tc(int n) {
-    int tc = 0;
-    with_size<Real>(n, [&](auto L) { tc = decltype(L)::S::TC; });
-    return tc;
-}
-
-template <typename Real>
 using Cplx = typename Cx<Real>::T;
 
 template <typename Real>
@@ -83,6 +76,7 @@ void fill_common(ns2d_handle* h, ColArgs<Real>& a, int branch) {
     a.kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
     a.band = h->dband;
     a.dealias = h->p.dealias;
+    a.filt = (const Real*)h->filt;
     a.houli_int = quirk(h, NS2D_QUIRK_HOU_LI_INT) ? 1 : 0;
     a.kolm = (h->p.forcing == NS2D_FORCING_KOLM) ? 1 : 0;
     a.has_force = h->forced ? 1 : 0;
@@ -96,7 +90,7 @@ void fill_common(ns2d_handle* h, ColArgs<Real>& a, int branch) {
     a.status = h->dstatus;
     a.final_tail = 1;
     a.force_field = h->ffield_on ? (const C*)h->ffield : nullptr;
-    a.ntiles = (h->nyf + col_tc<Real>(h->nx) - 1) / col_tc<Real>(h->nx);
+    a.ntiles = (h->nyf + engine_ops<Real>(h->nx)->tc - 1) / engine_ops<Real>(h->nx)->tc;
     a.lin = make_lin(h, branch);
     a.phase_only = h->p.model == NS2D_MODEL_PHASE_ONLY ? 1 : 0;
 }
@@ -174,7 +168,7 @@ struct TimedLaunch {
 template <typename Real>
 void build_col_maps(ns2d_handle* h) {
     if (!tma_copies_enabled()) return;
-    const int tc = col_tc<Real>(h->nx);
+    const int tc = engine_ops<Real>(h->nx)->tc;
     auto* m = new (std::nothrow) ColMaps;
     if (!m) return;
     void* const bases[7] = {h->f[0], h->f[1], h->f[2], h->f[3], h->acc, h->state, h->nl};
@@ -188,7 +182,8 @@ void build_col_maps(ns2d_handle* h) {
 // The TMA maps when the pass reads and writes exactly the arrays they describe.
 template <typename Real>
 const ColMaps* col_maps_for(const ns2d_handle* h, int mode, const ColArgs<Real>& a) {
-    if (!h->col_maps || mode == COL_RHS) return nullptr;
+    if (!h->col_maps) return nullptr;
+    if (mode == COL_RHS) return a.src == h->nl ? static_cast<const ColMaps*>(h->col_maps) : nullptr;
     if (mode == COL_P1)
         return a.src == h->state && a.f0 == h->f[0] && a.f1 == h->f[1] && a.f2 == h->f[2] && a.f3 == h->f[3]
                    ? static_cast<const ColMaps*>(h->col_maps)
@@ -199,10 +194,10 @@ const ColMaps* col_maps_for(const ns2d_handle* h, int mode, const ColArgs<Real>&
 }
 
 template <typename Real>
-void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a) {
+void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a, int scheme = SCH_CN) {
     TimedLaunch t(h, mode == COL_STAGE ? 1 : mode == COL_FINAL ? 2 : 0);
     const ColMaps* maps = col_maps_for<Real>(h, mode, a);
-    with_size<Real>(h->nx, [&](auto L) { decltype(L)::col(mode, a, h->stream, maps); });
+    engine_ops<Real>(h->nx)->col(mode, scheme, a, h->stream, maps);
 }
 // Row pass of stage `stage` (1..4); with a capture target set, the stage's real
 // fields go to planes 2(stage-1) and 2(stage-1)+1 of it.
@@ -216,7 +211,7 @@ void launch_row(ns2d_handle* h, int stage = 0, bool use_band = true) {
         r.cap_uv = (Cplx<Real>*)h->cap_step + (size_t)(2 * (stage - 1)) * plane;
         r.cap_w = r.cap_uv + plane;
     }
-    with_size<Real>(h->nx, [&](auto L) { decltype(L)::row(r, h->stream); });
+    engine_ops<Real>(h->nx)->row(r, h->stream);
 }
 
 // Whether this handle's steps and evaluations run in the resident kernel: a
@@ -323,6 +318,21 @@ ns2d_status ensure_cn(ns2d_handle* h, double dt, int branch) {
     return NS2D_OK;
 }
 
+// The same for the brackets of the explicit linear term (scale: dt for the
+// quirk's form of RK4's stages, 1 otherwise).
+ns2d_status ensure_lin(ns2d_handle* h, double scale, int branch) {
+    if (h->lint && h->lin_scale == scale && h->lin_branch == branch) return NS2D_OK;
+    if (!h->lint) CK(h, cudaMalloc(&h->lint, sizeof(double) * (size_t)h->nx * h->ldc));
+    CK(h, cudaMemsetAsync(h->dband + 2, 0, sizeof(int), h->stream));
+    lin_table_kernel<<<296, 256, 0, h->stream>>>(h->lint, h->nx, h->nyf, h->ldc, scale, make_lin(h, branch),
+                                                 kept_columns(h->nx, h->p.dealias, h->p.dealias_edge), h->dband + 2);
+    h->launches++;
+    CKL(h);
+    h->lin_scale = scale;
+    h->lin_branch = branch;
+    return NS2D_OK;
+}
+
 template <typename Real>
 ns2d_status resident_rk4(ns2d_handle* h, int nsteps, double dt, void* rk1_out);
 
@@ -345,6 +355,12 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
     const double B_cn[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
     const double B_ex[4] = {1.0, 2.0, 2.0, 1.0};
     const bool conj_quirk = quirk(h, NS2D_QUIRK_CONJ_STATE);
+    const int scheme = explicit_rk4 ? SCH_EX : SCH_CN;
+    // the tables the passes read, built before the first of them
+    ns2d_status s2 = lin_stage       ? ensure_lin(h, lin_stage == 1 ? dt : 1.0, branch)
+                     : !explicit_rk4 ? ensure_cn(h, dt, branch)
+                                     : NS2D_OK;
+    if (s2) return s2;
 
     ColArgs<Real> a;
     fill_common<Real>(h, a, branch);
@@ -364,6 +380,7 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
             a.conj_stride = 1;
         }
         a.lin_stage = lin_stage;
+        a.lint = lin_stage ? h->lint : nullptr;
         a.xin = (lin_stage && s > 1) ? (const C*)h->tmpfull : nullptr;
         a.b_cur = explicit_rk4 ? B_ex[s - 1] : B_cn[s - 1];
         if (s == 1 && rk1_out) a.rhs_store = (C*)rk1_out;
@@ -372,15 +389,10 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
             a.first = (s == 1);
             a.col0_out = (C*)h->col0[s & 1];
             a.out = lin_stage ? (C*)h->tmpfull : nullptr;
-            launch_col<Real>(h, COL_STAGE, a);
+            launch_col<Real>(h, COL_STAGE, a, scheme);
         } else {
-            a.scheme = explicit_rk4 ? 1 : 0;
-            if (!explicit_rk4) {
-                ns2d_status s2 = ensure_cn(h, dt, branch);
-                if (s2) return s2;
-                a.cn = h->cn;
-            }
-            launch_col<Real>(h, COL_FINAL, a);
+            if (!explicit_rk4) a.cn = h->cn;
+            launch_col<Real>(h, COL_FINAL, a, scheme);
         }
     }
     CKL(h);
@@ -469,7 +481,6 @@ ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
     a.conj_mode = 1;
     a.conj_src = (const C*)h->col0[0];
     a.conj_stride = 1;
-    a.scheme = euler ? 3 : 2;
     if (!euler) {
         ns2d_status s2 = ensure_cn(h, dt, branch);
         if (s2) return s2;
@@ -479,7 +490,7 @@ ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
     a.h1 = (const C*)h->ab[1];
     a.h2 = (const C*)h->ab[2];
     a.rhs_store = (C*)h->ab[3];
-    launch_col<Real>(h, COL_FINAL, a);
+    launch_col<Real>(h, COL_FINAL, a, SCH_AB4);
     CKL(h);
     void* oldest = h->ab[0];
     h->ab[0] = h->ab[1];
@@ -551,6 +562,9 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
+    if (!euler) {
+        if (ns2d_status sl = ensure_lin(h, 1.0, branch)) return sl;
+    }
     void* y0 = h->dp[7];
     void* x = h->dp[8];
     CK(h, cudaMemcpyAsync(y0, h->state, h->field_bytes, cudaMemcpyDeviceToDevice, h->stream));
@@ -577,6 +591,7 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
         a.rhs_store = (C*)h->dp[s];
         a.conj_mode = 0;
         a.lin_stage = euler ? 0 : 2;
+        a.lint = euler ? nullptr : h->lint;
         a.xin = (const C*)xs;
         launch_col<Real>(h, COL_RHS, a);
     }
@@ -708,7 +723,7 @@ ns2d_status c2r_impl(ns2d_handle* h, const InvField<Real>* fields, int nf, int o
     ia.nyf = h->nyf;
     ia.ldc = h->ldc;
     ia.tw = (const C*)h->tw;
-    with_size<Real>(h->nx, [&](auto L) { decltype(L)::col_inv(ia, h->stream); });
+    engine_ops<Real>(h->nx)->col_inv(ia, h->stream);
     h->launches++;
     RowC2RArgs<Real> ra;
     std::memset(&ra, 0, sizeof(ra));
@@ -723,7 +738,7 @@ ns2d_status c2r_impl(ns2d_handle* h, const InvField<Real>* fields, int nf, int o
     ra.outA = outA;
     ra.outB = outB;
     if (op != R2_STORE) CK(h, cudaMemsetAsync(h->dmax, 0, sizeof(unsigned long long), h->stream));
-    with_size<Real>(h->nx, [&](auto L) { decltype(L)::row_c2r(op, ra, h->stream); });
+    engine_ops<Real>(h->nx)->row_c2r(op, ra, h->stream);
     h->launches++;
     CKL(h);
     if (result) {
@@ -794,7 +809,7 @@ void fill_twiddles(std::vector<Cplx<Real>>& tw, int n) {
 void free_all(ns2d_handle* h) {
     void* ptrs[] = {h->state, h->acc, h->nl, h->f[0], h->f[1], h->f[2], h->f[3], h->tmpfull, h->col0[0], h->col0[1],
                     h->tw, h->rhsbuf, h->ab[0], h->ab[1], h->ab[2], h->ab[3], h->uhat_ref, h->dreal, h->dscal, h->dmax,
-                    h->dstatus, h->dband, h->dio, h->ddiag, h->dpart, h->cn, h->dp_last};
+                    h->dstatus, h->dband, h->dio, h->ddiag, h->dpart, h->cn, h->dp_last, h->lint, h->filt};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (void* p : h->dp)
@@ -830,8 +845,14 @@ ns2d_status create_impl(ns2d_handle* h) {
     CK(h, cudaMalloc(&h->dmax, sizeof(unsigned long long) * 2));
     CK(h, cudaMalloc(&h->dstatus, sizeof(int) * 4));
     CK(h, cudaMemsetAsync(h->dstatus, 0, sizeof(int) * 4, h->stream));
-    CK(h, cudaMalloc(&h->dband, sizeof(int) * 2));
-    CK(h, cudaMemsetAsync(h->dband, 0, sizeof(int) * 2, h->stream));
+    CK(h, cudaMalloc(&h->dband, sizeof(int) * 3));
+    CK(h, cudaMemsetAsync(h->dband, 0, sizeof(int) * 3, h->stream));
+    if (h->p.dealias == NS2D_DEALIAS_HOU_LI) {
+        CK(h, cudaMalloc(&h->filt, sizeof(Real) * (size_t)h->nx * h->ldc));
+        filter_table_kernel<Real><<<296, 256, 0, h->stream>>>((Real*)h->filt, h->nx, h->nyf, h->ldc,
+                                                              quirk(h, NS2D_QUIRK_HOU_LI_INT) ? 1 : 0);
+        CKL(h);
+    }
     CK(h, cudaMalloc(&h->dio, sizeof(double2) * (size_t)h->nx * h->nyf));
     CK(h, cudaMalloc(&h->ddiag, sizeof(double) * (DG_N + 8 * (size_t)h->n_spect)));
     CK(h, cudaMalloc(&h->dpart, sizeof(double) * 4096));
@@ -844,9 +865,7 @@ ns2d_status create_impl(ns2d_handle* h) {
     fill_twiddles<Real>(tw, h->nx);
     CK(h, cudaMalloc(&h->tw, sizeof(C) * h->nx));
     CK(h, cudaMemcpy(h->tw, tw.data(), sizeof(C) * h->nx, cudaMemcpyHostToDevice));
-    cudaError_t e = cudaSuccess;
-    with_size<Real>(h->nx, [&](auto L) { e = decltype(L)::setup(); });
-    CK(h, e);
+    CK(h, engine_ops<Real>(h->nx)->setup());
     CK(h, cudaStreamSynchronize(h->stream));
     return NS2D_OK;
 }
@@ -901,7 +920,7 @@ ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out) {
 
 // One fixed-dt RK4/RK4CN step for the time loops (ns2d_step_n, ns2d_step_async,
 // the adjoint's record).  The first step with a given dt runs eagerly (it
-// settles the operator branch and the CN table); the step is then captured
+// settles the operator branch and its table); the step is then captured
 // once as a CUDA graph of its nine launches and replayed for the following
 // steps.  With kernel timing on, a second graph carries an event pair around
 // every launch and is read back after each replay.  Stage capture for the
@@ -910,10 +929,16 @@ ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
     if (h->cap_step || resident_ok(h)) return DISPATCH(h, rk4_step_impl, h, dt, nullptr);
     if (ns2d_status sb = ensure_band(h)) return sb;
     int hf = h->hyper_flag;
-    const int branch = (h->p.system == NS2D_EULER && h->p.integrator != NS2D_RK4)
+    const bool rk4_lin = h->p.system != NS2D_EULER && h->p.integrator == NS2D_RK4;
+    const int branch = h->p.system == NS2D_EULER
                            ? 4
                            : ns2d::resolve_branch(hf, h->p.ekmn_drag_flag, quirk(h, NS2D_QUIRK_HYPER_LATCH));
-    const bool settled = (hf == h->hyper_flag) && h->cn_dt == dt && h->cn_branch == branch;
+    // the tables the captured launches read are those of this dt and branch
+    const bool tables = h->p.system == NS2D_EULER ||
+                        (rk4_lin ? h->lint && h->lin_branch == branch &&
+                                       h->lin_scale == (quirk(h, NS2D_QUIRK_RK4_LINEAR) ? dt : 1.0)
+                                 : h->cn_dt == dt && h->cn_branch == branch);
+    const bool settled = (hf == h->hyper_flag) && tables;
     cudaGraphExec_t* gx = h->timing ? &h->timed_graph : &h->step_graph;
     double* gdt = h->timing ? &h->timed_dt : &h->graph_dt;
     int* gbr = h->timing ? &h->timed_branch : &h->graph_branch;
@@ -931,7 +956,7 @@ ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
         if (s) return s;
         h->gev_n_of[set] = h->gev_n;
         *gdt = dt;
-        *gbr = h->cn_branch;
+        *gbr = branch;
         return NS2D_OK;
     }
     cudaError_t e = cudaGraphLaunch(*gx, h->stream);
@@ -1018,11 +1043,9 @@ template <typename Real>
 ns2d_status r2c_host_impl(ns2d_handle* h, const double* real, double* spec) {
     using C = Cplx<Real>;
     CK(h, cudaMemcpyAsync(h->dreal, real, sizeof(double) * (size_t)h->nx * h->ny, cudaMemcpyHostToDevice, h->stream));
-    with_size<Real>(h->nx, [&](auto L) {
-        decltype(L)::fwd(FWD_ROWS, h->dreal, nullptr, (C*)h->f[0], h->nx, h->ldc, (const C*)h->tw, h->stream);
-        decltype(L)::fwd(FWD_COLS, nullptr, (const C*)h->f[0], (C*)h->f[1], h->nyf, h->ldc, (const C*)h->tw,
-                         h->stream);
-    });
+    const auto* ops = engine_ops<Real>(h->nx);
+    ops->fwd(FWD_ROWS, h->dreal, nullptr, (C*)h->f[0], h->nx, h->ldc, (const C*)h->tw, h->stream);
+    ops->fwd(FWD_COLS, nullptr, (const C*)h->f[0], (C*)h->f[1], h->nyf, h->ldc, (const C*)h->tw, h->stream);
     h->launches += 2;
     CKL(h);
     return state_to_host(h, h->f[1], spec);

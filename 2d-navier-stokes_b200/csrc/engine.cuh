@@ -38,21 +38,26 @@ struct Launch {
         return a > b ? a : b;
     }
 
+    template <int MODE, int SCH, typename F>
+    static void set_col(const F& set) {
+        set((const void*)col_kernel<Real, N, S::TC, MODE, SCH>, col_smem());
+        set((const void*)col_tma_kernel<Real, N, S::TC, MODE, SCH>, col_tma_smem());
+    }
     static cudaError_t setup() {
         cudaError_t e = cudaSuccess;
         auto set = [&](const void* f, size_t bytes) {
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         };
-        set((const void*)col_kernel<Real, N, S::TC, COL_P1>, col_smem());
-        set((const void*)col_kernel<Real, N, S::TC, COL_RHS>, col_smem());
-        set((const void*)col_kernel<Real, N, S::TC, COL_STAGE>, col_smem());
-        set((const void*)col_kernel<Real, N, S::TC, COL_FINAL>, col_smem());
-        set((const void*)col_kernel<Real, N, S::TC, COL_STAGE, true>, col_smem());
-        set((const void*)col_kernel<Real, N, S::TC, COL_FINAL, true>, col_smem());
-        set((const void*)col_tma_kernel<Real, N, S::TC, COL_P1>, col_tma_smem());
-        set((const void*)col_tma_kernel<Real, N, S::TC, COL_STAGE>, col_tma_smem());
-        set((const void*)col_tma_kernel<Real, N, S::TC, COL_FINAL>, col_tma_smem());
+        set_col<COL_P1, SCH_CNX>(set);
+        set_col<COL_RHS, SCH_CNX>(set);
+        set_col<COL_STAGE, SCH_CNX>(set);
+        set_col<COL_STAGE, SCH_EX>(set);
+        set_col<COL_FINAL, SCH_CNX>(set);
+        set_col<COL_FINAL, SCH_EX>(set);
+        set_col<COL_FINAL, SCH_AB4>(set);
+        set((const void*)col_tma_kernel<Real, N, S::TC, COL_STAGE, SCH_CN>, col_tma_smem());
+        set((const void*)col_tma_kernel<Real, N, S::TC, COL_FINAL, SCH_CN>, col_tma_smem());
         set((const void*)row_kernel<Real, N, S::PAIRS>, row_smem());
         set((const void*)col_inv_kernel<Real, N, S::TC>, inv_smem());
         set((const void*)row_c2r_kernel<Real, N, S::PAIRS, R2_MAXABS>, c2r_smem());
@@ -63,26 +68,35 @@ struct Launch {
         return e;
     }
 
-    // maps: tensor maps of the arrays the pass reads and writes (null: per-thread
-    // copies); the first, stage and final passes then move their tiles by TMA.
-    static void col(int mode, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps = nullptr) {
+    template <int MODE, int SCH>
+    static void col_one(const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps) {
         dim3 grid((a.nyf + S::TC - 1) / S::TC), block(S::T * S::TC);
-        const bool fast = col_fast_ok(a);
+        if (maps && col_tma_ok(a)) {
+            if constexpr (SCH == SCH_CNX && (MODE == COL_STAGE || MODE == COL_FINAL)) {
+                if (a.dealias == 0 && !a.rhs_store) {
+                    col_tma_kernel<Real, N, S::TC, MODE, SCH_CN><<<grid, block, col_tma_smem(), s>>>(a, *maps);
+                    return;
+                }
+            }
+            col_tma_kernel<Real, N, S::TC, MODE, SCH><<<grid, block, col_tma_smem(), s>>>(a, *maps);
+        } else {
+            col_kernel<Real, N, S::TC, MODE, SCH><<<grid, block, col_smem(), s>>>(a);
+        }
+    }
+    // scheme: SCH_CN, SCH_EX or SCH_AB4 (stage and final passes); maps: tensor maps
+    // of the arrays the pass reads and writes (null: per-thread copies).
+    static void col(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps = nullptr) {
         switch (mode) {
-            case COL_P1:
-                if (maps) col_tma_kernel<Real, N, S::TC, COL_P1><<<grid, block, col_tma_smem(), s>>>(a, *maps);
-                else col_kernel<Real, N, S::TC, COL_P1><<<grid, block, col_smem(), s>>>(a);
-                break;
-            case COL_RHS: col_kernel<Real, N, S::TC, COL_RHS><<<grid, block, col_smem(), s>>>(a); break;
+            case COL_P1: col_one<COL_P1, SCH_CNX>(a, s, maps); break;
+            case COL_RHS: col_one<COL_RHS, SCH_CNX>(a, s, maps); break;
             case COL_STAGE:
-                if (fast && maps) col_tma_kernel<Real, N, S::TC, COL_STAGE><<<grid, block, col_tma_smem(), s>>>(a, *maps);
-                else if (fast) col_kernel<Real, N, S::TC, COL_STAGE, true><<<grid, block, col_smem(), s>>>(a);
-                else col_kernel<Real, N, S::TC, COL_STAGE><<<grid, block, col_smem(), s>>>(a);
+                if (scheme == SCH_EX) col_one<COL_STAGE, SCH_EX>(a, s, maps);
+                else col_one<COL_STAGE, SCH_CNX>(a, s, maps);
                 break;
             default:
-                if (fast && maps) col_tma_kernel<Real, N, S::TC, COL_FINAL><<<grid, block, col_tma_smem(), s>>>(a, *maps);
-                else if (fast) col_kernel<Real, N, S::TC, COL_FINAL, true><<<grid, block, col_smem(), s>>>(a);
-                else col_kernel<Real, N, S::TC, COL_FINAL><<<grid, block, col_smem(), s>>>(a);
+                if (scheme == SCH_EX) col_one<COL_FINAL, SCH_EX>(a, s, maps);
+                else if (scheme == SCH_AB4) col_one<COL_FINAL, SCH_AB4>(a, s, maps);
+                else col_one<COL_FINAL, SCH_CNX>(a, s, maps);
                 break;
         }
     }
@@ -128,5 +142,22 @@ inline bool with_size(int n, F&& f) {
         default: return false;
     }
 }
+
+// The launch functions of one grid size in one precision, compiled in
+// engine_f32.cu and engine_f64.cu.
+template <typename Real>
+struct EngineOps {
+    int tc;  // column-tile width
+    cudaError_t (*setup)();
+    void (*col)(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps);
+    void (*row)(const RowArgs<Real>& a, cudaStream_t s);
+    void (*col_inv)(const InvArgs<Real>& a, cudaStream_t s);
+    void (*fwd)(int pass, const double* real_in, const typename Cx<Real>::T* in, typename Cx<Real>::T* out, int nlines,
+                int ldc, const typename Cx<Real>::T* tw, cudaStream_t s);
+    void (*row_c2r)(int op, const RowC2RArgs<Real>& a, cudaStream_t s);
+};
+// Null for a size that has none.
+template <typename Real>
+const EngineOps<Real>* engine_ops(int n);
 
 }  // namespace ns2d

@@ -53,7 +53,7 @@ struct ns2d_ensemble {
     std::vector<void*> state, nl, acc, tw;
     std::vector<double2*> cn;
     std::vector<int> ldc;
-    int* band = nullptr;          // [n][2]: band_narrow words of each member
+    int* band = nullptr;          // [n][3]: band_narrow words of each member
     double2* io = nullptr;        // staging for host I/O, largest member
     int col_grid = 0, row_grid = 0;
     // CN tables and graph for the current dt
@@ -127,20 +127,20 @@ cudaError_t ens_set_smem(ns2d_ensemble* e) {
     auto set = [&](const void* f, size_t b) {
         if (r == cudaSuccess) r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
     };
-    set((const void*)ens_col_kernel<Real, COL_P1, TH>, e->col_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_STAGE, TH>, e->col_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_FINAL, TH>, e->col_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_STAGE, TH, true>, e->col_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_FINAL, TH, true>, e->col_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_P1, TH, true, true>, e->col_tma_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_STAGE, TH, true, true>, e->col_tma_smem[V]);
-    set((const void*)ens_col_kernel<Real, COL_FINAL, TH, true, true>, e->col_tma_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_P1, TH, SCH_CNX, true, false>, e->col_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_STAGE, TH, SCH_CNX, true, false>, e->col_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_STAGE, TH, SCH_EX, true, false>, e->col_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_FINAL, TH, SCH_CNX, true, false>, e->col_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_FINAL, TH, SCH_EX, true, false>, e->col_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_P1, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_STAGE, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_FINAL, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
     set((const void*)ens_row_kernel<Real, TH>, e->row_smem[V]);
     return r;
 }
 
-// Whether the stage and final column passes of this ensemble can run the
-// epilogue compiled for the common step (col_fast_ok of the single passes).
+// Whether the column passes of this ensemble can run the form compiled for the
+// common step (members have no factor tables for the others).
 bool ens_fast(const ns2d_ensemble* e) {
     return e->p.dealias == 0 && e->p.system != NS2D_EULER && e->p.integrator == NS2D_RK4CN &&
            e->p.model == NS2D_MODEL_FULL;
@@ -151,41 +151,35 @@ template <typename Real, int V>
 void ens_occupancy(const ns2d_ensemble* e, int* col_per_sm, int* row_per_sm) {
     constexpr int TH = kEnsThreadChoices[V];
     if (e->maps && ens_fast(e))
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(col_per_sm, ens_col_kernel<Real, COL_STAGE, TH, true, true>, TH,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(col_per_sm, ens_col_kernel<Real, COL_STAGE, TH, SCH_CN, false, true>, TH,
                                                       e->col_tma_smem[V]);
     else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(col_per_sm, ens_col_kernel<Real, COL_STAGE, TH>, TH, e->col_smem[V]);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(col_per_sm, ens_col_kernel<Real, COL_STAGE, TH, SCH_CNX, true, false>, TH,
+                                                      e->col_smem[V]);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(row_per_sm, ens_row_kernel<Real, TH>, TH, e->row_smem[V]);
 }
 
 
-template <typename Real, int MODE, int V, bool FAST, bool TMA = false>
+template <typename Real, int MODE, int V, int SCH, bool TMA>
 void ens_launch_col_v(ns2d_ensemble* e, const EnsMember<Real>* mb, const EnsStage& st) {
     constexpr int TH = kEnsThreadChoices[V];
-    ens_col_kernel<Real, MODE, TH, FAST, TMA><<<e->col_grid, TH, TMA ? e->col_tma_smem[V] : e->col_smem[V], e->stream>>>(
+    ens_col_kernel<Real, MODE, TH, SCH, !TMA, TMA><<<e->col_grid, TH, TMA ? e->col_tma_smem[V] : e->col_smem[V], e->stream>>>(
         mb, e->col_items[V], e->n_col_items[V], st, e->maps);
 }
 
 // The TMA column kernels run the common step (ens_fast) when the members'
-// tensor maps exist; otherwise per-thread copies.
+// tensor maps exist; otherwise the general ones.
+template <typename Real, int MODE, int V>
+void ens_launch_col_s(ns2d_ensemble* e, const EnsMember<Real>* mb, const EnsStage& st) {
+    const bool ex = e->p.system == NS2D_EULER || e->p.integrator == NS2D_RK4;
+    if (ens_fast(e) && e->maps) ens_launch_col_v<Real, MODE, V, SCH_CN, true>(e, mb, st);
+    else if (MODE != COL_P1 && ex) ens_launch_col_v<Real, MODE, V, MODE == COL_P1 ? SCH_CNX : SCH_EX, false>(e, mb, st);
+    else ens_launch_col_v<Real, MODE, V, SCH_CNX, false>(e, mb, st);
+}
 template <typename Real, int MODE>
 void ens_launch_col(ns2d_ensemble* e, const EnsMember<Real>* mb, const EnsStage& st) {
-    const bool fast = ens_fast(e);
-    if (fast && e->maps) {
-        if (e->col_var == 0) ens_launch_col_v<Real, MODE, 0, true, true>(e, mb, st);
-        else ens_launch_col_v<Real, MODE, 1, true, true>(e, mb, st);
-    } else if constexpr (MODE == COL_P1) {
-        if (e->col_var == 0) ens_launch_col_v<Real, MODE, 0, false>(e, mb, st);
-        else ens_launch_col_v<Real, MODE, 1, false>(e, mb, st);
-    } else {
-        if (e->col_var == 0) {
-            if (fast) ens_launch_col_v<Real, MODE, 0, true>(e, mb, st);
-            else ens_launch_col_v<Real, MODE, 0, false>(e, mb, st);
-        } else {
-            if (fast) ens_launch_col_v<Real, MODE, 1, true>(e, mb, st);
-            else ens_launch_col_v<Real, MODE, 1, false>(e, mb, st);
-        }
-    }
+    if (e->col_var == 0) ens_launch_col_s<Real, MODE, 0>(e, mb, st);
+    else ens_launch_col_s<Real, MODE, 1>(e, mb, st);
 }
 
 template <typename Real>
@@ -218,7 +212,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
     e->tw.resize(e->n);
     e->cn.resize(e->n);
     e->ldc.resize(e->n);
-    ECK(e, alloc(sizeof(int) * 2 * (size_t)e->n, (void**)&e->band));
+    ECK(e, alloc(sizeof(int) * 3 * (size_t)e->n, (void**)&e->band));
     for (int m = 0; m < e->n; ++m) {
         const int n = e->sizes[m];
         const int nyf = n / 2 + 1;
@@ -274,7 +268,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
             a.force_val.y = (Real)0;
         }
         // a forced mode among the emptied columns keeps them in the transforms
-        if (!(a.has_force && a.force_j >= a.kc)) a.band = e->band + 2 * m;
+        if (!(a.has_force && a.force_j >= a.kc)) a.band = e->band + 3 * m;
         a.norm2 = (Real)std::pow(1.0 / (double)(n * n), 2.0);
         a.inv_nxny = 1.0 / (double)(n * n);
         a.cn = (const double2*)cn;
@@ -369,12 +363,16 @@ ns2d_status create_t(ns2d_ensemble* e) {
         ECK(e, cudaMemcpyAsync(e->need, need.data(), sizeof(int) * need.size(), cudaMemcpyHostToDevice, e->stream));
         constexpr int TH = kEnsThreadChoices[0];
         e->stage_smem = EnsSmem<Real, TH>::stage();
-        ECK(e, cudaFuncSetAttribute((const void*)ens_stage_kernel<Real, COL_STAGE, TH>,
+        ECK(e, cudaFuncSetAttribute((const void*)ens_stage_kernel<Real, COL_STAGE, TH, SCH_CNX>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->stage_smem));
-        ECK(e, cudaFuncSetAttribute((const void*)ens_stage_kernel<Real, COL_FINAL, TH>,
+        ECK(e, cudaFuncSetAttribute((const void*)ens_stage_kernel<Real, COL_STAGE, TH, SCH_EX>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->stage_smem));
+        ECK(e, cudaFuncSetAttribute((const void*)ens_stage_kernel<Real, COL_FINAL, TH, SCH_CNX>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->stage_smem));
+        ECK(e, cudaFuncSetAttribute((const void*)ens_stage_kernel<Real, COL_FINAL, TH, SCH_EX>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->stage_smem));
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ens_stage_kernel<Real, COL_STAGE, TH>, TH, e->stage_smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ens_stage_kernel<Real, COL_STAGE, TH, SCH_CNX>, TH, e->stage_smem);
         e->stage_per_sm = std::max(1, per_sm);
     }
     ECK(e, (ens_set_smem<Real, 0>(e)));
@@ -404,7 +402,7 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
         const LinOp L = make_lin_params(e->p, branch);
         for (int m = 0; m < e->n; ++m) {
             const int n = e->sizes[m];
-            int* const odd = e->band + 2 * m + 1;
+            int* const odd = e->band + 3 * m + 1;
             ECK(e, cudaMemsetAsync(odd, 0, sizeof(int), e->stream));
             cn_table_kernel<<<148, 256, 0, e->stream>>>(e->cn[m], n, n / 2 + 1, e->ldc[m], dt, L,
                                                         kept_columns(n, e->p.dealias, 0), odd);
@@ -441,10 +439,11 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
             if (s < 4) {
                 st.a_next = A[s - 1];
                 st.first = (s == 1);
-                ens_stage_kernel<Real, COL_STAGE, TH><<<e->stage_grid, TH, e->stage_smem, e->stream>>>(mb, tl, nt, st, sy);
+                if (explicit_rk4) ens_stage_kernel<Real, COL_STAGE, TH, SCH_EX><<<e->stage_grid, TH, e->stage_smem, e->stream>>>(mb, tl, nt, st, sy);
+                else ens_stage_kernel<Real, COL_STAGE, TH, SCH_CNX><<<e->stage_grid, TH, e->stage_smem, e->stream>>>(mb, tl, nt, st, sy);
             } else {
-                st.scheme = explicit_rk4 ? 1 : 0;
-                ens_stage_kernel<Real, COL_FINAL, TH><<<e->stage_grid, TH, e->stage_smem, e->stream>>>(mb, tl, nt, st, sy);
+                if (explicit_rk4) ens_stage_kernel<Real, COL_FINAL, TH, SCH_EX><<<e->stage_grid, TH, e->stage_smem, e->stream>>>(mb, tl, nt, st, sy);
+                else ens_stage_kernel<Real, COL_FINAL, TH, SCH_CNX><<<e->stage_grid, TH, e->stage_smem, e->stream>>>(mb, tl, nt, st, sy);
             }
             e->launches++;
         }
@@ -465,7 +464,6 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
             st.first = (s == 1);
             ens_launch_col<Real, COL_STAGE>(e, mb, st);
         } else {
-            st.scheme = explicit_rk4 ? 1 : 0;
             ens_launch_col<Real, COL_FINAL>(e, mb, st);
         }
         e->launches++;
@@ -559,10 +557,10 @@ ns2d_status set_t(ns2d_ensemble* e, int m, const double* host) {
     const int n = e->sizes[m], nyf = n / 2 + 1;
     using C = typename Cx<Real>::T;
     ECK(e, cudaMemcpyAsync(e->io, host, sizeof(double2) * (size_t)n * nyf, cudaMemcpyHostToDevice, e->stream));
-    ECK(e, cudaMemsetAsync(e->band + 2 * m, 0, sizeof(int), e->stream));
+    ECK(e, cudaMemsetAsync(e->band + 3 * m, 0, sizeof(int), e->stream));
     pack_kernel<Real><<<148, 256, 0, e->stream>>>(e->io, (C*)e->state[m], n, nyf, e->ldc[m]);
     band_scan_kernel<Real><<<32, 256, 0, e->stream>>>((const C*)e->state[m], n, nyf, e->ldc[m],
-                                                      kept_columns(n, e->p.dealias, 0), e->band + 2 * m);
+                                                      kept_columns(n, e->p.dealias, 0), e->band + 3 * m);
     e->launches += 2;
     ECK(e, cudaGetLastError());
     ECK(e, cudaStreamSynchronize(e->stream));

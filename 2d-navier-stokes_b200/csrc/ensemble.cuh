@@ -43,7 +43,7 @@ struct EnsItem {
 // Per-launch stage parameters shared by all members.
 struct EnsStage {
     double dt, a_next, b_cur;
-    int first, scheme, conj_quirk, stage;  // stage 1..4; 0 = P1 of the step
+    int first, conj_quirk, stage;  // stage 1..4; 0 = P1 of the step
     LinOp lin;
     int* status;
 };
@@ -54,7 +54,6 @@ __device__ __forceinline__ void ens_apply_stage(ColArgs<Real>& a, const EnsMembe
     a.a_next = st.a_next;
     a.b_cur = st.b_cur;
     a.first = st.first;
-    a.scheme = st.scheme;
     a.lin = st.lin;
     a.final_tail = 0;
     a.status = st.status;
@@ -83,11 +82,11 @@ struct EnsMinBlocks {
     static constexpr int value = sizeof(Real) == 4 ? 512 / THREADS : 256 / THREADS;
 };
 
-// TMA (with FAST): the tiles move by TMA copies through maps[2 m + v], the
+// SCH, GEN: as col_body.  TMA: the tiles move by TMA copies through maps[2 m + v], the
 // tensor maps of member m for this block size (v = 0 for kEnsThreadChoices[0],
 // 1 for the other); shared memory EnsSmem::col_tma().  A tile whose loads do
 // not land within their bound stops the block (status bit 8).
-template <typename Real, int MODE, int THREADS, bool FAST = false, bool TMA = false>
+template <typename Real, int MODE, int THREADS, int SCH, bool GEN, bool TMA>
 __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value)) ens_col_kernel(const EnsMember<Real>* __restrict__ members,
                                                       const EnsItem* __restrict__ items, int nitems, EnsStage st,
                                                       const ColMaps* __restrict__ maps) {
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
         switch (mb.n) {
 #define NS2D_ENS_COL(NN)                                                                           \
     case NN:                                                                                       \
-        go = col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE, FAST, TMA>(a, begin, item.tile, sm, mp); \
+        go = col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE, SCH, GEN, TMA>(a, begin, item.tile, sm, mp); \
         break;
             NS2D_ENS_SIZES(NS2D_ENS_COL)
 #undef NS2D_ENS_COL
@@ -180,7 +179,7 @@ __device__ __forceinline__ bool ens_wait_count(const int* cnt, int need, int* st
     return true;
 }
 
-template <typename Real, int MODE, int THREADS>
+template <typename Real, int MODE, int THREADS, int SCH>
 __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
     ens_stage_kernel(const EnsMember<Real>* __restrict__ members, const EnsTask* __restrict__ tasks, int ntasks,
                      EnsStage st, EnsSync sy) {
@@ -227,9 +226,9 @@ __global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
 #define NS2D_ENS_SCOL(NN)                                                                          \
     case NN:                                                                                       \
         if (task.kind == 0) {                                                                      \
-            col_body<Real, NN, EnsShape<NN, THREADS>::TC, COL_P1>(a, begin, task.tile, smraw);            \
+            col_body<Real, NN, EnsShape<NN, THREADS>::TC, COL_P1, SCH, true>(a, begin, task.tile, smraw);            \
         } else {                                                                                   \
-            col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE>(a, begin, task.tile, smraw);              \
+            col_body<Real, NN, EnsShape<NN, THREADS>::TC, MODE, SCH, true>(a, begin, task.tile, smraw);              \
         }                                                                                          \
         break;
                 NS2D_ENS_SIZES(NS2D_ENS_SCOL)

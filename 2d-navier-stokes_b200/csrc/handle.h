@@ -39,7 +39,7 @@ struct ns2d_handle {
     double* dscal = nullptr;   // [0] bound accumulator, [1] ticket
     unsigned long long* dmax = nullptr;
     int* dstatus = nullptr;    // [0] bits, [1] completed steps
-    int* dband = nullptr;      // band_narrow words: [0] the state, [1] the update factors
+    int* dband = nullptr;      // band_narrow words: [0] the state, [1] the update factors, [2] the explicit linear ones
     bool band_known = false;   // dband[0] describes the state
     bool ffield_band = false;  // the listed forcing has modes in the columns dealiasing empties
     bool band_forced = false;  // and the state may hold their trace
@@ -49,6 +49,10 @@ struct ns2d_handle {
     double2* cn = nullptr;     // Crank-Nicolson factors per mode ([nx][ldc])
     double cn_dt = 0.0;        // dt and branch the table was built for
     int cn_branch = -1;
+    double* lint = nullptr;    // brackets of the explicit linear term per mode (on first use)
+    double lin_scale = 0.0;    // scale and branch the table was built for
+    int lin_branch = -1;
+    void* filt = nullptr;      // Hou-Li factors per mode
     // model state kept on the host
     int hyper_flag = 0;
     bool forced = false;

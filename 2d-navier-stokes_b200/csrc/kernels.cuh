@@ -34,6 +34,13 @@ namespace ns2d {
 
 enum ColMode : int { COL_P1 = 0, COL_RHS = 1, COL_STAGE = 2, COL_FINAL = 3 };
 
+// Update schemes of the stage and final column passes: RK4 with Crank-Nicolson
+// factors under the 2/3 rule (the common step), the same with Hou-Li dealiasing or
+// a stored RHS too, explicit RK4 (or Euler system), AB4 (explicit or Crank-
+// Nicolson).  Each is compiled by itself, with what it needs: the common step's
+// stage pass at 2048^2 FP64 takes 70.6 us, 77.5 with the second form's branches in.
+enum ColScheme : int { SCH_CN = 0, SCH_CNX = 1, SCH_EX = 2, SCH_AB4 = 3 };
+
 // Linear-operator bracket selection (Solver/src/solver.c:839-856):
 // 1: nu k^2p + a k^2q, 2: nu k^2 + a k^2q, 3: nu k^2p, 4: nu k^2.
 struct LinOp {
@@ -103,13 +110,14 @@ struct ColArgs {
     double a_next;       // next stage input = state + (dt a_next) rhs
     double b_cur;        // accumulator coefficient of this stage's RHS
     int first;           // acc = b rhs (instead of acc += b rhs)
-    int scheme;          // 0: RK4CN, 1: explicit RK4 (Euler or __RK4), 2: AB4 + CN, 3: AB4 explicit
     const C* h0;         // AB4 history: RHS of steps n-3, n-2, n-1 (AB_tmp_nonlin[0..2])
     const C* h1;
     const C* h2;
     int lin_stage;       // 0 none, 1: rhs += dt D X (quirk), 2: rhs -= D X (corrected)
     LinOp lin;
     const double2* cn;   // COL_FINAL, CN schemes: per-mode ((2-D)/(2+D), 2dt/(2+D)), stride ldc
+    const double* lint;  // per-mode bracket of the linear term (times dt for lin_stage 1), stride ldc; null: formed per mode (GEN)
+    const Real* filt;    // Hou-Li factors, stride ldc; null: formed per mode (GEN)
     const C* force_field;  // forcing added to every mode of the RHS ([nx][ldc]), may be null
     double inv_nxny;     // 1/(Nx Ny)
     int final_tail;      // COL_FINAL: 1 = SystemCheck bound over ntiles tiles, 0 = non-finite check only
@@ -120,13 +128,13 @@ struct ColArgs {
 
 // Whether the evaluation's input is known to be zero in the columns ky >= kc
 // that the 2/3 rule empties: band[0] is set when the state holds something there
-// (it may: the caller sets it), band[1] when an update factor there is not finite
-// (0 times it is not 0).  The x-space fields of those columns are then zero too,
+// (it may: the caller sets it), band[1] and band[2] when an update factor or an
+// explicit linear factor there is not finite (0 times it is not 0).  The x-space fields of those columns are then zero too,
 // so the passes neither form, store nor read them: a third of the columns, and a
 // third of every pass's x-space traffic.  null: not known.  Per step, FP64 / FP32:
 // 2048^2 678 / 400 -> 542 / 329 us, the 64-member FP32 ensemble 421 -> 328 us;
 // 1024^2, where the tiles fill one wave either way, 149 / 97 -> 144 / 94 us.
-__device__ __forceinline__ bool band_narrow(const int* band) { return band && (band[0] | band[1]) == 0; }
+__device__ __forceinline__ bool band_narrow(const int* band) { return band && (band[0] | band[1] | band[2]) == 0; }
 
 // Start of a pass block: early exit once the device status word is set (a failed
 // SystemCheck), and band_narrow of the evaluation.  One thread reads the words
@@ -141,7 +149,8 @@ __device__ __forceinline__ BlockBegin block_begin(const int* status, const int* 
         const int st = status ? *(volatile const int*)status : 0;
         const int b0 = band ? band[0] : 1;
         const int b1 = band ? band[1] : 1;
-        flags = (st != 0 ? 1 : 0) | ((b0 | b1) == 0 ? 2 : 0);
+        const int b2 = band ? band[2] : 1;
+        flags = (st != 0 ? 1 : 0) | ((b0 | b1 | b2) == 0 ? 2 : 0);
     }
     __syncthreads();
     const int f = flags;
@@ -506,24 +515,26 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 // threads of a block, thread (t, c) with c = threadIdx.x % TC.  Shared memory:
 // ColSmem::bytes().  Ends with the block synchronised (the shared memory may be
 // reused for another tile).
-// TMA (with FAST, modes P1, STAGE and FINAL): the pass's inputs (a.src, a.state,
-// a.acc) arrive by TMA tile loads and its outputs (the x-space fields, the
-// accumulator, the final state) leave by bulk-async tile stores, through `maps`
-// (which must describe those arrays), instead of per-thread copies; smraw
-// 1024-byte aligned; SPLIT: the last inverse pair as two single transforms
-// (derived_ifft_tma).  Its mbarriers are invalidated once used, so a persistent
-// caller can run the body again on the same shared memory.  A load that does
-// not land within its bound sets status bit 8 and the body returns false (the
-// block must stop); otherwise it returns true.
-// A tile of emptied columns (all ky >= kc) needs no
-// forward transform (its RHS is zero) and, when narrow, no inverse ones; in the
-// FAST modes there is then nothing left to do (state and accumulator stay zero).
+// SCH: the update scheme of the stage and final modes (ColScheme).  GEN: listed-
+// mode forcing, the phase-only model and members without factor tables compiled
+// in.
+// TMA: the pass's inputs (a.src, a.state, a.acc) arrive by TMA tile loads and its
+// outputs (the x-space fields, the accumulator, the final state) leave by
+// bulk-async tile stores, through `maps` (which must describe those arrays),
+// instead of per-thread copies; smraw 1024-byte aligned; SPLIT: the last inverse
+// pair as two single transforms (derived_ifft_tma).  Its mbarriers are
+// invalidated once used, so a persistent caller can run the body again on the
+// same shared memory.  A load that does not land within its bound sets status
+// bit 8 and the body returns false (the block must stop); otherwise it returns
+// true.
+// A tile of emptied columns (all ky >= kc) needs no forward transform (its RHS is
+// zero) and, when the band is narrow, nothing else either: state and accumulator
+// stay zero there.
 // begin(): the block's flags (BlockBegin) and a block barrier; called once the
 // TMA tile loads are under way, so the flags' latency runs under theirs.
-template <typename Real, int N, int TC, int MODE, bool FAST = false, bool TMA = false, bool SPLIT = false, typename Begin>
+template <typename Real, int N, int TC, int MODE, int SCH, bool GEN = false, bool TMA = false, bool SPLIT = false, typename Begin>
 __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& begin, int tile, unsigned char* smraw,
                                          const ColMaps* maps = nullptr) {
-    static_assert(!TMA || (FAST && MODE != COL_RHS), "TMA copies: FAST P1, STAGE and FINAL only");
     using C = typename Cx<Real>::T;
     using P = Plan<N>;
     using SM = ColSmem<Real, N, TC>;
@@ -540,21 +551,21 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
     const int ldc = a.ldc;
     const bool dead = tile * TC >= a.kc;
     const auto seed = twiddle_seeds<N>(a.tw, t);
+    constexpr bool XTRA = SCH != SCH_CN;  // Hou-Li factors, a stored RHS
     constexpr bool need_state = (MODE == COL_STAGE || MODE == COL_FINAL);
-    const bool need_acc = (MODE == COL_STAGE && !a.first) || (MODE == COL_FINAL && a.scheme < 2);
-    // TMA: [0] the input, [1] state and accumulator (P1: the input alone)
+    const bool need_acc = (MODE == COL_STAGE && !a.first) || (MODE == COL_FINAL && SCH != SCH_AB4);
+    // TMA: [0] the input, [1] state and accumulator
     __shared__ __align__(8) unsigned long long bar_tile[2];
     auto issue = [&] {
         if constexpr (TMA) {
             if (threadIdx.x == 0) {
                 constexpr unsigned tile_bytes = (unsigned)(sizeof(C) * N * TC);
                 mbar_init(&bar_tile[0]);
-                if constexpr (MODE != COL_P1) mbar_init(&bar_tile[1]);
+                if constexpr (need_state) mbar_init(&bar_tile[1]);
                 mbar_expect_tx(&bar_tile[0], tile_bytes);
-                if constexpr (MODE == COL_P1) {
-                    tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_tile[0]);
-                } else {
-                    tma_load_tile<C, N, TC>(&maps->nl, tile, sm, &bar_tile[0]);
+                if constexpr (MODE == COL_P1) tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_tile[0]);
+                else tma_load_tile<C, N, TC>(&maps->nl, tile, sm, &bar_tile[0]);
+                if constexpr (need_state) {
                     mbar_expect_tx(&bar_tile[1], need_acc ? 2 * tile_bytes : tile_bytes);
                     tma_load_tile<C, N, TC>(&maps->state, tile, pre0, &bar_tile[1]);
                     if (need_acc) tma_load_tile<C, N, TC>(&maps->acc, tile, pre1, &bar_tile[1]);
@@ -562,15 +573,15 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             }
         }
     };
-    // Waits for the loads of `bar`; false (status bit 8 set, and every copy still
-    // in flight waited for once more, bounded) when they do not land.  A block
-    // barrier after the wait: it also orders the reads before it.
+    // A block barrier after a wait for loads (late: they did not land), which also
+    // orders the reads before it; false (status bit 8 set, and every copy still in
+    // flight waited for once more, bounded) when any thread's wait ran out.
     auto landed = [&](bool late) {
         if (__syncthreads_or(late)) {
             if (threadIdx.x == 0) {
                 atomicOr(a.status, 8);
                 mbar_wait0(&bar_tile[0]);
-                if constexpr (MODE != COL_P1) mbar_wait0(&bar_tile[1]);
+                if constexpr (need_state) mbar_wait0(&bar_tile[1]);
             }
             return false;
         }
@@ -584,13 +595,19 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         if constexpr (TMA) {
             if (!dead && threadIdx.x == 0) {
                 mbar_wait0(&bar_tile[0]);
-                if constexpr (MODE != COL_P1) mbar_wait0(&bar_tile[1]);
+                if constexpr (need_state) mbar_wait0(&bar_tile[1]);
             }
         }
         return false;
     }
     if (dead) {
-        if ((FAST || MODE == COL_P1) && narrow) return true;
+        if (narrow && MODE != COL_RHS) {
+            if (XTRA && MODE != COL_P1 && a.rhs_store && valid) {
+#pragma unroll
+                for (int m = 0; m < E; ++m) a.rhs_store[(size_t)(t + T * m) * ldc + ky] = cmake<C>(0, 0);
+            }
+            return true;
+        }
         issue();
         if constexpr (TMA) __syncthreads();
     }
@@ -617,7 +634,6 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             for (int m = 0; m < E; ++m) a.col0_out[t + T * m] = pre0[(t + T * m) * TC + c];
         }
     } else {
-        const C* __restrict__ src = a.src;
         C v[1][E];
         if constexpr (TMA) {
             const bool late = !mbar_wait0(&bar_tile[0]);
@@ -627,11 +643,10 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             if (!landed(late)) return false;
             if (threadIdx.x == 0) mbar_inval(&bar_tile[0]);
         } else {
+            const C* __restrict__ src = a.src;
 #pragma unroll
-            for (int m = 0; m < E; ++m) {
-                const int i = t + T * m;
-                v[0][m] = valid && !dead ? src[(size_t)i * ldc + kyc] : cmake<C>(0, 0);
-            }
+            for (int m = 0; m < E; ++m)
+                v[0][m] = valid && !dead ? src[(size_t)(t + T * m) * ldc + kyc] : cmake<C>(0, 0);
         }
         // prefetch the epilogue operands while the forward transform runs
         if constexpr (need_state && !TMA) {
@@ -651,209 +666,193 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         if constexpr (MODE == COL_FINAL) {
             // the Crank-Nicolson factors are read in the epilogue: start bringing
             // this thread's entries into L2 now, under the forward transform
-            if (a.cn && valid) {
+            if (SCH != SCH_EX && a.cn && valid) {
 #pragma unroll
                 for (int m = 0; m < E; ++m) prefetch_l2(a.cn + (size_t)(t + T * m) * ldc + ky);
             }
         }
-        if (FAST || !dead) fft_batched<N, -1, 1>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
-        double bsum = 0.0;
-        bool bad = false;
-        if constexpr (FAST) {
-            // The common step's epilogue, straight from the transform's registers.
-            // Operands come in batches that are read before any result of the batch
-            // is written (a load after a store to shared memory would wait for it).
-            // Stage pass at 1024^2 FP64, transform to transform: 4,540 -> 3,200 cycles;
-            // final pass at 256^2 13.8 -> 9.6 us.
+        if (!dead) {
+            fft_batched<N, -1, 1>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
+        } else {
+#pragma unroll
+            for (int m = 0; m < E; ++m) v[0][m] = cmake<C>(0, 0);
+        }
+        if constexpr (need_state) {
             if constexpr (TMA) {
                 if (!landed(!mbar_wait0(&bar_tile[1]))) return false;
                 if (threadIdx.x == 0) mbar_inval(&bar_tile[1]);
             } else {
                 cp_async_wait_all();
             }
+        }
+        // The epilogue, straight from the transform's registers.  Operands come in
+        // batches that are read before any result of the batch is written (a load
+        // after a store to shared memory would wait for it).  Stage pass at 1024^2
+        // FP64, transform to transform: 4,540 -> 3,200 cycles against one element at
+        // a time; final pass at 256^2 13.8 -> 9.6 us.
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+            const int i = t + T * m;
+            const int kx = (i <= N / 2) ? i : i - N;
+            // normalisation and zero mean (solver.c:998-1013), 2/3 mask (solver.c:1039-1099)
+            const bool zero = (m == 0 && i == 0 && ky == 0) ||
+                              ((!XTRA || a.dealias == 0) && (kx * kx + ky * ky >= a.kmax_sqr || (a.kolm && kx == 0)));
+            v[0][m] = zero ? cmake<C>(0, 0) : cscale(v[0][m], a.norm2);
+        }
+        if (XTRA && a.dealias != 0) {
+            // Hou-Li factors: with the reference's integer ratios they are 1 except
+            // where |kx| or ky is N/2
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const int i = t + T * m;
-                const int kx = (i <= N / 2) ? i : i - N;
-                // normalisation and zero mean (solver.c:998-1013), 2/3 mask (solver.c:1039-1099)
-                const bool zero = (m == 0 && i == 0 && ky == 0) || kx * kx + ky * ky >= a.kmax_sqr || (a.kolm && kx == 0);
-                v[0][m] = zero ? cmake<C>(0, 0) : cscale(v[0][m], a.norm2);
+                if (a.houli_int && i != N / 2 && 2 * ky != N) continue;
+                Real d;
+                if (!GEN || a.filt) d = a.filt[(size_t)i * ldc + kyc];
+                else d = houli_filter<Real>((i <= N / 2) ? i : i - N, ky, N, N, a.houli_int);
+                v[0][m] = cscale(v[0][m], d);
             }
-            // forcing (solver.c:1022-1027)
-            if (a.has_force && ky == a.force_j) {
+        }
+        // forcing (solver.c:1022-1027)
+        if (a.has_force && ky == a.force_j) {
 #pragma unroll
-                for (int m = 0; m < E; ++m)
-                    if (t + T * m == a.force_i) v[0][m] = cadd(v[0][m], a.force_val);
+            for (int m = 0; m < E; ++m)
+                if (t + T * m == a.force_i) v[0][m] = cadd(v[0][m], a.force_val);
+        }
+        if constexpr (GEN) {
+            if (a.force_field) {
+#pragma unroll
+                for (int m = 0; m < E; ++m) v[0][m] = cadd(v[0][m], a.force_field[(size_t)(t + T * m) * ldc + kyc]);
             }
-            // ForceConjugacy side effect on the state (solver.c:1031, 2096-2103)
-            if (a.conj_mode && ky == 0) {
+        }
+        // The bracket of the linear term at element m, times dt for the quirk's form.
+        auto linear = [&](int m) -> Real {
+            const int i = t + T * m;
+            if (!GEN || a.lint) return (Real)a.lint[(size_t)i * ldc + kyc];
+            const int kx = (i <= N / 2) ? i : i - N;
+            const double br = lin_bracket(a.lin, (double)(kx * kx + ky * ky));
+            return (Real)(a.lin_stage == 1 ? a.dt * br : br);
+        };
+        if constexpr (MODE == COL_RHS) {
+            // stage derivative with the explicit linear term (Dormand-Prince
+            // stages): r -= bracket(|k|^2) X, X the RHS input
+            if (a.lin_stage == 2 && a.xin) {
 #pragma unroll
-                for (int m = E / 2; m < E; ++m) {
-                    const int i = t + T * m;
-                    if (i > N / 2) {
-                        const C w = cconj(a.conj_src[(size_t)(N - i) * a.conj_stride]);
-                        pre0[i * TC + c] = w;
-                        // (the TMA final pass stores this element's update through the tile copy)
-                        if constexpr (!(TMA && MODE == COL_FINAL)) a.state[(size_t)i * ldc] = w;
-                    }
+                for (int m = 0; m < E; ++m) {
+                    const C r = csub(v[0][m], cscale(a.xin[(size_t)(t + T * m) * ldc + kyc], linear(m)));
+                    if (!(m == 0 && t == 0 && ky == 0)) v[0][m] = r;
                 }
             }
-            constexpr int EB = E < 4 ? E : (MODE == COL_FINAL && E >= 8) ? 8 : 4;
-            const Real bc = (Real)a.b_cur;
-            const Real adt = (Real)(a.dt * a.a_next);
+        }
+        if (XTRA && a.rhs_store && valid) {
 #pragma unroll
-            for (int m0 = 0; m0 < E; m0 += EB) {
-                C w[EB], acc[EB];
-                double2 f[MODE == COL_FINAL ? EB : 1];
-                if constexpr (MODE == COL_FINAL) {
-                    // Crank-Nicolson factors (solver.c:853), from the table
+            for (int m = 0; m < E; ++m) a.rhs_store[(size_t)(t + T * m) * ldc + ky] = v[0][m];
+        }
+        // ForceConjugacy side effect on the state (solver.c:1031, 2096-2103)
+        if (a.conj_mode && ky == 0) {
+#pragma unroll
+            for (int m = E / 2; m < E; ++m) {
+                const int i = t + T * m;
+                if (i > N / 2) {
+                    const C w = cconj(a.conj_src[(size_t)(N - i) * a.conj_stride]);
+                    if constexpr (need_state) pre0[i * TC + c] = w;
+                    // (the TMA final pass stores this element's update through the tile copy)
+                    if constexpr (!(TMA && MODE == COL_FINAL)) a.state[(size_t)i * ldc] = w;
+                }
+            }
+        }
+        if constexpr (MODE == COL_RHS) return true;
+        double bsum = 0.0;
+        bool bad = false;
+        constexpr int EB = E < 4 ? E : (MODE == COL_FINAL && (SCH == SCH_CN || SCH == SCH_CNX) && E >= 8) ? 8 : 4;
+        const Real bc = (Real)a.b_cur;
+        const Real adt = (Real)(a.dt * a.a_next);
+#pragma unroll
+        for (int m0 = 0; m0 < E; m0 += EB) {
+            C w[EB], acc[EB], xs[SCH == SCH_EX ? EB : 1], p0[SCH == SCH_AB4 ? EB : 1], p1[SCH == SCH_AB4 ? EB : 1],
+                p2[SCH == SCH_AB4 ? EB : 1];
+            double2 f[MODE == COL_FINAL ? EB : 1];
+            Real br[SCH == SCH_EX ? EB : 1];
+            if constexpr (MODE == COL_FINAL && SCH != SCH_EX) {
+                // Crank-Nicolson factors (solver.c:853), from the table
+                if (SCH != SCH_AB4 || a.cn) {
 #pragma unroll
                     for (int m = 0; m < EB; ++m) f[m] = a.cn[(size_t)(t + T * (m0 + m)) * ldc + kyc];
                 }
+            }
+            if constexpr (SCH == SCH_AB4) {
 #pragma unroll
                 for (int m = 0; m < EB; ++m) {
-                    const int q = (t + T * (m0 + m)) * TC + c;
-                    w[m] = pre0[q];
-                    if (MODE == COL_FINAL || !a.first) acc[m] = pre1[q];
+                    const size_t g = (size_t)(t + T * (m0 + m)) * ldc + kyc;
+                    p0[m] = a.h0[g];
+                    p1[m] = a.h1[g];
+                    p2[m] = a.h2[g];
                 }
+            }
+            if constexpr (SCH == SCH_EX) {
+                if (a.lin_stage) {
 #pragma unroll
-                for (int m = 0; m < EB; ++m) {
-                    const int i = t + T * (m0 + m);
-                    const int q = i * TC + c;
-                    const C r = v[0][m0 + m];
-                    if constexpr (MODE == COL_STAGE) {
-                        const C ac = a.first ? cscale(r, bc) : cadd(acc[m], cscale(r, bc));
-                        if constexpr (TMA) pre1[q] = ac;  // staged for the tile store
-                        else if (valid) a.acc[(size_t)i * ldc + ky] = ac;
-                        pre0[q] = cadd(w[m], cscale(r, adt));
-                    } else {
-                        C wn = cn_update<C>(w[m], cadd(acc[m], cscale(r, bc)), (Real)f[m].x, (Real)f[m].y);
-                        if (m0 + m == 0 && i == 0 && ky == 0) wn = cmake<C>(0, 0);
-                        if constexpr (TMA) pre0[q] = wn;  // staged for the tile store
-                        else if (valid) a.state[(size_t)i * ldc + ky] = wn;
-                        if (valid) {
-                            const double mag = fabs((double)wn.x) + fabs((double)wn.y);
-                            bad |= !isfinite(mag);
-                            bsum += (ky == 0 || 2 * ky == N) ? mag : 2.0 * mag;
-                        }
+                    for (int m = 0; m < EB; ++m) {
+                        br[m] = linear(m0 + m);
+                        if (a.xin) xs[m] = a.xin[(size_t)(t + T * (m0 + m)) * ldc + kyc];
                     }
                 }
             }
-            if constexpr (MODE == COL_STAGE) {
-                if (ky == 0) {
 #pragma unroll
-                    for (int m = 0; m < E; ++m) a.col0_out[t + T * m] = pre0[(t + T * m) * TC + c];
-                }
+            for (int m = 0; m < EB; ++m) {
+                const int q = (t + T * (m0 + m)) * TC + c;
+                w[m] = pre0[q];
+                if (need_acc) acc[m] = pre1[q];
             }
-        } else {
-        // The epilogue runs as a rolled loop over this thread's elements (one
-        // copy of its code): the transform output is parked in the exchange
-        // buffer, in slots only this thread touches.
 #pragma unroll
-        for (int m = 0; m < E; ++m) sm[(t + T * m) * TC + c] = v[0][m];
-        if constexpr (need_state) cp_async_wait_all();
-#pragma unroll 4
-        for (int m = 0; m < E; ++m) {
-            const int i = t + T * m;
-            const int q = i * TC + c;
-            const int kx = (i <= N / 2) ? i : i - N;
-            const int k2 = kx * kx + ky * ky;
-            // normalisation and zero mean (solver.c:998-1013)
-            C r = (kx == 0 && ky == 0) ? cmake<C>(0, 0) : cscale(sm[q], a.norm2);
-            // dealiasing (solver.c:1039-1099)
-            if (FAST || a.dealias == 0) {
-                if (k2 >= a.kmax_sqr || (a.kolm && kx == 0)) r = cmake<C>(0, 0);
-            } else {
-                r = cscale(r, houli_filter<Real>(kx, ky, N, N, a.houli_int));
-            }
-            // forcing (solver.c:1022-1027)
-            if (a.has_force && i == a.force_i && ky == a.force_j) r = cadd(r, a.force_val);
-            if constexpr (!FAST) {
-                if (a.force_field) r = cadd(r, a.force_field[(size_t)i * ldc + kyc]);
-            }
-            if constexpr (MODE == COL_RHS) {
-                // stage derivative with the explicit linear term (Dormand-Prince
-                // stages): r -= bracket(|k|^2) X, X the RHS input
-                if (a.lin_stage == 2 && a.xin && k2 != 0)
-                    r = csub(r, cscale(a.xin[(size_t)i * ldc + kyc], (Real)lin_bracket(a.lin, (double)k2)));
-            }
-            if constexpr (!FAST) {
-                if (a.rhs_store && valid) a.rhs_store[(size_t)i * ldc + ky] = r;
-            }
-            // ForceConjugacy side effect on the state (solver.c:1031, 2096-2103)
-            C w = cmake<C>(0, 0);
-            if constexpr (need_state) w = pre0[q];
-            if (a.conj_mode && ky == 0 && kx < 0 && valid) {
-                w = cconj(a.conj_src[(size_t)(-kx) * a.conj_stride]);
-                // (the TMA final pass stores this element's update through the tile copy)
-                if constexpr (!(TMA && MODE == COL_FINAL)) a.state[(size_t)i * ldc] = w;
-            }
-            if constexpr (need_state) {
-                // linear term of explicit RK4 stages (solver.c:664-684)
-                if (!FAST && a.lin_stage && k2 != 0) {
-                    const C xs = a.xin ? a.xin[(size_t)i * ldc + kyc] : w;
-                    const double br = lin_bracket(a.lin, (double)k2);
-                    if (a.lin_stage == 1) r = cadd(r, cscale(xs, (Real)(a.dt * br)));
-                    else r = csub(r, cscale(xs, (Real)br));
+            for (int m = 0; m < EB; ++m) {
+                const int i = t + T * (m0 + m);
+                const int q = i * TC + c;
+                const bool mean = m0 + m == 0 && i == 0 && ky == 0;
+                C r = v[0][m0 + m];
+                if constexpr (SCH == SCH_EX) {
+                    // linear term of explicit RK4 stages (solver.c:664-684)
+                    if (a.lin_stage && !mean) {
+                        const C x = a.xin ? xs[m] : w[m];
+                        r = a.lin_stage == 1 ? cadd(r, cscale(x, br[m])) : csub(r, cscale(x, br[m]));
+                    }
                 }
                 if constexpr (MODE == COL_STAGE) {
-                    C acc;
-                    if (a.first) acc = cscale(r, (Real)a.b_cur);
-                    else acc = cadd(pre1[q], cscale(r, (Real)a.b_cur));
-                    if constexpr (TMA) pre1[q] = acc;  // staged for the tile store
-                    else if (valid) a.acc[(size_t)i * ldc + ky] = acc;
-                    const Real adt = (Real)(a.dt * a.a_next);
-                    const C nx = cadd(w, cscale(r, adt));
+                    const C ac = a.first ? cscale(r, bc) : cadd(acc[m], cscale(r, bc));
+                    if constexpr (TMA) pre1[q] = ac;  // staged for the tile store
+                    else if (valid) a.acc[(size_t)i * ldc + ky] = ac;
+                    const C nx = cadd(w[m], cscale(r, adt));
                     pre0[q] = nx;
-                    if (valid) {
-                        if (ky == 0) a.col0_out[i] = nx;
-                        if constexpr (!FAST) {
-                            if (a.out) a.out[(size_t)i * ldc + ky] = nx;
-                        }
-                    }
-                } else {  // COL_FINAL
-                    C tot;
-                    if (!FAST && a.scheme >= 2) {
-                        // AB4 (solver.c:303-331): 55/24 N_n - 59/24 N_n-1 + 37/24 N_n-2 - 3/8 N_n-3
-                        const size_t g = (size_t)i * ldc + kyc;
-                        const C p2 = a.h2[g], p1 = a.h1[g], p0 = a.h0[g];
-                        if (a.scheme == 3) {
-                            const Real dt = (Real)a.dt;
-                            tot = cadd(cadd(cadd(cscale(r, dt * (Real)(55.0 / 24.0)), cscale(p2, dt * (Real)(-59.0 / 24.0))),
-                                            cscale(p1, dt * (Real)(37.0 / 24.0))),
-                                       cscale(p0, dt * (Real)(-3.0 / 8.0)));
-                        } else {
-                            tot = cadd(cadd(cadd(cscale(r, (Real)(55.0 / 24.0)), cscale(p2, (Real)(-59.0 / 24.0))),
-                                            cscale(p1, (Real)(37.0 / 24.0))),
-                                       cscale(p0, (Real)(-3.0 / 8.0)));
-                        }
-                    } else {
-                        tot = cadd(pre1[q], cscale(r, (Real)a.b_cur));
-                    }
+                    if (SCH == SCH_EX && a.out && valid) a.out[(size_t)i * ldc + ky] = nx;
+                } else {
                     C wn;
-                    if (kx == 0 && ky == 0) {
-                        wn = cmake<C>(0, 0);
-                    } else if (!FAST && a.scheme == 1) {
-                        wn = cadd(w, cscale(tot, (Real)(a.dt / 6.0)));
-                    } else if (!FAST && a.scheme == 3) {
-                        wn = cadd(w, tot);
+                    if constexpr (SCH == SCH_CN || SCH == SCH_CNX) {
+                        wn = cn_update<C>(w[m], cadd(acc[m], cscale(r, bc)), (Real)f[m].x, (Real)f[m].y);
+                    } else if constexpr (SCH == SCH_EX) {
+                        wn = cadd(w[m], cscale(cadd(acc[m], cscale(r, bc)), (Real)(a.dt / 6.0)));
                     } else {
-                        // Crank-Nicolson factors (solver.c:853), from the table
-                        const double2 f = a.cn[(size_t)i * ldc + kyc];
-                        wn = cn_update<C>(w, tot, (Real)f.x, (Real)f.y);
+                        // AB4 (solver.c:303-331): 55/24 N_n - 59/24 N_n-1 + 37/24 N_n-2 - 3/8 N_n-3,
+                        // explicit (Euler system: no table) or with the Crank-Nicolson factors
+                        const Real dt = a.cn ? (Real)1 : (Real)a.dt;
+                        const C tot = cadd(cadd(cadd(cscale(r, dt * (Real)(55.0 / 24.0)), cscale(p2[m], dt * (Real)(-59.0 / 24.0))),
+                                                cscale(p1[m], dt * (Real)(37.0 / 24.0))),
+                                           cscale(p0[m], dt * (Real)(-3.0 / 8.0)));
+                        wn = a.cn ? cn_update<C>(w[m], tot, (Real)f[m].x, (Real)f[m].y) : cadd(w[m], tot);
                     }
-                    if (!FAST && a.phase_only && (kx != 0 || ky != 0)) {
-                        // amplitude reset of the phase-only model (solver.c:822-824, 855-857):
-                        // w_new *= |w_old| / |w_new|; a mode updated to exactly 0 stays 0
-                        const double an = hypot((double)wn.x, (double)wn.y);
-                        if (an > 0.0) {
-                            const double r = hypot((double)w.x, (double)w.y) / an;
-                            wn = cmake<C>((Real)((double)wn.x * r), (Real)((double)wn.y * r));
+                    if (mean) wn = cmake<C>(0, 0);
+                    if constexpr (GEN) {
+                        if (a.phase_only && !mean) {
+                            // amplitude reset of the phase-only model (solver.c:822-824, 855-857):
+                            // w_new *= |w_old| / |w_new|; a mode updated to exactly 0 stays 0
+                            const double an = hypot((double)wn.x, (double)wn.y);
+                            if (an > 0.0) {
+                                const double s = hypot((double)w[m].x, (double)w[m].y) / an;
+                                wn = cmake<C>((Real)((double)wn.x * s), (Real)((double)wn.y * s));
+                            }
                         }
                     }
                     if constexpr (TMA) pre0[q] = wn;  // staged for the tile store
+                    else if (valid) a.state[(size_t)i * ldc + ky] = wn;
                     if (valid) {
-                        if constexpr (!TMA) a.state[(size_t)i * ldc + ky] = wn;
                         const double mag = fabs((double)wn.x) + fabs((double)wn.y);
                         bad |= !isfinite(mag);
                         bsum += (ky == 0 || 2 * ky == N) ? mag : 2.0 * mag;
@@ -861,8 +860,13 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                 }
             }
         }
+        if constexpr (MODE == COL_STAGE) {
+            if (ky == 0) {
+#pragma unroll
+                for (int m = 0; m < E; ++m) a.col0_out[t + T * m] = pre0[(t + T * m) * TC + c];
+            }
         }
-        // the next transform's first stage writes other threads' parked slots
+        // the staged results are complete before one thread stores them
         if constexpr (TMA) fence_async_smem();
         __syncthreads();
         if constexpr (TMA && MODE == COL_STAGE) {
@@ -916,39 +920,34 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             }
             return true;
         }
-        if constexpr (MODE == COL_RHS) return true;
     }
 
-    if (!FAST && dead && narrow) return true;
     if constexpr (TMA) derived_ifft_tma<Real, N, TC, SPLIT>(pre0, sm, maps, tile, ky, t, c, seed, MODE == COL_STAGE);
     else derived_ifft<Real, N, TC>(pre0, sm, a.f0, a.f1, a.f2, a.f3, ldc, ky, valid, t, c, seed);
     return true;
 }
 
 // Column pass of one field.  Grid: ceil(nyf / TC) blocks; block: T * TC threads.
-// FAST: the epilogue compiled for the common step only (2/3 dealiasing, no
-// listed-mode forcing, no stored RHS, no explicit linear term, Crank-Nicolson
-// update of the full model); the launcher picks it when the arguments allow.
-template <typename Real, int N, int TC, int MODE, bool FAST = false>
+template <typename Real, int N, int TC, int MODE, int SCH>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_kernel(ColArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    col_body<Real, N, TC, MODE, FAST>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, smraw);
+    col_body<Real, N, TC, MODE, SCH, true>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, smraw);
 }
 
-// Column pass with TMA tile loads and stores (FAST P1, STAGE and FINAL).  Shared
-// memory: ColSmem::bytes_tma() + 1024 (the body's base is rounded up to 1024 bytes).
-template <typename Real, int N, int TC, int MODE>
+// Column pass with TMA tile loads and stores, without the rarely used parts (see
+// col_tma_ok).  Shared memory: ColSmem::bytes_tma() + 1024 (the body's base is
+// rounded up to 1024 bytes).
+template <typename Real, int N, int TC, int MODE, int SCH>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_tma_kernel(ColArgs<Real> a, const __grid_constant__ ColMaps maps) {
     extern __shared__ __align__(16) unsigned char smraw[];
     unsigned char* sm = smraw + ((1024u - ((unsigned)__cvta_generic_to_shared(smraw) & 1023u)) & 1023u);
-    col_body<Real, N, TC, MODE, true, true, true>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, sm, &maps);
+    col_body<Real, N, TC, MODE, SCH, false, true, true>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, sm, &maps);
 }
 
-// Whether a stage or final column pass can run the FAST epilogue.
+// Whether a column pass can run without its GEN parts.
 template <typename Real>
-inline bool col_fast_ok(const ColArgs<Real>& a) {
-    return a.dealias == 0 && !a.force_field && !a.rhs_store && a.lin_stage == 0 && !a.xin && !a.out &&
-           a.scheme == 0 && !a.phase_only;
+inline bool col_tma_ok(const ColArgs<Real>& a) {
+    return !a.force_field && !a.phase_only && (a.dealias == 0 || a.filt) && (a.lin_stage == 0 || a.lint);
 }
 
 template <typename Real>
@@ -1166,6 +1165,32 @@ static __global__ void cn_table_kernel(double2* cn, int nx, int nyf, int ldc, do
             if (ky >= kc && !(isfinite(f.x) && isfinite(f.y))) atomicOr(odd, 1);
         }
         cn[(size_t)i * ldc + ky] = f;
+    }
+}
+
+// Brackets of the explicit linear term per mode (times scale): see ColArgs::lint.
+// *odd as in cn_table_kernel.
+static __global__ void lin_table_kernel(double* lt, int nx, int nyf, int ldc, double scale, LinOp lin, int kc, int* odd) {
+    const long long n = (long long)nx * nyf;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(q / nyf), ky = (int)(q % nyf);
+        const int kx = (i <= nx / 2) ? i : i - nx;
+        double br = 0.0;
+        if (kx != 0 || ky != 0) {
+            br = scale * lin_bracket(lin, (double)(kx * kx + ky * ky));
+            if (ky >= kc && !isfinite(br)) atomicOr(odd, 1);
+        }
+        lt[(size_t)i * ldc + ky] = br;
+    }
+}
+
+// Hou-Li factors per mode: see ColArgs::filt.
+template <typename Real>
+__global__ void filter_table_kernel(Real* ft, int n, int nyf, int ldc, int quirk) {
+    const long long tot = (long long)n * nyf;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(q / nyf), ky = (int)(q % nyf);
+        ft[(size_t)i * ldc + ky] = houli_filter<Real>((i <= n / 2) ? i : i - n, ky, n, n, quirk);
     }
 }
 

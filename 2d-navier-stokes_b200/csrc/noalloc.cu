@@ -42,19 +42,6 @@ std::mutex g_mu;
 void* g_scratch_ptr[kMaxDevices] = {};
 bool g_size_ready[kMaxDevices][5] = {};  // N = 16, 32, 64, 128, 256
 
-// Dispatch over the sizes this entry point supports (16..256).
-template <typename F>
-bool with_small_size(int n, F&& f) {
-    switch (n) {
-        case 16: f(Launch<double, 16>{}); return true;
-        case 32: f(Launch<double, 32>{}); return true;
-        case 64: f(Launch<double, 64>{}); return true;
-        case 128: f(Launch<double, 128>{}); return true;
-        case 256: f(Launch<double, 256>{}); return true;
-        default: return false;
-    }
-}
-
 int size_slot(int n) {
     switch (n) {
         case 16: return 0;
@@ -89,9 +76,7 @@ ns2d_status setup(int dev, int n, double2** base) {
     const int slot = size_slot(n);
     if (slot < 0) return NS2D_ERR_UNSUPPORTED;
     if (!g_size_ready[dev][slot]) {
-        cudaError_t e = cudaSuccess;
-        with_small_size(n, [&](auto L) { e = decltype(L)::setup(); });
-        if (e != cudaSuccess) return NS2D_ERR_CUDA;
+        if (engine_ops<double>(n)->setup() != cudaSuccess) return NS2D_ERR_CUDA;
         g_size_ready[dev][slot] = true;
     }
     *base = (double2*)g_scratch_ptr[dev];
@@ -159,7 +144,8 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
         a.force_val = make_double2(-0.5 * p->force_scale * (double)p->force_k, 0.0);
     }
     a.norm2 = std::pow(1.0 / (double)(n * n), 2.0);
-    with_small_size(n, [&](auto L) { decltype(L)::col(COL_P1, a, st); });
+    const EngineOps<double>* ops = engine_ops<double>(n);
+    ops->col(COL_P1, SCH_CN, a, st, nullptr);
 
     RowArgs<double> r{};
     r.f0 = f[0];
@@ -172,12 +158,12 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
     r.nrows = n;
     r.kc = a.kc;
     r.status = nullptr;
-    with_small_size(n, [&](auto L) { decltype(L)::row(r, st); });
+    ops->row(r, st);
 
     a.src = nl;
     a.rhs_store = (double2*)d_rhs;  // no state here: the conjugacy side effect is not applied
     a.conj_mode = 0;
-    with_small_size(n, [&](auto L) { decltype(L)::col(COL_RHS, a, st); });
+    ops->col(COL_RHS, SCH_CN, a, st, nullptr);
     // no error was pending on entry, so one found now is a launch of this call
     if (cudaGetLastError() != cudaSuccess) return NS2D_ERR_CUDA;
     return NS2D_OK;

@@ -118,3 +118,26 @@ def test_reverse_sweep_after_the_state_was_replaced():
         grads.append(s.adjoint_backward(lam))
         s.close()
     assert np.array_equal(grads[0], grads[1])
+
+
+@pytest.mark.parametrize("quirks", [abi.QUIRKS_REFERENCE, abi.QUIRKS_REFERENCE & ~abi.QUIRK_HOU_LI_INT & ~abi.QUIRK_RK4_LINEAR])
+@pytest.mark.parametrize("integ", [abi.RK4CN, abi.RK4, abi.AB4])
+@pytest.mark.parametrize("n", [256, 512])
+def test_houli_steps_match_oracle(n, integ, quirks):
+    """Hou-Li dealiasing empties no column; its factors (integer or real ratios)
+    and the explicit linear term's brackets come from per-mode tables."""
+    dt = 1e-4
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, ekmn_drag_flag=1, integrator=integ, dealias=abi.DEALIAS_HOU_LI,
+                           quirks=quirks, dt=dt)
+    w0 = initial.decaying(n, seed=6, k0=n / 10.0)
+    s = Solver(p)
+    s.set_w_hat(w0)
+    s.step_n(3, dt)
+    s.step_n(2, 0.5 * dt)  # another table
+    o = Oracle(p, threads=8)
+    o.set_w_hat(w0)
+    for k in range(5):
+        d = dt if k < 3 else 0.5 * dt
+        o.ab4_step(d, k + 1) if integ == abi.AB4 else o.rk4_step(d)
+    assert rel_err(s.get_w_hat(), o.get_w_hat()) <= 1e-12
+    s.close()
