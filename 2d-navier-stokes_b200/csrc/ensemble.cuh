@@ -74,12 +74,14 @@ __device__ __forceinline__ void ens_apply_stage(ColArgs<Real>& a, const EnsMembe
     }
 }
 
-// Resident blocks per SM the ensemble kernels are compiled for: at most 128
-// registers a thread in FP32 (two 256-thread or four 128-thread blocks), the
-// register need of one FP64 body otherwise.
+// Resident blocks per SM the ensemble kernels are compiled for, now that every
+// size's transforms hold eight elements a thread: in FP32 three 256-thread (six
+// 128-thread) blocks, 85 registers a thread (a step of the 64-member ensemble
+// 292 us; two blocks 317, four 314 with spills), in FP64 two of 256, 128 registers
+// (453 us; one 547, three 533).
 template <typename Real, int THREADS>
 struct EnsMinBlocks {
-    static constexpr int value = sizeof(Real) == 4 ? 512 / THREADS : 256 / THREADS;
+    static constexpr int value = sizeof(Real) == 4 ? 768 / THREADS : 512 / THREADS;
 };
 
 // SCH, GEN: as col_body.  TMA: the tiles move by TMA copies through maps[2 m + v], the
