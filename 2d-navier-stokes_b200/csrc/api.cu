@@ -723,6 +723,7 @@ ns2d_status c2r_impl(ns2d_handle* h, const InvField<Real>* fields, int nf, int o
     ia.nyf = h->nyf;
     ia.ldc = h->ldc;
     ia.tw = (const C*)h->tw;
+    ia.maxbits = op != R2_STORE ? h->dmax : nullptr;
     engine_ops<Real>(h->nx)->col_inv(ia, h->stream);
     h->launches++;
     RowC2RArgs<Real> ra;
@@ -737,7 +738,6 @@ ns2d_status c2r_impl(ns2d_handle* h, const InvField<Real>* fields, int nf, int o
     ra.maxbits = h->dmax;
     ra.outA = outA;
     ra.outB = outB;
-    if (op != R2_STORE) CK(h, cudaMemsetAsync(h->dmax, 0, sizeof(unsigned long long), h->stream));
     engine_ops<Real>(h->nx)->row_c2r(op, ra, h->stream);
     h->launches++;
     CKL(h);
@@ -752,13 +752,12 @@ ns2d_status c2r_impl(ns2d_handle* h, const InvField<Real>* fields, int nf, int o
     return NS2D_OK;
 }
 
-// Velocity of the state into the persistent reference-layout u_hat buffer
-// (regular or CFL-quirk row index), then c2r with a max reduction.
+// Largest velocity component (GetMaxData): the velocity spectrum into the
+// persistent reference-layout u_hat buffer, then c2r with a max reduction.
 template <typename Real>
-ns2d_status velocity_c2r(ns2d_handle* h, int scrambled, int op, double* result) {
+ns2d_status max_velocity(ns2d_handle* h, double* result) {
     using C = Cplx<Real>;
-    cfl_scramble_kernel<Real><<<296, 256, 0, h->stream>>>((const C*)h->state, h->ldc, (C*)h->uhat_ref, h->nx, h->ny,
-                                                          scrambled);
+    velocity_spec_kernel<Real><<<296, 256, 0, h->stream>>>((const C*)h->state, h->ldc, (C*)h->uhat_ref, h->nx, h->ny);
     h->launches++;
     CKL(h);
     InvField<Real> f[2];
@@ -769,7 +768,7 @@ ns2d_status velocity_c2r(ns2d_handle* h, int scrambled, int op, double* result) 
         f[k].es = 2;
         f[k].op = 0;
     }
-    return c2r_impl<Real>(h, f, 2, op, nullptr, nullptr, result);
+    return c2r_impl<Real>(h, f, 2, R2_MAXABS, nullptr, nullptr, result);
 }
 
 template <typename Real>
@@ -787,14 +786,26 @@ ns2d_status max_data_impl(ns2d_handle* h, int kind, double* out) {
     if (kind == NS2D_MAX_VEL) {
         // run_data->u_hat is rewritten with the regular index (solver.c:2184-2196);
         // the CFL path later reads the entries its own index misses.
-        return velocity_c2r<Real>(h, 0, R2_MAXABS, out);
+        return max_velocity<Real>(h, out);
     }
     return fail(h, NS2D_ERR_UNSUPPORTED, "NS2D_MAX_VORT_FOUR is evaluated by ns2d_get_max_data on the host copy");
 }
 
 template <typename Real>
 ns2d_status cfl_impl(ns2d_handle* h, double* scales_convect) {
-    return velocity_c2r<Real>(h, quirk(h, NS2D_QUIRK_CFL_INDEX) ? 1 : 0, R2_CFL, scales_convect);
+    using C = Cplx<Real>;
+    // the velocity spectra are formed as the inverse x-transforms load the state
+    const bool q = quirk(h, NS2D_QUIRK_CFL_INDEX);
+    InvField<Real> f[2];
+    std::memset(f, 0, sizeof(f));
+    for (int k = 0; k < 2; ++k) {
+        f[k].p = (const C*)h->state;
+        f[k].rs = h->ldc;
+        f[k].es = 1;
+        f[k].op = q ? 3 + k : 1 + k;
+        f[k].keep = (const C*)h->uhat_ref;
+    }
+    return c2r_impl<Real>(h, f, 2, R2_CFL, nullptr, nullptr, scales_convect);
 }
 template <typename Real>
 void fill_twiddles(std::vector<Cplx<Real>>& tw, int n) {
@@ -860,7 +871,7 @@ ns2d_status create_impl(ns2d_handle* h) {
     build_col_maps<Real>(h);
     h->resident = resident_setup(h->nx, h->fp32);
     CK(h, cudaFuncSetAttribute((const void*)diag_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(sizeof(double) * (8 * (size_t)h->n_spect + DG_N * 8))));
+                               (int)diag_smem(h->n_spect)));
     std::vector<C> tw;
     fill_twiddles<Real>(tw, h->nx);
     CK(h, cudaMalloc(&h->tw, sizeof(C) * h->nx));
@@ -1152,8 +1163,7 @@ ns2d_status measurables_impl(ns2d_handle* h, ns2d_measures* out, double* spectra
     d.ffield = h->ffield_on ? (const C*)h->ffield : nullptr;
     d.n_spect = ns;
     d.out = h->ddiag;
-    const size_t smem = sizeof(double) * (8 * (size_t)ns + DG_N * 8);
-    diag_kernel<Real><<<148, 256, smem, h->stream>>>(d);
+    diag_kernel<Real><<<148, kDiagThreads, diag_smem(ns), h->stream>>>(d);
     h->launches++;
     CKL(h);
     std::vector<double> raw(nout);

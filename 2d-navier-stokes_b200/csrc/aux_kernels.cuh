@@ -7,7 +7,8 @@ namespace ns2d {
 
 // Spectral source of one inverse x-FFT: element (i, j) at p[i*rs + j*es];
 // op 0 = as is, 1 = u_hat = ky (i/k^2) w, 2 = v_hat = -kx (i/k^2) w
-// (Solver/src/solver.c:2184-2196, 2393-2410).
+// (Solver/src/solver.c:2184-2196, 2393-2410), 3 and 4 = the same two as
+// GetTimestep forms them in its u_hat buffer (cfl_velocity).
 template <typename Real>
 struct InvField {
     using C = typename Cx<Real>::T;
@@ -15,7 +16,29 @@ struct InvField {
     long long rs, es;
     int op;
     C* dst;  // [nx][ldc] x-space output
+    const C* keep;  // op 3, 4: the u_hat buffer ([nx][nyf][2])
 };
+
+// u_hat (comp 0) or v_hat (comp 1) at flat position e of the half spectrum as
+// GetTimestep's row index leaves them (Solver/src/solver.c:2393-2410): its loop over
+// (i, j) writes position i Ny/2 + 1 + j with the wavenumbers of (i, j) and the state
+// at that same position, and where rows overlap by one element the later row's
+// value stays; so position e in 1..N Ny/2 + 1 belongs to i = (e-1)/(Ny/2),
+// j = (e-1) mod (Ny/2), the last one to (Nx-1, Ny/2).  The positions it never reaches
+// keep what the buffer held (GetMaxData's velocity, or 0).
+template <typename C, int N>
+__device__ __forceinline__ C cfl_velocity(int e, int comp, C w, const C* keep) {
+    using Real = decltype(C::x);
+    constexpr int H = N / 2, LAST = N * H + 1;
+    if (e < 1 || e > LAST) return keep[2 * (size_t)e + comp];
+    const int i = e == LAST ? N - 1 : (e - 1) / H;
+    const int j = e == LAST ? H : (e - 1) % H;
+    const int kx = (i <= N / 2) ? i : i - N;
+    if (kx == 0 && j == 0) return cmake<C>(0, 0);
+    const double inv = 1.0 / (double)(kx * kx + j * j);
+    const Real s = (Real)((double)(comp == 0 ? j : kx) * inv);
+    return comp == 0 ? cmake<C>(-s * w.y, s * w.x) : cmake<C>(s * w.y, -s * w.x);
+}
 
 template <typename Real>
 struct InvArgs {
@@ -23,8 +46,7 @@ struct InvArgs {
     int nf;
     int nyf, ldc;
     const typename Cx<Real>::T* tw;
-    // op 1/2 wavenumbers for a scrambled index: kx from row i of the loop, the
-    // source element from the flat position (see cfl_scramble_kernel)
+    unsigned long long* maxbits;  // cleared here for the row pass's maximum, may be null
 };
 
 template <typename Real, int N, int TC>
@@ -40,6 +62,7 @@ __global__ void __launch_bounds__(Plan<N>::T * TC) col_inv_kernel(InvArgs<Real> 
     const bool valid = ky < a.nyf;
     const int kyc = valid ? ky : 0;
     const auto seed = twiddle_seeds<N>(a.tw, t);
+    if (a.maxbits && blockIdx.x == 0 && threadIdx.x == 0) *a.maxbits = 0ull;
     for (int f = 0; f < a.nf; ++f) {
         const InvField<Real> F = a.f[f];
         C v[E];
@@ -48,7 +71,9 @@ __global__ void __launch_bounds__(Plan<N>::T * TC) col_inv_kernel(InvArgs<Real> 
             const int i = t + T * m;
             const int kx = (i <= N / 2) ? i : i - N;
             C w = valid ? F.p[(long long)i * F.rs + (long long)kyc * F.es] : cmake<C>(0, 0);
-            if (F.op != 0) {
+            if (F.op >= 3) {
+                if (valid) w = cfl_velocity<C, N>(i * a.nyf + ky, F.op - 3, w, F.keep);
+            } else if (F.op != 0) {
                 if (kx == 0 && ky == 0) {
                     w = cmake<C>(0, 0);
                 } else {
@@ -146,37 +171,30 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) row_c2r_kernel(RowC2RA
     }
 }
 
-// CFL velocity spectrum with the reference's row index tmp = (i*Ny)/2 + 1
-// (Solver/src/solver.c:2393-2410), written into a persistent buffer with the
-// reference's interleaved [nx][nyf][2] layout; the state is read at the same
-// scrambled flat position.  Entries the loop never reaches keep their previous
-// contents, as in the reference.  Consecutive rows overlap by one element;
-// the reference's sequential loop leaves row i+1's j = 0 value there, so the
-// last element of every row but the last is not written here.
+// Velocity spectrum of the state with the regular index (GetMaxData, Solver/src/
+// solver.c:2184-2196) into the persistent buffer with the reference's interleaved
+// [nx][nyf][2] layout, which GetTimestep's own index partly leaves in place.
 template <typename Real>
-__global__ void cfl_scramble_kernel(const typename Cx<Real>::T* __restrict__ state, int ldc,
-                                    typename Cx<Real>::T* __restrict__ uhat, int nx, int ny, int quirk) {
+__global__ void velocity_spec_kernel(const typename Cx<Real>::T* __restrict__ state, int ldc,
+                                     typename Cx<Real>::T* __restrict__ uhat, int nx, int ny) {
     using C = typename Cx<Real>::T;
     const int nyf = ny / 2 + 1;
     const long long n = (long long)nx * nyf;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(q / nyf);
-        const int j = (int)(q % nyf);
-        if (quirk && j == nyf - 1 && i < nx - 1) continue;
-        const long long idx = quirk ? ((long long)i * ny / 2 + 1 + j) : q;
+        const int ky = (int)(q % nyf);
         const int kx = (i <= nx / 2) ? i : i - nx;
-        const int ky = j;
         C u = cmake<C>(0, 0), v = cmake<C>(0, 0);
         if (kx != 0 || ky != 0) {
-            const C w = state[(size_t)(idx / nyf) * ldc + (size_t)(idx % nyf)];
+            const C w = state[(size_t)i * ldc + ky];
             const double inv = 1.0 / (double)(kx * kx + ky * ky);
             const Real su = (Real)((double)ky * inv);
             const Real sv = (Real)((double)kx * inv);
             u = cmake<C>(-su * w.y, su * w.x);
             v = cmake<C>(sv * w.y, -sv * w.x);
         }
-        uhat[2 * idx + 0] = u;
-        uhat[2 * idx + 1] = v;
+        uhat[2 * q + 0] = u;
+        uhat[2 * q + 1] = v;
     }
 }
 

@@ -314,7 +314,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
     for (int n : e->sizes) nspect_max = std::max(nspect_max, (int)std::round(std::sqrt(2.0 * (n / 2.0) * (n / 2.0)) + 1));
     ECK(e, alloc(sizeof(double) * (DG_N + 8 * (size_t)nspect_max), (void**)&e->ddiag));
     ECK(e, cudaFuncSetAttribute((const void*)diag_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(double) * (8 * (size_t)nspect_max + DG_N * 8))));
+                                (int)diag_smem(nspect_max)));
     // work items of each block-size choice, largest grids first
     // (longest-processing-time order)
     std::vector<int> order(e->n);
@@ -600,7 +600,7 @@ ns2d_status meas_t(ns2d_ensemble* e, int m, ns2d_measures* out) {
     d.enst_quirk = (e->p.quirks & NS2D_QUIRK_ENST_DISS) ? 1 : 0;
     d.n_spect = ns;
     d.out = e->ddiag;
-    diag_kernel<Real><<<148, 256, sizeof(double) * (8 * (size_t)ns + DG_N * 8), e->stream>>>(d);
+    diag_kernel<Real><<<148, kDiagThreads, diag_smem(ns), e->stream>>>(d);
     e->launches++;
     ECK(e, cudaGetLastError());
     std::vector<double> raw(DG_N);
