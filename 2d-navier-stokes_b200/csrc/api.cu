@@ -565,26 +565,14 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
     if (!euler) {
         if (ns2d_status sl = ensure_lin(h, 1.0, branch)) return sl;
     }
-    void* y0 = h->dp[7];
+    // Each stage's column pass forms its derivative k_s and, from the state (y0
+    // until the end) and k_0..k_s, the next stage input with its derived spectra.
     void* x = h->dp[8];
-    CK(h, cudaMemcpyAsync(y0, h->state, h->field_bytes, cudaMemcpyDeviceToDevice, h->stream));
+    ColArgs<Real> a;
+    fill_common<Real>(h, a, branch);
+    a.src = (const C*)h->state;
+    launch_col<Real>(h, COL_P1, a);
     for (int s = 0; s < 7; ++s) {
-        const void* xs = y0;
-        if (s > 0) {
-            DpCoef cf{};
-            cf.n = s;
-            for (int r = 0; r < s; ++r) cf.c[r] = A[s - 1][r];
-            const C* k[6];
-            for (int r = 0; r < 6; ++r) k[r] = (const C*)h->dp[r];
-            dp_combine_kernel<Real><<<296, 256, 0, h->stream>>>((C*)x, (const C*)y0, k[0], k[1], k[2], k[3], k[4],
-                                                               k[5], cf, dt, h->nx, h->nyf, h->ldc);
-            h->launches++;
-            xs = x;
-        }
-        ColArgs<Real> a;
-        fill_common<Real>(h, a, branch);
-        a.src = (const C*)xs;
-        launch_col<Real>(h, COL_P1, a);
         launch_row<Real>(h);
         fill_common<Real>(h, a, branch);
         a.src = (const C*)h->nl;
@@ -592,8 +580,20 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
         a.conj_mode = 0;
         a.lin_stage = euler ? 0 : 2;
         a.lint = euler ? nullptr : h->lint;
-        a.xin = (const C*)xs;
-        launch_col<Real>(h, COL_RHS, a);
+        a.xin = (const C*)(s == 0 ? h->state : x);
+        if (s == 6) {
+            launch_col<Real>(h, COL_RHS, a);
+            break;
+        }
+        a.dt = dt;
+        a.out = (C*)x;
+        a.nk = s;
+        for (int r = 0; r < s; ++r) {
+            a.kd[r] = (const C*)h->dp[r];
+            a.kw[r] = A[s][r];
+        }
+        a.kw[5] = A[s][s];
+        launch_col<Real>(h, COL_STAGE, a, SCH_DP);
     }
     DpCoef b5{}, b4{};
     const double B5[7] = {35.0 / 384.0, 0.0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0, 0.0};
@@ -604,7 +604,7 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
         b4.c[r] = B4[r];
     }
     b5.n = b4.n = 7;
-    dp_final_kernel<Real><<<296, 256, 0, h->stream>>>((C*)h->state, (const C*)y0, (const C* const*)h->dp_kptr, b5, b4,
+    dp_final_kernel<Real><<<296, 256, 0, h->stream>>>((C*)h->state, (const C* const*)h->dp_kptr, b5, b4,
                                                      dt, 1e-7, 1e-7, h->nx, h->nyf, h->ldc, h->dpart);
     h->launches++;
     CKL(h);

@@ -53,6 +53,7 @@ struct Launch {
         set_col<COL_RHS, SCH_CNX>(set);
         set_col<COL_STAGE, SCH_CNX>(set);
         set_col<COL_STAGE, SCH_EX>(set);
+        set_col<COL_STAGE, SCH_DP>(set);
         set_col<COL_FINAL, SCH_CNX>(set);
         set_col<COL_FINAL, SCH_EX>(set);
         set_col<COL_FINAL, SCH_AB4>(set);
@@ -83,7 +84,7 @@ struct Launch {
             col_kernel<Real, N, S::TC, MODE, SCH><<<grid, block, col_smem(), s>>>(a);
         }
     }
-    // scheme: SCH_CN, SCH_EX or SCH_AB4 (stage and final passes); maps: tensor maps
+    // scheme: SCH_CN, SCH_EX, SCH_AB4 or SCH_DP (stage and final passes); maps: tensor maps
     // of the arrays the pass reads and writes (null: per-thread copies).
     static void col(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps = nullptr) {
         switch (mode) {
@@ -91,6 +92,7 @@ struct Launch {
             case COL_RHS: col_one<COL_RHS, SCH_CNX>(a, s, maps); break;
             case COL_STAGE:
                 if (scheme == SCH_EX) col_one<COL_STAGE, SCH_EX>(a, s, maps);
+                else if (scheme == SCH_DP) col_one<COL_STAGE, SCH_DP>(a, s, maps);
                 else col_one<COL_STAGE, SCH_CNX>(a, s, maps);
                 break;
             default:

@@ -37,9 +37,10 @@ enum ColMode : int { COL_P1 = 0, COL_RHS = 1, COL_STAGE = 2, COL_FINAL = 3 };
 // Update schemes of the stage and final column passes: RK4 with Crank-Nicolson
 // factors under the 2/3 rule (the common step), the same with Hou-Li dealiasing or
 // a stored RHS too, explicit RK4 (or Euler system), AB4 (explicit or Crank-
-// Nicolson).  Each is compiled by itself, with what it needs: the common step's
+// Nicolson), a Dormand-Prince stage (the next stage input from the state and all
+// derivatives so far).  Each is compiled by itself, with what it needs: the common step's
 // stage pass at 2048^2 FP64 takes 70.6 us, 77.5 with the second form's branches in.
-enum ColScheme : int { SCH_CN = 0, SCH_CNX = 1, SCH_EX = 2, SCH_AB4 = 3 };
+enum ColScheme : int { SCH_CN = 0, SCH_CNX = 1, SCH_EX = 2, SCH_AB4 = 3, SCH_DP = 4 };
 
 // Linear-operator bracket selection (Solver/src/solver.c:839-856):
 // 1: nu k^2p + a k^2q, 2: nu k^2 + a k^2q, 3: nu k^2p, 4: nu k^2.
@@ -113,6 +114,9 @@ struct ColArgs {
     const C* h0;         // AB4 history: RHS of steps n-3, n-2, n-1 (AB_tmp_nonlin[0..2])
     const C* h1;
     const C* h2;
+    const C* kd[5];      // SCH_DP: the earlier stages' derivatives
+    double kw[6];        // their weights in the next stage input, then this stage's
+    int nk;              // how many there are
     int lin_stage;       // 0 none, 1: rhs += dt D X (quirk), 2: rhs -= D X (corrected)
     LinOp lin;
     const double2* cn;   // COL_FINAL, CN schemes: per-mode ((2-D)/(2+D), 2dt/(2+D)), stride ldc
@@ -553,7 +557,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
     const auto seed = twiddle_seeds<N>(a.tw, t);
     constexpr bool XTRA = SCH != SCH_CN;  // Hou-Li factors, a stored RHS
     constexpr bool need_state = (MODE == COL_STAGE || MODE == COL_FINAL);
-    const bool need_acc = (MODE == COL_STAGE && !a.first) || (MODE == COL_FINAL && SCH != SCH_AB4);
+    const bool need_acc = (MODE == COL_STAGE && SCH != SCH_DP && !a.first) || (MODE == COL_FINAL && SCH != SCH_AB4);
     // TMA: [0] the input, [1] state and accumulator
     __shared__ __align__(8) unsigned long long bar_tile[2];
     auto issue = [&] {
@@ -604,7 +608,10 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         if (narrow && MODE != COL_RHS) {
             if (XTRA && MODE != COL_P1 && a.rhs_store && valid) {
 #pragma unroll
-                for (int m = 0; m < E; ++m) a.rhs_store[(size_t)(t + T * m) * ldc + ky] = cmake<C>(0, 0);
+                for (int m = 0; m < E; ++m) {
+                    a.rhs_store[(size_t)(t + T * m) * ldc + ky] = cmake<C>(0, 0);
+                    if constexpr (SCH == SCH_DP) a.out[(size_t)(t + T * m) * ldc + ky] = cmake<C>(0, 0);
+                }
             }
             return true;
         }
@@ -732,7 +739,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             const double br = lin_bracket(a.lin, (double)(kx * kx + ky * ky));
             return (Real)(a.lin_stage == 1 ? a.dt * br : br);
         };
-        if constexpr (MODE == COL_RHS) {
+        if constexpr (MODE == COL_RHS || SCH == SCH_DP) {
             // stage derivative with the explicit linear term (Dormand-Prince
             // stages): r -= bracket(|k|^2) X, X the RHS input
             if (a.lin_stage == 2 && a.xin) {
@@ -761,13 +768,45 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             }
         }
         if constexpr (MODE == COL_RHS) return true;
+        if constexpr (SCH == SCH_DP) {
+            // next stage input X = w + dt sum_r kw_r k_r, summed in FP64
+#pragma unroll
+            for (int m0 = 0; m0 < E; m0 += 2) {
+                C kk[5][2];
+#pragma unroll
+                for (int r = 0; r < 5; ++r) {
+                    if (r < a.nk) {
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) kk[r][m] = a.kd[r][(size_t)(t + T * (m0 + m)) * ldc + kyc];
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int i = t + T * (m0 + m);
+                    double ar = 0.0, ai = 0.0;
+#pragma unroll
+                    for (int r = 0; r < 5; ++r) {
+                        if (r < a.nk) {
+                            ar += a.kw[r] * (double)kk[r][m].x;
+                            ai += a.kw[r] * (double)kk[r][m].y;
+                        }
+                    }
+                    ar += a.kw[5] * (double)v[0][m0 + m].x;
+                    ai += a.kw[5] * (double)v[0][m0 + m].y;
+                    const C w = pre0[i * TC + c];
+                    const C nx = cmake<C>((Real)((double)w.x + a.dt * ar), (Real)((double)w.y + a.dt * ai));
+                    pre0[i * TC + c] = nx;
+                    if (valid) a.out[(size_t)i * ldc + ky] = nx;
+                }
+            }
+        }
         double bsum = 0.0;
         bool bad = false;
         constexpr int EB = E < 4 ? E : (MODE == COL_FINAL && (SCH == SCH_CN || SCH == SCH_CNX) && E >= 8) ? 8 : 4;
         const Real bc = (Real)a.b_cur;
         const Real adt = (Real)(a.dt * a.a_next);
 #pragma unroll
-        for (int m0 = 0; m0 < E; m0 += EB) {
+        for (int m0 = 0; m0 < (SCH == SCH_DP ? 0 : E); m0 += EB) {
             C w[EB], acc[EB], xs[SCH == SCH_EX ? EB : 1], p0[SCH == SCH_AB4 ? EB : 1], p1[SCH == SCH_AB4 ? EB : 1],
                 p2[SCH == SCH_AB4 ? EB : 1];
             double2 f[MODE == COL_FINAL ? EB : 1];
@@ -860,7 +899,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                 }
             }
         }
-        if constexpr (MODE == COL_STAGE) {
+        if constexpr (MODE == COL_STAGE && SCH != SCH_DP) {
             if (ky == 0) {
 #pragma unroll
                 for (int m = 0; m < E; ++m) a.col0_out[t + T * m] = pre0[(t + T * m) * TC + c];
@@ -869,7 +908,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         // the staged results are complete before one thread stores them
         if constexpr (TMA) fence_async_smem();
         __syncthreads();
-        if constexpr (TMA && MODE == COL_STAGE) {
+        if constexpr (TMA && MODE == COL_STAGE && SCH != SCH_DP) {
             if (threadIdx.x == 0) {
                 tma_store_tile<C, N, TC>(&maps->acc, tile, pre1);
                 bulk_commit();
@@ -922,7 +961,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         }
     }
 
-    if constexpr (TMA) derived_ifft_tma<Real, N, TC, SPLIT>(pre0, sm, maps, tile, ky, t, c, seed, MODE == COL_STAGE);
+    if constexpr (TMA) derived_ifft_tma<Real, N, TC, SPLIT>(pre0, sm, maps, tile, ky, t, c, seed, MODE == COL_STAGE && SCH != SCH_DP);
     else derived_ifft<Real, N, TC>(pre0, sm, a.f0, a.f1, a.f2, a.f3, ldc, ky, valid, t, c, seed);
     return true;
 }
