@@ -31,6 +31,7 @@
 #include "adjoint.cuh"
 #include "engine.cuh"
 #include "handle.h"
+#include "host_common.h"
 
 using namespace ns2d;
 using ns2d::internal::fail;
@@ -88,7 +89,7 @@ const double kA[3] = {0.5, 0.5, 1.0};
 template <typename Real, int N>
 struct AdjLaunch {
     using S = Shape<Real, N>;
-    static constexpr size_t col_smem() { return ColSmem<Real, N, S::TC>::bytes(); }
+    static constexpr size_t col_smem() { return AdjColSmem<Real, N, S::TC>::bytes(); }
     static constexpr size_t row_smem() { return RowSmem<Real, N, 2 * S::PAIRS>::bytes(); }
     static cudaError_t setup() {
         cudaError_t e = cudaSuccess;
@@ -102,7 +103,7 @@ struct AdjLaunch {
         return e;
     }
     static void col(int mode, const AdjColArgs<Real>& a, cudaStream_t s) {
-        dim3 grid((a.nyf + S::TC - 1) / S::TC), block(S::T * S::TC);
+        dim3 grid((a.nyf + S::TC - 1) / S::TC), block(S::T * S::TC * adj_groups<N>());
         switch (mode) {
             case ADJ_START: adj_col_kernel<Real, N, S::TC, ADJ_START><<<grid, block, col_smem(), s>>>(a); break;
             case ADJ_MID: adj_col_kernel<Real, N, S::TC, ADJ_MID><<<grid, block, col_smem(), s>>>(a); break;
@@ -234,6 +235,7 @@ AdjColArgs<Real> col_common(ns2d_handle* h) {
     a.norm2 = (Real)std::pow(1.0 / (double)(h->nx * h->ny), 2.0);
     const int m = (int)(h->nx / 3.0);
     a.kmax_sqr = m * m + h->p.dealias_edge;
+    a.kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
     a.dealias = h->p.dealias;
     a.houli_int = (h->p.quirks & NS2D_QUIRK_HOU_LI_INT) ? 1 : 0;
     a.kolm = (h->p.forcing == NS2D_FORCING_KOLM) ? 1 : 0;
@@ -263,6 +265,7 @@ void adjoint_step(ns2d_handle* h, const void* cap, const void* lam_p, void* lam_
     r.P3 = (C*)st->P[3];
     r.tw = (const C*)h->tw;
     r.ldc = h->ldc;
+    r.kc = a.kc;
     const size_t plane = plane_elems(h);
     const C* capc = (const C*)cap;
     cudaStream_t s = st->stream;

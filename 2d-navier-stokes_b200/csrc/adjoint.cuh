@@ -13,12 +13,15 @@
 // the forward stage, captured while the forward step is recomputed.
 //
 // Passes per adjoint stage (mirroring the forward step):
-//   adj row pass  (y): mu = c2r(mu_x); products wx mu, wy mu, u mu, v mu; two
-//                      packed r2c -> four x-space half spectra P0..P3.
-//   adj col pass  (x): four forward x-FFTs of P0..P3, L = sum conj(m) P (the
+//   adj row pass  (y): mu = c2r(mu_x); products wx mu, wy mu, u mu, v mu, packed as
+//                      Q = (wx + i wy) mu and R = (u + i v) mu; two forward y-FFTs;
+//                      Q(ky) and conj Q(-ky) at ky >= 0 are P0 +- i P1 of the real
+//                      products' half spectra (R: P2 +- i P3) and go out as they are.
+//   adj col pass  (x): four forward x-FFTs of those, L = sum conj(m) P (the
 //                      adjoint of this stage's input); lambda_x += L; the
 //                      previous stage's kappa = b B lambda' + a dt L; then
-//                      s^2 D kappa -> inverse x-FFT -> mu_x for the next row pass.
+//                      s^2 D kappa -> inverse x-FFT -> mu_x for the next row pass
+//                      (columns that D empties are neither formed nor read).
 #pragma once
 #include "kernels.cuh"
 
@@ -29,8 +32,8 @@ enum AdjMode : int { ADJ_START = 0, ADJ_MID = 1, ADJ_END = 2 };
 template <typename Real>
 struct AdjColArgs {
     using C = typename Cx<Real>::T;
-    const C* P0;          // x-space product spectra of the row pass (MID, END)
-    const C* P1;
+    const C* P0;          // x-space spectra of the row pass (MID, END): Q(ky), conj Q(-ky),
+    const C* P1;          // R(ky), conj R(-ky)
     const C* P2;
     const C* P3;
     C* lam_x;             // adjoint of the step input (accumulated), [kx][ldc]
@@ -41,6 +44,7 @@ struct AdjColArgs {
     int ldc, nyf;
     Real norm2;
     int kmax_sqr, dealias, houli_int, kolm;
+    int kc;               // columns ky >= kc are emptied by D
     double b_next;        // weight of lambda' in the next kappa: b_{s-1} (MID) or b_4 (START)
     double adt;           // a_{s-1} dt (MID)
 };
@@ -57,99 +61,138 @@ __device__ __forceinline__ Real dealias_factor(int kx, int ky, int N, int kmax_s
     return houli_filter<Real>(kx, ky, N, N, houli_int);
 }
 
-// conj(m_f) * P for the four multipliers (f = 0..3: m_u, m_v, m_x, m_y).
-template <typename C>
-__device__ __forceinline__ C conj_mult(int f, int kx, int ky, C P) {
-    using Real = decltype(C::x);
-    if (kx == 0 && ky == 0) return cmake<C>(0, 0);
-    Real s;
-    if (f < 2) {
-        const double inv = 1.0 / (double)(kx * kx + ky * ky);
-        s = (Real)((double)(f == 0 ? ky : kx) * inv);
-    } else {
-        s = (Real)(f == 2 ? kx : ky);
+// Exchange buffer of one group's transforms, synchronised with the group's own
+// named barrier.
+template <int N, int TC, typename C>
+struct IlvGroupPolicy {
+    C* sm;
+    int c, bar;
+    static constexpr int STRIDE = SmemLayout<N, TC>::ELEMS;
+    __device__ __forceinline__ C& at(int b, int e) const { return sm[b * STRIDE + SmemLayout<N, TC>::slot(e, c)]; }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "n"(Plan<N>::T * TC) : "memory");
     }
-    // conj(i s) = -i s;  conj(-i s) = i s  (f == 1 has m_v = -i kx/k^2)
-    return (f == 1) ? cmake<C>(-s * P.y, s * P.x) : cmake<C>(s * P.y, -s * P.x);
-}
+};
+
+// Thread groups of the adjoint column pass: two, each transforming one of the two
+// pairs of spectra, where a thread holds few enough elements for it (at 512^2
+// FP64 17 us with one group); one group takes the pairs in turn otherwise.
+template <int N>
+constexpr int adj_groups() { return N / Plan<N>::T <= 8 ? 2 : 1; }
+
+template <typename Real, int N, int TC>
+struct AdjColSmem {
+    using C = typename Cx<Real>::T;
+    static constexpr int G = adj_groups<N>();
+    static constexpr int FFT = SmemLayout<N, TC>::ELEMS;
+    static constexpr size_t bytes() { return sizeof(C) * (size_t)(2 * G * FFT + G * N * TC); }
+};
 
 template <typename Real, int N, int TC, int MODE>
-__global__ void __launch_bounds__(Plan<N>::T * TC) adj_col_kernel(AdjColArgs<Real> a) {
+__global__ void __launch_bounds__(Plan<N>::T * TC * adj_groups<N>()) adj_col_kernel(AdjColArgs<Real> a) {
     using C = typename Cx<Real>::T;
     using P = Plan<N>;
-    using SM = ColSmem<Real, N, TC>;
+    using SM = AdjColSmem<Real, N, TC>;
     constexpr int T = P::T;
     constexpr int E = N / T;
+    constexpr int G = SM::G;
+    constexpr int EG = E / G;  // elements of the epilogue per thread
     extern __shared__ __align__(16) unsigned char smraw[];
     C* sm = reinterpret_cast<C*>(smraw);
-    C* Lbuf = sm + 2 * SM::FFT;  // [N][TC]: L, then s^2 D kappa
+    C* Lbuf = sm + 2 * G * SM::FFT;  // [G][N][TC]: the groups' parts of L, then s^2 D kappa in the first
+    const int g = threadIdx.x / (T * TC);
     const int c = threadIdx.x % TC;
-    const int t = threadIdx.x / TC;
+    const int t = (threadIdx.x % (T * TC)) / TC;
     const int ky = blockIdx.x * TC + c;
     const bool valid = ky < a.nyf;
     const int kyc = valid ? ky : 0;
     const int ldc = a.ldc;
     const auto seed = twiddle_seeds<N>(a.tw, t);
+    const IlvGroupPolicy<N, TC, C> pol{sm + 2 * g * SM::FFT, c, 1 + g};
+    const Real tr = (Real)t, kyr = (Real)ky;
 
+    // operands of the epilogue, on their way under the transforms
+    C lx[EG], lp[MODE == ADJ_END ? 1 : EG];
+    double2 f[MODE == ADJ_END ? 1 : EG];
+#pragma unroll
+    for (int m = 0; m < EG; ++m) {
+        const size_t q = (size_t)(t + T * (m + g * EG)) * ldc + kyc;
+        if constexpr (MODE != ADJ_START) lx[m] = a.lam_x[q];
+        if constexpr (MODE != ADJ_END) {
+            lp[m] = a.lam_p[q];
+            f[m] = a.cn[q];
+        }
+    }
     if constexpr (MODE != ADJ_START) {
-        // L = conj(m_u) P0 + conj(m_v) P1 + conj(m_x) P2 + conj(m_y) P3
-        const C* Ps[4] = {a.P0, a.P1, a.P2, a.P3};
+        const C* const Ps[4] = {a.P0, a.P1, a.P2, a.P3};
 #pragma unroll 1
-        for (int fp = 0; fp < 4; fp += 2) {
+        for (int pair = g; pair < 2; pair += G) {
             C v[2][E];
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const size_t q = (size_t)(t + T * m) * ldc + kyc;
-                v[0][m] = valid ? Ps[fp][q] : cmake<C>(0, 0);
-                v[1][m] = valid ? Ps[fp + 1][q] : cmake<C>(0, 0);
+                v[0][m] = Ps[2 * pair][q];
+                v[1][m] = Ps[2 * pair + 1][q];
             }
-            fft_batched<N, -1, 2>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
+            fft_batched<N, -1, 2>(v, pol, seed, t);
+            // With q = kx + i ky the four terms conj(m) P are
+            //   pair 0: (conj(q) Q+ - q Q-) / (2 k^2),  pair 1: -i (conj(q) R+ + q R-) / 2
 #pragma unroll
             for (int m = 0; m < E; ++m) {
-                const int i = t + T * m;
-                const int kx = (i <= N / 2) ? i : i - N;
-                C L = cadd(conj_mult(fp, kx, ky, v[0][m]), conj_mult(fp + 1, kx, ky, v[1][m]));
-                if (fp > 0) L = cadd(Lbuf[i * TC + c], L);
-                Lbuf[i * TC + c] = L;
+                const Real kx = kx_of<Real, N, T>(m, t, tr);
+                const C p = v[0][m], n = v[1][m];
+                const C cp = cmake<C>(kx * p.x + kyr * p.y, kx * p.y - kyr * p.x);
+                const C qn = cmake<C>(kx * n.x - kyr * n.y, kx * n.y + kyr * n.x);
+                C L;
+                if (m == 0 && t == 0 && ky == 0) {
+                    L = cmake<C>(0, 0);
+                } else if (pair == 0) {
+                    const Real s = (Real)0.5 * inv_k2<Real>(kx * kx + kyr * kyr);
+                    L = cscale(csub(cp, qn), s);
+                } else {
+                    const C sum = cadd(cp, qn);
+                    L = cmake<C>((Real)0.5 * sum.y, (Real)-0.5 * sum.x);
+                }
+                C* const to = Lbuf + (G > 1 ? g * N * TC : 0) + (t + T * m) * TC + c;
+                if (G == 1 && pair > 0) L = cadd(*to, L);
+                *to = L;
             }
         }
+        if constexpr (G > 1) __syncthreads();
     }
-    if constexpr (MODE == ADJ_END) {
-#pragma unroll 4
-        for (int m = 0; m < E; ++m) {
-            const int i = t + T * m;
-            if (valid) {
-                const size_t q = (size_t)i * ldc + ky;
-                a.lam_x[q] = cadd(a.lam_x[q], Lbuf[i * TC + c]);
-            }
+#pragma unroll
+    for (int m = 0; m < EG; ++m) {
+        const int i = t + T * (m + g * EG);
+        const size_t q = (size_t)i * ldc + ky;
+        C L = cmake<C>(0, 0);
+        if constexpr (MODE != ADJ_START) {
+            L = Lbuf[i * TC + c];
+            if constexpr (G > 1) L = cadd(L, Lbuf[N * TC + i * TC + c]);
         }
-        return;
-    } else {
-        // kappa of the next (earlier) stage and the source of mu
-#pragma unroll 4
-        for (int m = 0; m < E; ++m) {
-            const int i = t + T * m;
-            const int kx = (i <= N / 2) ? i : i - N;
-            const size_t q = (size_t)i * ldc + kyc;
-            const C lp = valid ? a.lam_p[q] : cmake<C>(0, 0);
-            const double2 f = valid ? a.cn[q] : make_double2(0.0, 0.0);
-            C kappa = cscale(lp, (Real)(a.b_next * f.y));
+        if constexpr (MODE == ADJ_END) {
+            if (valid) a.lam_x[q] = cadd(lx[m], L);
+        } else {
+            // lambda_x, then kappa of the next (earlier) stage and the source of mu
+            C kappa = cscale(lp[m], (Real)(a.b_next * f[m].y));
             if constexpr (MODE == ADJ_MID) {
-                const C L = Lbuf[i * TC + c];
-                if (valid) a.lam_x[(size_t)i * ldc + ky] = cadd(a.lam_x[(size_t)i * ldc + ky], L);
+                if (valid) a.lam_x[q] = cadd(lx[m], L);
                 kappa = cadd(kappa, cscale(L, (Real)a.adt));
             } else {
-                // START: lambda_x = A lambda'
-                if (valid) a.lam_x[(size_t)i * ldc + ky] = cscale(lp, (Real)f.x);
+                if (valid) a.lam_x[q] = cscale(lp[m], (Real)f[m].x);  // lambda_x = A lambda'
             }
+            const int kx = (i <= N / 2) ? i : i - N;
             const Real d = dealias_factor<Real>(kx, ky, N, a.kmax_sqr, a.dealias, a.houli_int, a.kolm);
             Lbuf[i * TC + c] = cscale(kappa, a.norm2 * d);
         }
+    }
+    if constexpr (MODE != ADJ_END) {
+        if (blockIdx.x * TC >= a.kc) return;  // mu is zero here, and not read
         __syncthreads();
+        if (g > 0) return;
         C v[1][E];
 #pragma unroll
         for (int m = 0; m < E; ++m) v[0][m] = Lbuf[(t + T * m) * TC + c];
-        fft_batched<N, +1, 1>(v, IlvPolicy<N, TC, C>{sm, c}, seed, t);
+        fft_batched<N, +1, 1>(v, pol, seed, t);
         if (valid) {
 #pragma unroll
             for (int m = 0; m < E; ++m) a.mu[(size_t)(t + T * m) * ldc + ky] = v[0][m];
@@ -163,12 +206,13 @@ struct AdjRowArgs {
     const C* mu;          // x-space mu_x [x][ldc]
     const C* cap_uv;      // captured real fields of the forward stage: (u, v) and
     const C* cap_w;       // (w_x, w_y) as complex pairs, [x][y]
-    C* P0;                // outputs: x-space half spectra of w_x mu, w_y mu, u mu, v mu
+    C* P0;                // outputs at ky >= 0: Q(ky), conj Q(-ky), R(ky), conj R(-ky)
     C* P1;
     C* P2;
     C* P3;
     const C* tw;
     int ldc;
+    int kc;               // mu_x is zero (and not stored) from ky = kc on
 };
 
 // Adjoint row pass: one team of T threads per row x, TC = 2 PAIRS rows per block.
@@ -179,7 +223,6 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) adj_row_kernel(AdjRowA
     constexpr int T = P::T;
     constexpr int E = N / T;
     constexpr int TC = 2 * PAIRS;
-    using TL = TeamLayout<N>;
     using RS = RowSmem<Real, N, TC>;
     extern __shared__ __align__(16) unsigned char smraw[];
     const int g = threadIdx.x / T;
@@ -196,7 +239,7 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) adj_row_kernel(AdjRowA
         for (int m = 0; m < E; ++m) {
             const int y = t + T * m;
             const int yy = (y <= N / 2) ? y : N - y;
-            const C p = M[yy];
+            const C p = yy < a.kc ? M[yy] : cmake<C>(0, 0);
             if (y == 0 || y == N / 2) z[0][m] = cmake<C>(p.x, 0);
             else if (y < N / 2) z[0][m] = p;
             else z[0][m] = cconj(p);
@@ -218,26 +261,16 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) adj_row_kernel(AdjRowA
         }
     }
     fft_batched<N, -1, 2>(q, pol, seed, t);
-#pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int m = 0; m < E; ++m) region[b * TL::ROWS + TL::slot(t + T * m)] = q[b][m];
-    pol.sync();
-    // split each packed transform: X_a = (Z_k + conj Z_{N-k})/2, X_b = (Z_k - conj Z_{N-k})/(2i)
     C* outs[4] = {a.P0, a.P1, a.P2, a.P3};
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-        C* __restrict__ oa = outs[2 * b] + (size_t)x * a.ldc;
-        C* __restrict__ ob = outs[2 * b + 1] + (size_t)x * a.ldc;
+        C* __restrict__ op = outs[2 * b] + (size_t)x * a.ldc;
+        C* __restrict__ on = outs[2 * b + 1] + (size_t)x * a.ldc;
 #pragma unroll
         for (int m = 0; m < E; ++m) {
             const int k = t + T * m;
-            if (k <= N / 2) {
-                const C zk = region[b * TL::ROWS + TL::slot(k)];
-                const C zm = region[b * TL::ROWS + TL::slot((N - k) & (N - 1))];
-                oa[k] = cmake<C>((Real)0.5 * (zk.x + zm.x), (Real)0.5 * (zk.y - zm.y));
-                ob[k] = cmake<C>((Real)0.5 * (zk.y + zm.y), (Real)0.5 * (zm.x - zk.x));
-            }
+            if (k <= N / 2) op[k] = q[b][m];
+            if (k == 0 || k >= N / 2) on[k == 0 ? 0 : N - k] = cconj(q[b][m]);
         }
     }
 }
