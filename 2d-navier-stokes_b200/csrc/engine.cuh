@@ -43,6 +43,26 @@ struct Launch {
         set((const void*)col_kernel<Real, N, S::TC, MODE, SCH>, col_smem());
         set((const void*)col_tma_kernel<Real, N, S::TC, MODE, SCH>, col_tma_smem());
     }
+    // A pass's launch; programmatic dependent launch where the passes use it and are
+    // queued one by one (256^2: a step of changing dt 81 -> 71 us, a Dormand-Prince
+    // step 155 -> 134).  Not into a graph, whose own edges are faster (512^2 FP64 57
+    // us a step, 73 with programmatic ones).
+    template <typename... P, typename... A>
+    static void launch(void (*f)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (pass_pdl(N) && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+            cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, f, args...);  // a failure is left for cudaGetLastError
+    }
     static cudaError_t setup() {
         cudaError_t e = cudaSuccess;
         auto set = [&](const void* f, size_t bytes) {
@@ -75,13 +95,13 @@ struct Launch {
         if (maps && col_tma_ok(a)) {
             if constexpr (SCH == SCH_CNX && (MODE == COL_STAGE || MODE == COL_FINAL)) {
                 if (a.dealias == 0 && !a.rhs_store) {
-                    col_tma_kernel<Real, N, S::TC, MODE, SCH_CN><<<grid, block, col_tma_smem(), s>>>(a, *maps);
+                    launch(col_tma_kernel<Real, N, S::TC, MODE, SCH_CN>, grid, block, col_tma_smem(), s, a, *maps);
                     return;
                 }
             }
-            col_tma_kernel<Real, N, S::TC, MODE, SCH><<<grid, block, col_tma_smem(), s>>>(a, *maps);
+            launch(col_tma_kernel<Real, N, S::TC, MODE, SCH>, grid, block, col_tma_smem(), s, a, *maps);
         } else {
-            col_kernel<Real, N, S::TC, MODE, SCH><<<grid, block, col_smem(), s>>>(a);
+            launch(col_kernel<Real, N, S::TC, MODE, SCH>, grid, block, col_smem(), s, a);
         }
     }
     // scheme: SCH_CN, SCH_EX, SCH_AB4 or SCH_DP (stage and final passes); maps: tensor maps
@@ -104,7 +124,7 @@ struct Launch {
     }
     static void row(const RowArgs<Real>& a, cudaStream_t s) {
         dim3 grid(N / (2 * S::PAIRS)), block(S::T * 2 * S::PAIRS);
-        row_kernel<Real, N, S::PAIRS><<<grid, block, row_smem(), s>>>(a);
+        launch(row_kernel<Real, N, S::PAIRS>, grid, block, row_smem(), s, a);
     }
     static void col_inv(const InvArgs<Real>& a, cudaStream_t s) {
         dim3 grid((a.nyf + S::TC - 1) / S::TC), block(S::T * S::TC);

@@ -140,6 +140,13 @@ struct ColArgs {
 // 1024^2, where the tiles fill one wave either way, 149 / 97 -> 144 / 94 us.
 __device__ __forceinline__ bool band_narrow(const int* band) { return band && (band[0] | band[1] | band[2]) == 0; }
 
+// Programmatic dependent launch: pdl_launch lets the next kernel's blocks start
+// when every block of this one has called it; pdl_wait holds a block until the
+// kernels before it have completed and their writes are visible.  Whatever a pass
+// reads that another kernel writes comes after its pdl_wait.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // Start of a pass block: early exit once the device status word is set (a failed
 // SystemCheck), and band_narrow of the evaluation.  One thread reads the words
 // (independent loads) and the block agrees on them through shared memory, so
@@ -536,7 +543,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 // stay zero there.
 // begin(): the block's flags (BlockBegin) and a block barrier; called once the
 // TMA tile loads are under way, so the flags' latency runs under theirs.
-template <typename Real, int N, int TC, int MODE, int SCH, bool GEN = false, bool TMA = false, bool SPLIT = false, typename Begin>
+template <typename Real, int N, int TC, int MODE, int SCH, bool GEN = false, bool TMA = false, bool SPLIT = false, bool PDL = false, typename Begin>
 __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& begin, int tile, unsigned char* smraw,
                                          const ColMaps* maps = nullptr) {
     using C = typename Cx<Real>::T;
@@ -591,6 +598,10 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         }
         return true;
     };
+    if constexpr (PDL) {
+        pdl_launch();
+        pdl_wait();
+    }
     if (!dead) issue();
     const BlockBegin b = begin();
     const bool narrow = b.narrow;
@@ -966,11 +977,15 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
     return true;
 }
 
+// Grid sizes whose single-field passes use programmatic dependent launch: those
+// whose blocks leave room on the SMs for the next pass's.
+constexpr bool pass_pdl(int n) { return n <= 512; }
+
 // Column pass of one field.  Grid: ceil(nyf / TC) blocks; block: T * TC threads.
 template <typename Real, int N, int TC, int MODE, int SCH>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_kernel(ColArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    col_body<Real, N, TC, MODE, SCH, true>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, smraw);
+    col_body<Real, N, TC, MODE, SCH, true, false, false, pass_pdl(N)>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, smraw);
 }
 
 // Column pass with TMA tile loads and stores, without the rarely used parts (see
@@ -980,7 +995,7 @@ template <typename Real, int N, int TC, int MODE, int SCH>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_tma_kernel(ColArgs<Real> a, const __grid_constant__ ColMaps maps) {
     extern __shared__ __align__(16) unsigned char smraw[];
     unsigned char* sm = smraw + ((1024u - ((unsigned)__cvta_generic_to_shared(smraw) & 1023u)) & 1023u);
-    col_body<Real, N, TC, MODE, SCH, false, true, true>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, sm, &maps);
+    col_body<Real, N, TC, MODE, SCH, false, true, true, pass_pdl(N)>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, sm, &maps);
 }
 
 // Whether a column pass can run without its GEN parts.
@@ -1182,6 +1197,10 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
 template <typename Real, int N, int PAIRS, bool CAP = true>
 __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) row_kernel(RowArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smraw[];
+    if constexpr (pass_pdl(N)) {
+        pdl_launch();
+        pdl_wait();
+    }
     const BlockBegin b = block_begin(a.status, a.band);
     if (b.exit) return;
     row_body<Real, N, PAIRS, CAP>(a, b.narrow, blockIdx.x, smraw);
