@@ -438,6 +438,7 @@ ns2d_status backward_impl(ns2d_handle* h) {
     if (par != 0) ACK(h, cudaMemcpyAsync(a->lam[0], a->lam[1], h->field_bytes, cudaMemcpyDeviceToDevice, h->stream));
     ACK(h, cudaMemcpyAsync(h->state, a->w_final, h->field_bytes, cudaMemcpyDeviceToDevice, h->stream));
     ACK(h, cudaEventRecord(a->t[3], h->stream));
+    h->status_seen = false;  // the recomputed segments' graphs
     ns2d_status s2 = internal::check_status(h);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, a->t[2], a->t[3]);

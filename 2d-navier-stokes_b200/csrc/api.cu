@@ -113,6 +113,15 @@ RowArgs<Real> row_args(ns2d_handle* h) {
     return r;
 }
 
+// `bytes` of device memory into the handle's page-locked buffer, once the queued
+// work is done.  (A copy into pageable memory goes through a staging buffer of the
+// driver's and costs about as much again as the wait.)
+ns2d_status fetch(ns2d_handle* h, const void* dev, size_t bytes) {
+    CK(h, cudaMemcpyAsync(h->pin, dev, bytes, cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaStreamSynchronize(h->stream));
+    return NS2D_OK;
+}
+
 cudaEvent_t take_event(ns2d_handle* h) {
     if (!h->ev_pool.empty()) {
         cudaEvent_t e = h->ev_pool.back();
@@ -196,6 +205,7 @@ const ColMaps* col_maps_for(const ns2d_handle* h, int mode, const ColArgs<Real>&
 template <typename Real>
 void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a, int scheme = SCH_CN) {
     TimedLaunch t(h, mode == COL_STAGE ? 1 : mode == COL_FINAL ? 2 : 0);
+    h->status_seen = false;
     const ColMaps* maps = col_maps_for<Real>(h, mode, a);
     engine_ops<Real>(h->nx)->col(mode, scheme, a, h->stream, maps);
 }
@@ -251,6 +261,7 @@ void fill_resident(ns2d_handle* h, ResArgs<Real>& r, int branch) {
 
 template <typename Real>
 ns2d_status launch_resident(ns2d_handle* h, int scheme, const ResArgs<Real>& r) {
+    h->status_seen = false;
     CK(h, resident_launch<Real>(h->nx, scheme, r, h->stream));
     h->launches += r.nsteps;  // counted per step (ns2d_launch_count)
     return NS2D_OK;
@@ -608,9 +619,8 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
                                                      dt, 1e-7, 1e-7, h->nx, h->nyf, h->ldc, h->dpart);
     h->launches++;
     CKL(h);
-    double part[296];
-    CK(h, cudaMemcpyAsync(part, h->dpart, sizeof(part), cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (ns2d_status sf = fetch(h, h->dpart, sizeof(double) * 296)) return sf;
+    const double* part = (const double*)h->pin;
     double sum = 0.0;
     for (int b = 0; b < 296; ++b) sum += part[b];
     *err = std::sqrt(sum / (double)(h->nx * h->nyf));
@@ -696,9 +706,8 @@ ns2d_status rk5dp_step_impl(ns2d_handle* h, double dt, int iters, double* err) {
     h->launches++;
     CKL(h);
     if (iters > 1) {
-        double part[296];
-        CK(h, cudaMemcpyAsync(part, h->dpart, sizeof(part), cudaMemcpyDeviceToHost, h->stream));
-        CK(h, cudaStreamSynchronize(h->stream));
+        if (ns2d_status sf = fetch(h, h->dpart, sizeof(double) * 296)) return sf;
+        const double* part = (const double*)h->pin;
         double sum = 0.0;
         for (int b = 0; b < 296; ++b) sum += part[b];
         h->dp_err = std::sqrt(1.0 / (double)((long)h->nx * (long)h->nyf) * sum);
@@ -742,12 +751,8 @@ ns2d_status c2r_impl(ns2d_handle* h, const InvField<Real>* fields, int nf, int o
     h->launches++;
     CKL(h);
     if (result) {
-        unsigned long long bits = 0;
-        CK(h, cudaMemcpyAsync(&bits, h->dmax, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
-        CK(h, cudaStreamSynchronize(h->stream));
-        double v;
-        std::memcpy(&v, &bits, sizeof(v));
-        *result = v;
+        if (ns2d_status sf = fetch(h, h->dmax, sizeof(double))) return sf;
+        std::memcpy(result, h->pin, sizeof(double));
     }
     return NS2D_OK;
 }
@@ -819,7 +824,7 @@ void fill_twiddles(std::vector<Cplx<Real>>& tw, int n) {
 
 void free_all(ns2d_handle* h) {
     void* ptrs[] = {h->state, h->acc, h->nl, h->f[0], h->f[1], h->f[2], h->f[3], h->tmpfull, h->col0[0], h->col0[1],
-                    h->tw, h->rhsbuf, h->ab[0], h->ab[1], h->ab[2], h->ab[3], h->uhat_ref, h->dreal, h->dscal, h->dmax,
+                    h->tw, h->rhsbuf, h->ab[0], h->ab[1], h->ab[2], h->ab[3], h->uhat_ref, h->dreal, h->dmax,
                     h->dstatus, h->dband, h->dio, h->ddiag, h->dpart, h->cn, h->dp_last, h->lint, h->filt};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -829,6 +834,7 @@ void free_all(ns2d_handle* h) {
     for (void* p : fp)
         if (p) cudaFree(p);
     if (h->dp_kptr) cudaFree((void*)h->dp_kptr);
+    if (h->pin) cudaFreeHost(h->pin);
     delete static_cast<ColMaps*>(h->col_maps);
     h->col_maps = nullptr;
 }
@@ -851,8 +857,6 @@ ns2d_status create_impl(ns2d_handle* h) {
     CK(h, cudaMalloc(&h->uhat_ref, uref));
     CK(h, cudaMemsetAsync(h->uhat_ref, 0, uref, h->stream));
     CK(h, cudaMalloc(&h->dreal, sizeof(double) * (size_t)h->nx * h->ny));
-    CK(h, cudaMalloc(&h->dscal, sizeof(double) * 4));
-    CK(h, cudaMemsetAsync(h->dscal, 0, sizeof(double) * 4, h->stream));
     CK(h, cudaMalloc(&h->dmax, sizeof(unsigned long long) * 2));
     CK(h, cudaMalloc(&h->dstatus, sizeof(int) * 4));
     CK(h, cudaMemsetAsync(h->dstatus, 0, sizeof(int) * 4, h->stream));
@@ -865,6 +869,7 @@ ns2d_status create_impl(ns2d_handle* h) {
         CKL(h);
     }
     CK(h, cudaMalloc(&h->dio, sizeof(double2) * (size_t)h->nx * h->nyf));
+    CK(h, cudaMallocHost(&h->pin, sizeof(double) * std::max<size_t>(4096, DG_N + 8 * (size_t)h->n_spect)));
     CK(h, cudaMalloc(&h->ddiag, sizeof(double) * (DG_N + 8 * (size_t)h->n_spect)));
     CK(h, cudaMalloc(&h->dpart, sizeof(double) * 4096));
     CK(h, cudaMalloc(&h->cn, sizeof(double2) * (size_t)h->nx * h->ldc));
@@ -970,6 +975,7 @@ ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
         *gbr = branch;
         return NS2D_OK;
     }
+    h->status_seen = false;
     cudaError_t e = cudaGraphLaunch(*gx, h->stream);
     if (e != cudaSuccess) return fail(h, NS2D_ERR_CUDA, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e));
     h->launches += h->graph_kernels;
@@ -1036,7 +1042,7 @@ ns2d_status host_to_state(ns2d_handle* h, const double* host, void* dst) {
     CK(h, cudaMemcpyAsync(h->dio, host, sizeof(double2) * (size_t)h->nx * h->nyf, cudaMemcpyHostToDevice, h->stream));
     return DISPATCH(h, pack_in, h, h->dio, dst);
 }
-ns2d_status state_to_host(ns2d_handle* h, const void* src, double* host) {
+ns2d_status state_to_host(ns2d_handle* h, const void* src, double* host, bool wait = true) {
     if (!h->fp32) {
         CK(h, cudaMemcpy2DAsync(host, sizeof(double2) * (size_t)h->nyf, src, sizeof(double2) * (size_t)h->ldc,
                                 sizeof(double2) * (size_t)h->nyf, (size_t)h->nx, cudaMemcpyDeviceToHost, h->stream));
@@ -1045,7 +1051,7 @@ ns2d_status state_to_host(ns2d_handle* h, const void* src, double* host) {
         if (s) return s;
         CK(h, cudaMemcpyAsync(host, h->dio, sizeof(double2) * (size_t)h->nx * h->nyf, cudaMemcpyDeviceToHost, h->stream));
     }
-    CK(h, cudaStreamSynchronize(h->stream));
+    if (wait) CK(h, cudaStreamSynchronize(h->stream));
     return NS2D_OK;
 }
 
@@ -1084,26 +1090,28 @@ ns2d_status mean_flow_impl(ns2d_handle* h, double* mean_x, double* mean_y) {
                                                                 h->dpart);
     h->launches++;
     CKL(h);
-    std::vector<double> buf((size_t)h->nx + h->nyf);
-    CK(h, cudaMemcpyAsync(buf.data(), h->dpart, sizeof(double) * buf.size(), cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
-    if (mean_y) std::memcpy(mean_y, buf.data(), sizeof(double) * h->nx);
-    if (mean_x) std::memcpy(mean_x, buf.data() + h->nx, sizeof(double) * h->nyf);
+    if (ns2d_status sf = fetch(h, h->dpart, sizeof(double) * ((size_t)h->nx + h->nyf))) return sf;
+    const double* buf = (const double*)h->pin;
+    if (mean_y) std::memcpy(mean_y, buf, sizeof(double) * h->nx);
+    if (mean_x) std::memcpy(mean_x, buf + h->nx, sizeof(double) * h->nyf);
     return NS2D_OK;
 }
 
 ns2d_status read_status(ns2d_handle* h, int* bits, int* steps) {
-    int st[2];
-    CK(h, cudaMemcpyAsync(st, h->dstatus, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
-    *bits = st[0];
-    if (steps) *steps = st[1];
+    if (!h->status_seen) {
+        if (ns2d_status sf = fetch(h, h->dstatus, sizeof(int) * 2)) return sf;
+        std::memcpy(h->seen, h->pin, sizeof(int) * 2);
+        h->status_seen = true;
+    }
+    *bits = h->seen[0];
+    if (steps) *steps = h->seen[1];
     return NS2D_OK;
 }
 
 ns2d_status clear_status(ns2d_handle* h) {
     CK(h, cudaMemsetAsync(h->dstatus, 0, sizeof(int) * 2, h->stream));
-    CK(h, cudaMemsetAsync(h->dscal, 0, sizeof(double) * 2, h->stream));
+    h->seen[0] = h->seen[1] = 0;
+    h->status_seen = true;
     return NS2D_OK;
 }
 
@@ -1166,9 +1174,8 @@ ns2d_status measurables_impl(ns2d_handle* h, ns2d_measures* out, double* spectra
     diag_kernel<Real><<<148, kDiagThreads, diag_smem(ns), h->stream>>>(d);
     h->launches++;
     CKL(h);
-    std::vector<double> raw(nout);
-    CK(h, cudaMemcpyAsync(raw.data(), h->ddiag, sizeof(double) * nout, cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
+    if ((s = fetch(h, h->ddiag, sizeof(double) * nout))) return s;
+    const double* raw = (const double*)h->pin;
     const double norm_fac = 0.5 / std::pow((double)(h->nx * h->ny), 2.0);
     const double const_fac = 4.0 * std::pow(M_PI, 2.0);
     const double cn = const_fac * norm_fac;
@@ -1604,8 +1611,8 @@ ns2d_status ns2d_rk4_step_host(ns2d_handle* h, double* w_hat, double dt) {
     ns2d_status s = host_to_state(h, w_hat, h->state);
     if (s) return s;
     if ((s = single_step(h, dt))) return s;
-    if ((s = state_to_host(h, h->state, w_hat))) return s;
-    return check_status(h);
+    if ((s = state_to_host(h, h->state, w_hat, false))) return s;
+    return check_status(h);  // waits for the state too
 }
 
 ns2d_status ns2d_step_async(ns2d_handle* h, int32_t nsteps, double dt) {
@@ -1684,6 +1691,7 @@ ns2d_status ns2d_rk5dp_step(ns2d_handle* h, double dt, int32_t iters, double* er
 ns2d_status ns2d_check(ns2d_handle* h) {
     if (!h) return NS2D_ERR_INVALID;
     cudaSetDevice(h->p.device);
+    h->status_seen = false;  // it waits for all queued work
     return check_status(h);
 }
 

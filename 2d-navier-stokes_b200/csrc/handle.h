@@ -36,9 +36,11 @@ struct ns2d_handle {
     void* ab[4] = {nullptr, nullptr, nullptr, nullptr};  // AB4 ring: [0..2] history, [3] next
     void* uhat_ref = nullptr;  // persistent u_hat in the reference layout (CFL / VEL paths)
     double* dreal = nullptr;   // [nx][ny] real-space output
-    double* dscal = nullptr;   // [0] bound accumulator, [1] ticket
     unsigned long long* dmax = nullptr;
     int* dstatus = nullptr;    // [0] bits, [1] completed steps
+    int seen[2] = {0, 0};      // their values when last read (or cleared) ...
+    bool status_seen = false;  // ... and whether nothing queued since can have changed them
+    void* pin = nullptr;       // page-locked results of the calls that wait (fetch)
     int* dband = nullptr;      // band_narrow words: [0] the state, [1] the update factors, [2] the explicit linear ones
     bool band_known = false;   // dband[0] describes the state
     bool ffield_band = false;  // the listed forcing has modes in the columns dealiasing empties
