@@ -198,14 +198,15 @@ const ColMaps* col_maps_for(const ns2d_handle* h, int mode, const ColArgs<Real>&
                    ? static_cast<const ColMaps*>(h->col_maps)
                    : nullptr;
     if (a.src != h->nl || a.state != h->state || a.acc != h->acc) return nullptr;
-    if (mode == COL_STAGE && (a.f0 != h->f[0] || a.f1 != h->f[1] || a.f2 != h->f[2] || a.f3 != h->f[3])) return nullptr;
+    if ((mode == COL_STAGE || mode == COL_NEXT) && (a.f0 != h->f[0] || a.f1 != h->f[1] || a.f2 != h->f[2] || a.f3 != h->f[3])) return nullptr;
     return static_cast<const ColMaps*>(h->col_maps);
 }
 
 template <typename Real>
 void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a, int scheme = SCH_CN) {
-    TimedLaunch t(h, mode == COL_STAGE ? 1 : mode == COL_FINAL ? 2 : 0);
+    TimedLaunch t(h, mode == COL_STAGE ? 1 : mode == COL_FINAL || mode == COL_NEXT ? 2 : 0);
     h->status_seen = false;
+    if (mode == COL_NEXT) h->launches++;  // two passes (ns2d_launch_count)
     const ColMaps* maps = col_maps_for<Real>(h, mode, a);
     engine_ops<Real>(h->nx)->col(mode, scheme, a, h->stream, maps);
 }
@@ -348,9 +349,11 @@ template <typename Real>
 ns2d_status resident_rk4(ns2d_handle* h, int nsteps, double dt, void* rk1_out);
 
 // One RK4 / RK4CN step (RK4Step, Solver/src/solver.c:625-873).  If rk1_out is
-// non-null the stage-1 RHS is stored there (AB4 start-up, solver.c:283).
+// non-null the stage-1 RHS is stored there (AB4 start-up, solver.c:283).  first:
+// the x-space fields of the state are not there yet; next: leave them for another
+// step (COL_NEXT).
 template <typename Real>
-ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
+ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out, bool first = true, bool next = false) {
     using C = Cplx<Real>;
     if (resident_ok(h)) return resident_rk4<Real>(h, 1, dt, rk1_out);
     if (ns2d_status sb = ensure_band(h)) return sb;
@@ -374,9 +377,11 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
     if (s2) return s2;
 
     ColArgs<Real> a;
-    fill_common<Real>(h, a, branch);
-    a.src = (const C*)h->state;
-    launch_col<Real>(h, COL_P1, a);
+    if (first) {
+        fill_common<Real>(h, a, branch);
+        a.src = (const C*)h->state;
+        launch_col<Real>(h, COL_P1, a);
+    }
     for (int s = 1; s <= 4; ++s) {
         launch_row<Real>(h, s);
         fill_common<Real>(h, a, branch);
@@ -403,7 +408,7 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out) {
             launch_col<Real>(h, COL_STAGE, a, scheme);
         } else {
             if (!explicit_rk4) a.cn = h->cn;
-            launch_col<Real>(h, COL_FINAL, a, scheme);
+            launch_col<Real>(h, next ? COL_NEXT : COL_FINAL, a, scheme);
         }
     }
     CKL(h);
@@ -471,9 +476,22 @@ ns2d_status resident_ab4(ns2d_handle* h, int nsteps, double dt) {
     return NS2D_OK;
 }
 
-// AB4Step past the start-up (Solver/src/solver.c:286-349).
+// The x-space fields of the state, before a run's first step.
 template <typename Real>
-ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
+ns2d_status first_pass(ns2d_handle* h, int branch) {
+    ColArgs<Real> a;
+    fill_common<Real>(h, a, branch);
+    a.src = (const Cplx<Real>*)h->state;
+    launch_col<Real>(h, COL_P1, a);
+    CKL(h);
+    return NS2D_OK;
+}
+
+// AB4Step past the start-up (Solver/src/solver.c:286-349).
+// first, next: as rk4_step_impl; the state's column 0 for the conjugacy step
+// alternates between the two col0 arrays along a run.
+template <typename Real>
+ns2d_status ab4_update_impl(ns2d_handle* h, double dt, bool first = true, bool next = false) {
     using C = Cplx<Real>;
     if (resident_ok(h)) return resident_ab4<Real>(h, 1, dt);
     if (ns2d_status sb = ensure_band(h)) return sb;
@@ -481,16 +499,21 @@ ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
     ColArgs<Real> a;
-    fill_common<Real>(h, a, branch);
-    a.src = (const C*)h->state;
-    a.col0_out = (C*)h->col0[0];  // the final pass rewrites the state's column 0
-    launch_col<Real>(h, COL_P1, a);
+    if (first) {
+        h->ab_col0 = 0;
+        fill_common<Real>(h, a, branch);
+        a.src = (const C*)h->state;
+        a.col0_out = (C*)h->col0[0];  // the final pass rewrites the state's column 0
+        launch_col<Real>(h, COL_P1, a);
+    }
     launch_row<Real>(h);
     fill_common<Real>(h, a, branch);
     a.src = (const C*)h->nl;
     a.dt = dt;
     a.conj_mode = 1;
-    a.conj_src = (const C*)h->col0[0];
+    a.conj_src = (const C*)h->col0[h->ab_col0];
+    h->ab_col0 ^= 1;
+    if (next) a.col0_out = (C*)h->col0[h->ab_col0];
     a.conj_stride = 1;
     if (!euler) {
         ns2d_status s2 = ensure_cn(h, dt, branch);
@@ -501,7 +524,7 @@ ns2d_status ab4_update_impl(ns2d_handle* h, double dt) {
     a.h1 = (const C*)h->ab[1];
     a.h2 = (const C*)h->ab[2];
     a.rhs_store = (C*)h->ab[3];
-    launch_col<Real>(h, COL_FINAL, a, SCH_AB4);
+    launch_col<Real>(h, next ? COL_NEXT : COL_FINAL, a, SCH_AB4);
     CKL(h);
     void* oldest = h->ab[0];
     h->ab[0] = h->ab[1];
@@ -908,17 +931,22 @@ void drop_graph(ns2d_handle* h) {
     if (h->timed_graph) cudaGraphExecDestroy(h->timed_graph);
     h->timed_graph = nullptr;
     h->timed_branch = -1;
-
+    for (auto& g : h->run_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    h->run_branch = -1;
 }
 
-// Captures the launches of one RK4/RK4CN step (recorded, not executed).
-ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out) {
+// Captures the launches of one RK4/RK4CN step (recorded, not executed); first and
+// next as in rk4_step_impl.
+ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out, bool first = true, bool next = false) {
     const int64_t l0 = h->launches;
     cudaGraph_t g = nullptr;
     CK(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    ns2d_status s = DISPATCH(h, rk4_step_impl, h, dt, nullptr);
+    ns2d_status s = DISPATCH(h, rk4_step_impl, h, dt, nullptr, first, next);
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-    h->graph_kernels = (int)(h->launches - l0);
+    if (first) h->graph_kernels = (int)(h->launches - l0);
     h->launches = l0;
     if (s) {
         if (g) cudaGraphDestroy(g);
@@ -934,6 +962,23 @@ ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out) {
     return NS2D_OK;
 }
 
+// Whether a step of dt can be replayed from a graph captured for (dt, *branch): the
+// operator branch stays and the tables the launches read are those of dt.
+bool step_settled(const ns2d_handle* h, double dt, int* branch) {
+    int hf = h->hyper_flag;
+    const bool rk4_lin = h->p.system != NS2D_EULER && h->p.integrator == NS2D_RK4;
+    const int br = h->p.system == NS2D_EULER
+                       ? 4
+                       : ns2d::resolve_branch(hf, h->p.ekmn_drag_flag, quirk(h, NS2D_QUIRK_HYPER_LATCH));
+    // the tables the captured launches read are those of this dt and branch
+    const bool tables = h->p.system == NS2D_EULER ||
+                        (rk4_lin ? h->lint && h->lin_branch == br &&
+                                       h->lin_scale == (quirk(h, NS2D_QUIRK_RK4_LINEAR) ? dt : 1.0)
+                                 : h->cn_dt == dt && h->cn_branch == br);
+    *branch = br;
+    return hf == h->hyper_flag && tables;
+}
+
 // One fixed-dt RK4/RK4CN step for the time loops (ns2d_step_n, ns2d_step_async,
 // the adjoint's record).  The first step with a given dt runs eagerly (it
 // settles the operator branch and its table); the step is then captured
@@ -944,17 +989,8 @@ ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out) {
 ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
     if (h->cap_step || resident_ok(h)) return DISPATCH(h, rk4_step_impl, h, dt, nullptr);
     if (ns2d_status sb = ensure_band(h)) return sb;
-    int hf = h->hyper_flag;
-    const bool rk4_lin = h->p.system != NS2D_EULER && h->p.integrator == NS2D_RK4;
-    const int branch = h->p.system == NS2D_EULER
-                           ? 4
-                           : ns2d::resolve_branch(hf, h->p.ekmn_drag_flag, quirk(h, NS2D_QUIRK_HYPER_LATCH));
-    // the tables the captured launches read are those of this dt and branch
-    const bool tables = h->p.system == NS2D_EULER ||
-                        (rk4_lin ? h->lint && h->lin_branch == branch &&
-                                       h->lin_scale == (quirk(h, NS2D_QUIRK_RK4_LINEAR) ? dt : 1.0)
-                                 : h->cn_dt == dt && h->cn_branch == branch);
-    const bool settled = (hf == h->hyper_flag) && tables;
+    int branch;
+    const bool settled = step_settled(h, dt, &branch);
     cudaGraphExec_t* gx = h->timing ? &h->timed_graph : &h->step_graph;
     double* gdt = h->timing ? &h->timed_dt : &h->graph_dt;
     int* gbr = h->timing ? &h->timed_branch : &h->graph_branch;
@@ -991,6 +1027,39 @@ ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
     return NS2D_OK;
 }
 
+// n fixed-dt RK4/RK4CN steps in a row: between two of them the final pass goes on to
+// the next step's first (COL_NEXT), one launch and a read of the state less per
+// step.  The states are those of n single steps, bit for bit.
+ns2d_status rk4_run(ns2d_handle* h, int n, double dt) {
+    int branch = 0;
+    // ZERO forcing rewrites the state between steps; an unsettled step settles alone
+    while (n > 0 && (n < 2 || h->timing || h->cap_step || h->p.forcing == NS2D_FORCING_ZERO || !step_settled(h, dt, &branch))) {
+        if (ns2d_status s = rk4_step_loop(h, dt)) return s;
+        --n;
+    }
+    if (n == 0) return NS2D_OK;
+    if (ns2d_status sb = ensure_band(h)) return sb;
+    if (!(h->run_graph[0] && h->run_graph[1] && h->run_dt == dt && h->run_branch == branch)) {
+        for (int last = 0; last < 2; ++last) {
+            if (h->run_graph[last]) cudaGraphExecDestroy(h->run_graph[last]);
+            h->run_graph[last] = nullptr;
+        }
+        for (int last = 0; last < 2; ++last)
+            if (ns2d_status s = capture_step(h, dt, &h->run_graph[last], false, last == 0)) return s;
+        h->run_dt = dt;
+        h->run_branch = branch;
+    }
+    ns2d_status s = h->fp32 ? first_pass<float>(h, branch) : first_pass<double>(h, branch);
+    if (s) return s;
+    h->status_seen = false;
+    for (int k = 0; k < n; ++k) {
+        cudaError_t e = cudaGraphLaunch(h->run_graph[k == n - 1], h->stream);
+        if (e != cudaSuccess) return fail(h, NS2D_ERR_CUDA, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e));
+        h->launches += k == n - 1 ? 8 : 9;
+    }
+    return NS2D_OK;
+}
+
 // nsteps fixed-dt steps of the configured integrator, queued on the handle's
 // stream.
 ns2d_status queue_steps(ns2d_handle* h, int nsteps, double dt) {
@@ -1009,9 +1078,12 @@ ns2d_status queue_steps(ns2d_handle* h, int nsteps, double dt) {
             if (h->p.integrator == NS2D_AB4) s = DISPATCH(h, resident_ab4, h, n, dt);
             else s = DISPATCH(h, resident_rk4, h, n, dt, nullptr);
         } else if (h->p.integrator == NS2D_AB4) {
-            s = DISPATCH(h, ab4_update_impl, h, dt);
+            const bool alone = h->timing || h->p.forcing == NS2D_FORCING_ZERO;
+            n = alone ? 1 : nsteps - k;
+            for (int j = 0; j < n && s == NS2D_OK; ++j) s = DISPATCH(h, ab4_update_impl, h, dt, j == 0, j < n - 1);
         } else {
-            s = rk4_step_loop(h, dt);
+            n = nsteps - k;
+            s = rk4_run(h, n, dt);
         }
         k += n;
     }

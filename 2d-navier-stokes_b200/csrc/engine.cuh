@@ -77,8 +77,12 @@ struct Launch {
         set_col<COL_FINAL, SCH_CNX>(set);
         set_col<COL_FINAL, SCH_EX>(set);
         set_col<COL_FINAL, SCH_AB4>(set);
+        set_col<COL_NEXT, SCH_CNX>(set);
+        set_col<COL_NEXT, SCH_EX>(set);
+        set_col<COL_NEXT, SCH_AB4>(set);
         set((const void*)col_tma_kernel<Real, N, S::TC, COL_STAGE, SCH_CN>, col_tma_smem());
         set((const void*)col_tma_kernel<Real, N, S::TC, COL_FINAL, SCH_CN>, col_tma_smem());
+        set((const void*)col_tma_kernel<Real, N, S::TC, COL_NEXT, SCH_CN>, col_tma_smem());
         set((const void*)row_kernel<Real, N, S::PAIRS>, row_smem());
         set((const void*)col_inv_kernel<Real, N, S::TC>, inv_smem());
         set((const void*)row_c2r_kernel<Real, N, S::PAIRS, R2_MAXABS>, c2r_smem());
@@ -93,7 +97,7 @@ struct Launch {
     static void col_one(const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps) {
         dim3 grid((a.nyf + S::TC - 1) / S::TC), block(S::T * S::TC);
         if (maps && col_tma_ok(a)) {
-            if constexpr (SCH == SCH_CNX && (MODE == COL_STAGE || MODE == COL_FINAL)) {
+            if constexpr (SCH == SCH_CNX && (MODE == COL_STAGE || MODE == COL_FINAL || MODE == COL_NEXT)) {
                 if (a.dealias == 0 && !a.rhs_store) {
                     launch(col_tma_kernel<Real, N, S::TC, MODE, SCH_CN>, grid, block, col_tma_smem(), s, a, *maps);
                     return;
@@ -114,6 +118,11 @@ struct Launch {
                 if (scheme == SCH_EX) col_one<COL_STAGE, SCH_EX>(a, s, maps);
                 else if (scheme == SCH_DP) col_one<COL_STAGE, SCH_DP>(a, s, maps);
                 else col_one<COL_STAGE, SCH_CNX>(a, s, maps);
+                break;
+            case COL_NEXT:
+                if (scheme == SCH_EX) col_one<COL_NEXT, SCH_EX>(a, s, maps);
+                else if (scheme == SCH_AB4) col_one<COL_NEXT, SCH_AB4>(a, s, maps);
+                else col_one<COL_NEXT, SCH_CNX>(a, s, maps);
                 break;
             default:
                 if (scheme == SCH_EX) col_one<COL_FINAL, SCH_EX>(a, s, maps);

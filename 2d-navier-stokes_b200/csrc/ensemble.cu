@@ -59,8 +59,8 @@ struct ns2d_ensemble {
     // CN tables and graph for the current dt
     double cn_dt = -1.0;
     int cn_branch = -1;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    // one step alone, a step of a run followed by another, a run's last step
+    cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
     double graph_dt = -1.0;
     int graph_col_grid = 0, graph_row_grid = 0, graph_col_var = -1, graph_row_var = -1;
     int graph_fused = -1, graph_stage_grid = 0;
@@ -135,6 +135,7 @@ cudaError_t ens_set_smem(ns2d_ensemble* e) {
     set((const void*)ens_col_kernel<Real, COL_P1, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
     set((const void*)ens_col_kernel<Real, COL_STAGE, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
     set((const void*)ens_col_kernel<Real, COL_FINAL, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
+    set((const void*)ens_col_kernel<Real, COL_NEXT, TH, SCH_CN, false, true>, e->col_tma_smem[V]);
     set((const void*)ens_row_kernel<Real, TH>, e->row_smem[V]);
     return r;
 }
@@ -180,6 +181,14 @@ template <typename Real, int MODE>
 void ens_launch_col(ns2d_ensemble* e, const EnsMember<Real>* mb, const EnsStage& st) {
     if (e->col_var == 0) ens_launch_col_s<Real, MODE, 0>(e, mb, st);
     else ens_launch_col_s<Real, MODE, 1>(e, mb, st);
+}
+
+// Whether a run of steps can go from one step's final pass on to the next's first.
+bool ens_can_run(const ns2d_ensemble* e) { return e->maps && ens_fast(e) && !e->fused; }
+template <typename Real>
+void ens_launch_next(ns2d_ensemble* e, const EnsMember<Real>* mb, const EnsStage& st) {
+    if (e->col_var == 0) ens_launch_col_v<Real, COL_NEXT, 0, SCH_CN, true>(e, mb, st);
+    else ens_launch_col_v<Real, COL_NEXT, 1, SCH_CN, true>(e, mb, st);
 }
 
 template <typename Real>
@@ -391,9 +400,11 @@ ns2d_status create_t(ns2d_ensemble* e) {
     return NS2D_OK;
 }
 
-// One RK4CN / RK4 step of every member: 9 launches.
+// One RK4CN / RK4 step of every member: 9 launches.  first: the members' x-space
+// fields are not there yet; next: leave them for another step (COL_NEXT, in the
+// common step's form only).
 template <typename Real>
-ns2d_status step_t(ns2d_ensemble* e, double dt) {
+ns2d_status step_t(ns2d_ensemble* e, double dt, bool first = true, bool next = false) {
     const bool explicit_rk4 = e->p.system == NS2D_EULER || e->p.integrator == NS2D_RK4;
     const bool latch = (e->p.quirks & NS2D_QUIRK_HYPER_LATCH) != 0;
     int branch = 4;
@@ -451,9 +462,11 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
         if (rf != cudaSuccess) return efail(e, NS2D_ERR_CUDA, cudaGetErrorString(rf));
         return NS2D_OK;
     }
-    st.stage = 0;
-    ens_launch_col<Real, COL_P1>(e, mb, st);
-    e->launches++;
+    if (first) {
+        st.stage = 0;
+        ens_launch_col<Real, COL_P1>(e, mb, st);
+        e->launches++;
+    }
     for (int s = 1; s <= 4; ++s) {
         ens_launch_row<Real>(e, mb);
         e->launches++;
@@ -464,7 +477,8 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
             st.first = (s == 1);
             ens_launch_col<Real, COL_STAGE>(e, mb, st);
         } else {
-            ens_launch_col<Real, COL_FINAL>(e, mb, st);
+            if (next) ens_launch_next<Real>(e, mb, st);
+            else ens_launch_col<Real, COL_FINAL>(e, mb, st);
         }
         e->launches++;
     }
@@ -475,23 +489,26 @@ ns2d_status step_t(ns2d_ensemble* e, double dt) {
 
 #define EDISPATCH(e, fn, ...) ((e)->fp32 ? fn<float>(__VA_ARGS__) : fn<double>(__VA_ARGS__))
 
-// (Re)capture one step into a graph when dt or the grids changed.  Called only
-// after an eager step at this dt, so the CN tables exist and the operator
-// branch is settled: capturing records exactly the 9 pass launches.
-ns2d_status ensure_graph(ns2d_ensemble* e, double dt) {
-    if (e->exec && e->graph_dt == dt && e->graph_col_grid == e->col_grid && e->graph_row_grid == e->row_grid &&
-        e->graph_col_var == e->col_var && e->graph_row_var == e->row_var && e->graph_fused == (int)e->fused &&
-        e->graph_stage_grid == e->stage_grid)
-        return NS2D_OK;
-    if (e->exec) {
-        cudaGraphExecDestroy(e->exec);
-        cudaGraphDestroy(e->graph);
-        e->exec = nullptr;
-        e->graph = nullptr;
+void drop_graphs(ns2d_ensemble* e) {
+    for (auto& g : e->exec) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
     }
+}
+
+// The graph of one step (0: alone, 1: in a run, followed by another, 2: a run's
+// last), captured anew when dt or the grids changed.  Called only after an eager
+// step at this dt, so the CN tables exist and the operator branch is settled:
+// capturing records exactly the pass launches.
+ns2d_status ensure_graph(ns2d_ensemble* e, double dt, int kind) {
+    if (!(e->graph_dt == dt && e->graph_col_grid == e->col_grid && e->graph_row_grid == e->row_grid &&
+          e->graph_col_var == e->col_var && e->graph_row_var == e->row_var && e->graph_fused == (int)e->fused &&
+          e->graph_stage_grid == e->stage_grid))
+        drop_graphs(e);
+    if (e->exec[kind]) return NS2D_OK;
     const int64_t l0 = e->launches;
     ECK(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-    ns2d_status s = EDISPATCH(e, step_t, e, dt);
+    ns2d_status s = EDISPATCH(e, step_t, e, dt, kind == 0, kind == 1);
     cudaGraph_t g = nullptr;
     cudaError_t r = cudaStreamEndCapture(e->stream, &g);
     e->launches = l0;
@@ -500,12 +517,12 @@ ns2d_status ensure_graph(ns2d_ensemble* e, double dt) {
         return s;
     }
     if (r != cudaSuccess) return efail(e, NS2D_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(r));
-    r = cudaGraphInstantiate(&e->exec, g, 0);
+    r = cudaGraphInstantiate(&e->exec[kind], g, 0);
+    cudaGraphDestroy(g);
     if (r != cudaSuccess) {
-        cudaGraphDestroy(g);
+        e->exec[kind] = nullptr;
         return efail(e, NS2D_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(r));
     }
-    e->graph = g;
     e->graph_dt = dt;
     e->graph_col_grid = e->col_grid;
     e->graph_row_grid = e->row_grid;
@@ -513,6 +530,18 @@ ns2d_status ensure_graph(ns2d_ensemble* e, double dt) {
     e->graph_row_var = e->row_var;
     e->graph_fused = (int)e->fused;
     e->graph_stage_grid = e->stage_grid;
+    return NS2D_OK;
+}
+
+// The members' x-space fields, before a run's first step.
+template <typename Real>
+ns2d_status first_pass(ns2d_ensemble* e) {
+    EnsStage st;
+    std::memset(&st, 0, sizeof(st));
+    st.status = e->status;
+    ens_launch_col<Real, COL_P1>(e, (const EnsMember<Real>*)e->members, st);
+    e->launches++;
+    ECK(e, cudaGetLastError());
     return NS2D_OK;
 }
 
@@ -534,9 +563,19 @@ ns2d_status step_async_impl(ns2d_ensemble* e, int nsteps, double dt, bool use_gr
             if (e->p.integrator == NS2D_RK4 || e->p.system == NS2D_EULER) e->cn_dt = dt;
             continue;
         }
-        ns2d_status s = ensure_graph(e, dt);
-        if (s) return s;
-        ECK(e, cudaGraphLaunch(e->exec, e->stream));
+        const int left = nsteps - k;
+        if (left > 1 && ens_can_run(e)) {
+            for (int kind = 1; kind < 3; ++kind)
+                if (ns2d_status s = ensure_graph(e, dt, kind)) return s;
+            if (ns2d_status s = EDISPATCH(e, first_pass, e)) return s;
+            for (int j = 0; j < left; ++j) {
+                ECK(e, cudaGraphLaunch(e->exec[j == left - 1 ? 2 : 1], e->stream));
+                e->launches += j == left - 1 ? 8 : 9;
+            }
+            return NS2D_OK;
+        }
+        if (ns2d_status s = ensure_graph(e, dt, 0)) return s;
+        ECK(e, cudaGraphLaunch(e->exec[0], e->stream));
         e->launches += e->fused ? 4 : 9;
     }
     return NS2D_OK;
@@ -678,8 +717,7 @@ ns2d_status ns2d_ensemble_destroy(ns2d_ensemble* e) {
     if (!e) return NS2D_ERR_INVALID;
     cudaSetDevice(e->p.device);
     cudaStreamSynchronize(e->stream);
-    if (e->exec) cudaGraphExecDestroy(e->exec);
-    if (e->graph) cudaGraphDestroy(e->graph);
+    drop_graphs(e);
     for (void* p : e->allocs) cudaFree(p);
     cudaStreamDestroy(e->own);
     delete e;
@@ -841,12 +879,7 @@ ns2d_status ns2d_ensemble_set_stream(ns2d_ensemble* e, void* stream) {
     if (!e) return NS2D_ERR_INVALID;
     ECK(e, cudaStreamSynchronize(e->stream));
     e->stream = stream ? (cudaStream_t)stream : e->own;
-    if (e->exec) {
-        cudaGraphExecDestroy(e->exec);
-        cudaGraphDestroy(e->graph);
-        e->exec = nullptr;
-        e->graph = nullptr;
-    }
+    drop_graphs(e);
     return NS2D_OK;
 }
 

@@ -32,7 +32,9 @@
 
 namespace ns2d {
 
-enum ColMode : int { COL_P1 = 0, COL_RHS = 1, COL_STAGE = 2, COL_FINAL = 3 };
+// COL_NEXT is the final pass followed by the next step's first pass, for steps
+// that are known to be followed by another: the updated state is already at hand.
+enum ColMode : int { COL_P1 = 0, COL_RHS = 1, COL_STAGE = 2, COL_FINAL = 3, COL_NEXT = 4 };
 
 // Update schemes of the stage and final column passes: RK4 with Crank-Nicolson
 // factors under the 2/3 rule (the common step), the same with Hou-Li dealiasing or
@@ -413,12 +415,12 @@ __device__ __forceinline__ void derived_ifft(const typename Cx<Real>::T* pre0, t
 // to drain at the end.  Without SPLIT the second pair transforms batched in
 // (B2, B0) instead (a persistent caller's next tile overlaps the drain, and the
 // batched pair keeps the transforms' ILP).  pending: a store issued before
-// this call still reads B1 (the accumulator).  Thread 0 returns once all
-// stores have completed.
+// this call still reads B1 (1: the accumulator) or B2 (2: the state).  Thread 0
+// returns once all stores have completed.
 template <typename Real, int N, int TC, bool SPLIT>
 __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typename Cx<Real>::T* sm,
                                                  const ColMaps* maps, int tile, int ky, int t, int c,
-                                                 const TwSeed<typename Cx<Real>::T>& seed, bool pending) {
+                                                 const TwSeed<typename Cx<Real>::T>& seed, int pending) {
     using C = typename Cx<Real>::T;
     constexpr int T = Plan<N>::T;
     constexpr int E = N / T;
@@ -439,8 +441,9 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
             }
             // first pair: the accumulator store (if any) must have read B1;
             // second pair: the first pair's first field must have left B0 (at
-            // most its second group still pending), and every thread has read B2
-            if (fp == 0 ? pending : true) {
+            // most its second group still pending, the state's store before it
+            // done), and every thread has read B2
+            if (fp == 0 ? pending == 1 : true) {
                 if (threadIdx.x == 0) {
                     if (fp == 0) bulk_wait_read_all();
                     else asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
@@ -472,7 +475,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
                 const int i = t + T * m;
                 derived_pair(0, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
             }
-            if (pending) {  // the accumulator store must have read B1
+            if (pending == 1) {  // the accumulator store must have read B1
                 if (threadIdx.x == 0) bulk_wait_read_all();
                 __syncthreads();
             }
@@ -497,6 +500,8 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
             const int i = t + T * m;
             derived_pair(1, kx_of<Real, N, T>(m, t, tr), kyr, pre0[i * TC + c], v[0][m], v[1][m]);
         }
+        // the state's store (older than the first pair's two) must have read B2
+        if (pending == 2 && threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 2;\n" ::: "memory");
         __syncthreads();  // every thread has read B2
 #pragma unroll 1
         for (int b = 0; b < 2; ++b) {
@@ -563,8 +568,9 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
     const bool dead = tile * TC >= a.kc;
     const auto seed = twiddle_seeds<N>(a.tw, t);
     constexpr bool XTRA = SCH != SCH_CN;  // Hou-Li factors, a stored RHS
-    constexpr bool need_state = (MODE == COL_STAGE || MODE == COL_FINAL);
-    const bool need_acc = (MODE == COL_STAGE && SCH != SCH_DP && !a.first) || (MODE == COL_FINAL && SCH != SCH_AB4);
+    constexpr bool FIN = MODE == COL_FINAL || MODE == COL_NEXT;
+    constexpr bool need_state = MODE == COL_STAGE || FIN;
+    const bool need_acc = (MODE == COL_STAGE && SCH != SCH_DP && !a.first) || (FIN && SCH != SCH_AB4);
     // TMA: [0] the input, [1] state and accumulator
     __shared__ __align__(8) unsigned long long bar_tile[2];
     auto issue = [&] {
@@ -681,7 +687,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
             }
             cp_async_commit();
         }
-        if constexpr (MODE == COL_FINAL) {
+        if constexpr (FIN) {
             // the Crank-Nicolson factors are read in the epilogue: start bringing
             // this thread's entries into L2 now, under the forward transform
             if (SCH != SCH_EX && a.cn && valid) {
@@ -774,7 +780,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                     const C w = cconj(a.conj_src[(size_t)(N - i) * a.conj_stride]);
                     if constexpr (need_state) pre0[i * TC + c] = w;
                     // (the TMA final pass stores this element's update through the tile copy)
-                    if constexpr (!(TMA && MODE == COL_FINAL)) a.state[(size_t)i * ldc] = w;
+                    if constexpr (!(TMA && FIN)) a.state[(size_t)i * ldc] = w;
                 }
             }
         }
@@ -813,16 +819,16 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         }
         double bsum = 0.0;
         bool bad = false;
-        constexpr int EB = E < 4 ? E : (MODE == COL_FINAL && (SCH == SCH_CN || SCH == SCH_CNX) && E >= 8) ? 8 : 4;
+        constexpr int EB = E < 4 ? E : (FIN && (SCH == SCH_CN || SCH == SCH_CNX) && E >= 8) ? 8 : 4;
         const Real bc = (Real)a.b_cur;
         const Real adt = (Real)(a.dt * a.a_next);
 #pragma unroll
         for (int m0 = 0; m0 < (SCH == SCH_DP ? 0 : E); m0 += EB) {
             C w[EB], acc[EB], xs[SCH == SCH_EX ? EB : 1], p0[SCH == SCH_AB4 ? EB : 1], p1[SCH == SCH_AB4 ? EB : 1],
                 p2[SCH == SCH_AB4 ? EB : 1];
-            double2 f[MODE == COL_FINAL ? EB : 1];
+            double2 f[FIN ? EB : 1];
             Real br[SCH == SCH_EX ? EB : 1];
-            if constexpr (MODE == COL_FINAL && SCH != SCH_EX) {
+            if constexpr (FIN && SCH != SCH_EX) {
                 // Crank-Nicolson factors (solver.c:853), from the table
                 if (SCH != SCH_AB4 || a.cn) {
 #pragma unroll
@@ -900,8 +906,8 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                             }
                         }
                     }
-                    if constexpr (TMA) pre0[q] = wn;  // staged for the tile store
-                    else if (valid) a.state[(size_t)i * ldc + ky] = wn;
+                    if constexpr (TMA || MODE == COL_NEXT) pre0[q] = wn;  // staged for the tile store, the next stage input
+                    if (!TMA && valid) a.state[(size_t)i * ldc + ky] = wn;
                     if (valid) {
                         const double mag = fabs((double)wn.x) + fabs((double)wn.y);
                         bad |= !isfinite(mag);
@@ -910,8 +916,8 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                 }
             }
         }
-        if constexpr (MODE == COL_STAGE && SCH != SCH_DP) {
-            if (ky == 0) {
+        if constexpr ((MODE == COL_STAGE && SCH != SCH_DP) || MODE == COL_NEXT) {
+            if (ky == 0 && (MODE == COL_STAGE || a.col0_out)) {
 #pragma unroll
                 for (int m = 0; m < E; ++m) a.col0_out[t + T * m] = pre0[(t + T * m) * TC + c];
             }
@@ -925,22 +931,17 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                 bulk_commit();
             }
         }
-        if constexpr (TMA && MODE == COL_FINAL) {
+        if constexpr (TMA && FIN) {
             if (threadIdx.x == 0) {
                 tma_store_tile<C, N, TC>(&maps->state, tile, pre0);
                 bulk_commit();
             }
         }
-        if constexpr (MODE == COL_FINAL) {
+        if constexpr (FIN) {
             if (!a.final_tail) {
                 // ensemble form: only the non-finite check
                 if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(a.status, 1);
-                __syncthreads();
-                if constexpr (TMA) {
-                    if (threadIdx.x == 0) bulk_wait_all();
-                }
-                return true;
-            }
+            } else {
             // SystemCheck (solver.c:2301-2326) without a transform: max|w(x)| is
             // bounded by sum|w_hat|/(Nx Ny) over the full spectrum.  Status bit 1:
             // non-finite state; bit 2: the bound may reach 1e100 (the host then
@@ -964,15 +965,19 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
                 if (!(tot * a.inv_nxny < 1e100 / (double)a.ntiles)) atomicOr(a.status, 2);
                 if (tile == 0) atomicAdd(a.status + 1, 1);  // completed steps
             }
-            __syncthreads();
-            if constexpr (TMA) {
-                if (threadIdx.x == 0) bulk_wait_all();
             }
-            return true;
+            __syncthreads();
+            if constexpr (MODE == COL_FINAL) {
+                if constexpr (TMA) {
+                    if (threadIdx.x == 0) bulk_wait_all();
+                }
+                return true;
+            }
         }
     }
 
-    if constexpr (TMA) derived_ifft_tma<Real, N, TC, SPLIT>(pre0, sm, maps, tile, ky, t, c, seed, MODE == COL_STAGE && SCH != SCH_DP);
+    if constexpr (TMA) derived_ifft_tma<Real, N, TC, SPLIT>(pre0, sm, maps, tile, ky, t, c, seed,
+                                                        MODE == COL_NEXT ? 2 : MODE == COL_STAGE && SCH != SCH_DP ? 1 : 0);
     else derived_ifft<Real, N, TC>(pre0, sm, a.f0, a.f1, a.f2, a.f3, ldc, ky, valid, t, c, seed);
     return true;
 }

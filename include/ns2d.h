@@ -442,7 +442,8 @@ ns2d_status ns2d_set_kernel_timing(ns2d_handle* h, int32_t enable);
 ns2d_status ns2d_kernel_times(ns2d_handle* h, double* ms_total, int64_t* launches, int32_t nclasses);
 ns2d_status ns2d_synchronize(ns2d_handle* h);
 /* Number of kernel launches issued by this handle since creation; a launch that
-   advances several steps of a small grid (16..128) counts once per step. */
+   advances several steps of a small grid (16..128) counts once per step, and one
+   that ends a step and begins the next counts as the two passes it runs. */
 int64_t ns2d_launch_count(const ns2d_handle* h);
 
 #ifdef __cplusplus

@@ -141,3 +141,27 @@ def test_houli_steps_match_oracle(n, integ, quirks):
         o.ab4_step(d, k + 1) if integ == abi.AB4 else o.rk4_step(d)
     assert rel_err(s.get_w_hat(), o.get_w_hat()) <= 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("precision", [abi.FP64, abi.FP32])
+@pytest.mark.parametrize("integ", [abi.RK4CN, abi.RK4, abi.AB4])
+@pytest.mark.parametrize("dealias", [abi.DEALIAS_23, abi.DEALIAS_HOU_LI])
+@pytest.mark.parametrize("n", [256, 1024])
+def test_runs_equal_single_steps(n, dealias, integ, precision):
+    """In a run of steps the final pass goes on to the next step's first; the
+    states are those of single steps, bit for bit, over run lengths and changes
+    of dt, and so are the column 0 snapshots AB4's conjugacy takes."""
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, integrator=integ, dealias=dealias, precision=precision)
+    w0 = initial.decaying(n, seed=12, k0=n / 16.0, dealias="2/3")
+    a, b = Solver(p), Solver(p)
+    a.set_w_hat(w0)
+    b.set_w_hat(w0)
+    k = 0
+    for run, dt in ((5, 1e-4), (2, 1e-4), (1, 1e-4), (3, 5e-5), (4, 1e-4)):
+        a.step_n(run, dt)
+        for _ in range(run):
+            k += 1
+            b.ab4_step(dt, k) if integ == abi.AB4 else b.rk4_step(dt)
+        assert np.array_equal(a.get_w_hat(), b.get_w_hat()), k
+    a.close()
+    b.close()
