@@ -177,12 +177,13 @@ struct TimedLaunch {
 template <typename Real>
 void build_col_maps(ns2d_handle* h) {
     if (!tma_copies_enabled()) return;
-    const int tc = engine_ops<Real>(h->nx)->tc;
-    auto* m = new (std::nothrow) ColMaps;
+    const auto* ops = engine_ops<Real>(h->nx);
+    auto* m = new (std::nothrow) ColMaps[2];  // [1]: the stage pass's tiles
     if (!m) return;
     void* const bases[7] = {h->f[0], h->f[1], h->f[2], h->f[3], h->acc, h->state, h->nl};
-    if (!encode_col_maps<Real>(m, bases, h->nx, h->nyf, h->ldc, tc)) {
-        delete m;
+    if (!encode_col_maps<Real>(&m[0], bases, h->nx, h->nyf, h->ldc, ops->tc) ||
+        !encode_col_maps<Real>(&m[1], bases, h->nx, h->nyf, h->ldc, ops->tc_stage)) {
+        delete[] m;
         return;
     }
     h->col_maps = m;
@@ -208,7 +209,7 @@ void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a, int scheme = S
     h->status_seen = false;
     if (mode == COL_NEXT) h->launches++;  // two passes (ns2d_launch_count)
     const ColMaps* maps = col_maps_for<Real>(h, mode, a);
-    engine_ops<Real>(h->nx)->col(mode, scheme, a, h->stream, maps);
+    engine_ops<Real>(h->nx)->col(mode, scheme, a, h->stream, maps, maps ? maps + 1 : nullptr);
 }
 // Row pass of stage `stage` (1..4); with a capture target set, the stage's real
 // fields go to planes 2(stage-1) and 2(stage-1)+1 of it.
@@ -858,7 +859,7 @@ void free_all(ns2d_handle* h) {
         if (p) cudaFree(p);
     if (h->dp_kptr) cudaFree((void*)h->dp_kptr);
     if (h->pin) cudaFreeHost(h->pin);
-    delete static_cast<ColMaps*>(h->col_maps);
+    delete[] static_cast<ColMaps*>(h->col_maps);
     h->col_maps = nullptr;
 }
 
@@ -940,11 +941,12 @@ void drop_graph(ns2d_handle* h) {
 
 // Captures the launches of one RK4/RK4CN step (recorded, not executed); first and
 // next as in rk4_step_impl.
-ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out, bool first = true, bool next = false) {
+ns2d_status capture_step(ns2d_handle* h, double dt, cudaGraphExec_t* out, bool first = true, bool next = false, int steps = 1) {
     const int64_t l0 = h->launches;
     cudaGraph_t g = nullptr;
     CK(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    ns2d_status s = DISPATCH(h, rk4_step_impl, h, dt, nullptr, first, next);
+    ns2d_status s = NS2D_OK;
+    for (int k = 0; k < steps && s == NS2D_OK; ++k) s = DISPATCH(h, rk4_step_impl, h, dt, nullptr, first, next);
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (first) h->graph_kernels = (int)(h->launches - l0);
     h->launches = l0;
@@ -1027,6 +1029,11 @@ ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {
     return NS2D_OK;
 }
 
+// Steps of a run in one graph: between graphs the GPU waits a microsecond or two
+// for the next (1024^2 FP32 88.1 -> 86.1 us a step).  Captured once the steps of
+// this dt are many enough to pay for it.
+constexpr int kRunSteps = 8, kRunStepsFrom = 64;
+
 // n fixed-dt RK4/RK4CN steps in a row: between two of them the final pass goes on to
 // the next step's first (COL_NEXT), one launch and a read of the state less per
 // step.  The states are those of n single steps, bit for bit.
@@ -1039,23 +1046,28 @@ ns2d_status rk4_run(ns2d_handle* h, int n, double dt) {
     }
     if (n == 0) return NS2D_OK;
     if (ns2d_status sb = ensure_band(h)) return sb;
-    if (!(h->run_graph[0] && h->run_graph[1] && h->run_dt == dt && h->run_branch == branch)) {
-        for (int last = 0; last < 2; ++last) {
-            if (h->run_graph[last]) cudaGraphExecDestroy(h->run_graph[last]);
-            h->run_graph[last] = nullptr;
+    if (!(h->run_dt == dt && h->run_branch == branch)) {
+        for (auto& g : h->run_graph) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
         }
-        for (int last = 0; last < 2; ++last)
-            if (ns2d_status s = capture_step(h, dt, &h->run_graph[last], false, last == 0)) return s;
         h->run_dt = dt;
         h->run_branch = branch;
+        h->run_total = 0;
     }
+    h->run_total += n;
     ns2d_status s = h->fp32 ? first_pass<float>(h, branch) : first_pass<double>(h, branch);
     if (s) return s;
     h->status_seen = false;
-    for (int k = 0; k < n; ++k) {
-        cudaError_t e = cudaGraphLaunch(h->run_graph[k == n - 1], h->stream);
+    for (int k = 0; k < n;) {
+        const int kind = k == n - 1 ? 1 : n - 1 - k >= kRunSteps && h->run_total >= kRunStepsFrom ? 2 : 0;
+        const int steps = kind == 2 ? kRunSteps : 1;
+        if (!h->run_graph[kind])
+            if (ns2d_status sc = capture_step(h, dt, &h->run_graph[kind], false, kind != 1, steps)) return sc;
+        cudaError_t e = cudaGraphLaunch(h->run_graph[kind], h->stream);
         if (e != cudaSuccess) return fail(h, NS2D_ERR_CUDA, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e));
-        h->launches += k == n - 1 ? 8 : 9;
+        h->launches += kind == 1 ? 8 : 9 * steps;
+        k += steps;
     }
     return NS2D_OK;
 }

@@ -19,6 +19,12 @@ struct Shape {
     static constexpr int T = Plan<N>::T;
     static constexpr int TC_RAW = 128 / T < 2 ? 2 : 128 / T;
     static constexpr int TC = (N == 16) ? 8 : (N == 1024) ? 4 : (N == 256) ? 2 : TC_RAW;
+    // The common step's stage pass, which moves everything by TMA, two columns per
+    // block at 1024 in FP64: two blocks share an SM and overlap their phases (22.5 us
+    // a launch against 24.0).  Passes that read per-thread arrays keep four (AB4 step
+    // 47 us, 53 with two; 32-byte rows are two to a line), and so does FP32 (17.7
+    // against 19.1: 16-byte rows).
+    static constexpr int TC_STAGE = (N == 1024 && sizeof(Real) == 8) ? 2 : TC;
     static constexpr int PAIRS_RAW = (N == 256) ? 1 : (128 / T) / 2 < 1 ? 1 : (128 / T) / 2;
     static constexpr int PAIRS = PAIRS_RAW > N / 2 ? N / 2 : PAIRS_RAW;
 };
@@ -30,6 +36,7 @@ struct Launch {
     static constexpr int SIZE = N;
     static constexpr size_t col_smem() { return ColSmem<Real, N, S::TC>::bytes(); }
     static constexpr size_t col_tma_smem() { return ColSmem<Real, N, S::TC>::bytes_tma() + 1024; }
+    static constexpr size_t stage_tma_smem() { return ColSmem<Real, N, S::TC_STAGE>::bytes_tma() + 1024; }
     static constexpr size_t row_smem() { return RowSmem<Real, N, 2 * S::PAIRS>::bytes(); }
     static constexpr size_t inv_smem() { return sizeof(C) * SmemLayout<N, S::TC>::ELEMS; }
     static constexpr size_t c2r_smem() {
@@ -80,7 +87,7 @@ struct Launch {
         set_col<COL_NEXT, SCH_CNX>(set);
         set_col<COL_NEXT, SCH_EX>(set);
         set_col<COL_NEXT, SCH_AB4>(set);
-        set((const void*)col_tma_kernel<Real, N, S::TC, COL_STAGE, SCH_CN>, col_tma_smem());
+        set((const void*)col_tma_kernel<Real, N, S::TC_STAGE, COL_STAGE, SCH_CN>, stage_tma_smem());
         set((const void*)col_tma_kernel<Real, N, S::TC, COL_FINAL, SCH_CN>, col_tma_smem());
         set((const void*)col_tma_kernel<Real, N, S::TC, COL_NEXT, SCH_CN>, col_tma_smem());
         set((const void*)row_kernel<Real, N, S::PAIRS>, row_smem());
@@ -94,11 +101,16 @@ struct Launch {
     }
 
     template <int MODE, int SCH>
-    static void col_one(const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps) {
+    static void col_one(const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps, const ColMaps* stage_maps) {
         dim3 grid((a.nyf + S::TC - 1) / S::TC), block(S::T * S::TC);
         if (maps && col_tma_ok(a)) {
             if constexpr (SCH == SCH_CNX && (MODE == COL_STAGE || MODE == COL_FINAL || MODE == COL_NEXT)) {
-                if (a.dealias == 0 && !a.rhs_store) {
+                if (MODE == COL_STAGE && a.dealias == 0 && !a.rhs_store && stage_maps) {
+                    dim3 sgrid((a.nyf + S::TC_STAGE - 1) / S::TC_STAGE), sblock(S::T * S::TC_STAGE);
+                    launch(col_tma_kernel<Real, N, S::TC_STAGE, MODE, SCH_CN>, sgrid, sblock, stage_tma_smem(), s, a, *stage_maps);
+                    return;
+                }
+                if (MODE != COL_STAGE && a.dealias == 0 && !a.rhs_store) {
                     launch(col_tma_kernel<Real, N, S::TC, MODE, SCH_CN>, grid, block, col_tma_smem(), s, a, *maps);
                     return;
                 }
@@ -109,25 +121,26 @@ struct Launch {
         }
     }
     // scheme: SCH_CN, SCH_EX, SCH_AB4 or SCH_DP (stage and final passes); maps: tensor maps
-    // of the arrays the pass reads and writes (null: per-thread copies).
-    static void col(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps = nullptr) {
+    // of the arrays the pass reads and writes (null: per-thread copies), stage_maps
+    // the same for the stage pass's tiles.
+    static void col(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps, const ColMaps* stage_maps) {
         switch (mode) {
-            case COL_P1: col_one<COL_P1, SCH_CNX>(a, s, maps); break;
-            case COL_RHS: col_one<COL_RHS, SCH_CNX>(a, s, maps); break;
+            case COL_P1: col_one<COL_P1, SCH_CNX>(a, s, maps, stage_maps); break;
+            case COL_RHS: col_one<COL_RHS, SCH_CNX>(a, s, maps, stage_maps); break;
             case COL_STAGE:
-                if (scheme == SCH_EX) col_one<COL_STAGE, SCH_EX>(a, s, maps);
-                else if (scheme == SCH_DP) col_one<COL_STAGE, SCH_DP>(a, s, maps);
-                else col_one<COL_STAGE, SCH_CNX>(a, s, maps);
+                if (scheme == SCH_EX) col_one<COL_STAGE, SCH_EX>(a, s, maps, stage_maps);
+                else if (scheme == SCH_DP) col_one<COL_STAGE, SCH_DP>(a, s, maps, stage_maps);
+                else col_one<COL_STAGE, SCH_CNX>(a, s, maps, stage_maps);
                 break;
             case COL_NEXT:
-                if (scheme == SCH_EX) col_one<COL_NEXT, SCH_EX>(a, s, maps);
-                else if (scheme == SCH_AB4) col_one<COL_NEXT, SCH_AB4>(a, s, maps);
-                else col_one<COL_NEXT, SCH_CNX>(a, s, maps);
+                if (scheme == SCH_EX) col_one<COL_NEXT, SCH_EX>(a, s, maps, stage_maps);
+                else if (scheme == SCH_AB4) col_one<COL_NEXT, SCH_AB4>(a, s, maps, stage_maps);
+                else col_one<COL_NEXT, SCH_CNX>(a, s, maps, stage_maps);
                 break;
             default:
-                if (scheme == SCH_EX) col_one<COL_FINAL, SCH_EX>(a, s, maps);
-                else if (scheme == SCH_AB4) col_one<COL_FINAL, SCH_AB4>(a, s, maps);
-                else col_one<COL_FINAL, SCH_CNX>(a, s, maps);
+                if (scheme == SCH_EX) col_one<COL_FINAL, SCH_EX>(a, s, maps, stage_maps);
+                else if (scheme == SCH_AB4) col_one<COL_FINAL, SCH_AB4>(a, s, maps, stage_maps);
+                else col_one<COL_FINAL, SCH_CNX>(a, s, maps, stage_maps);
                 break;
         }
     }
@@ -178,9 +191,9 @@ inline bool with_size(int n, F&& f) {
 // engine_f32.cu and engine_f64.cu.
 template <typename Real>
 struct EngineOps {
-    int tc;  // column-tile width
+    int tc, tc_stage;  // column-tile widths: of the passes, of the common step's stage pass
     cudaError_t (*setup)();
-    void (*col)(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps);
+    void (*col)(int mode, int scheme, const ColArgs<Real>& a, cudaStream_t s, const ColMaps* maps, const ColMaps* stage_maps);
     void (*row)(const RowArgs<Real>& a, cudaStream_t s);
     void (*col_inv)(const InvArgs<Real>& a, cudaStream_t s);
     void (*fwd)(int pass, const double* real_in, const typename Cx<Real>::T* in, typename Cx<Real>::T* out, int nlines,

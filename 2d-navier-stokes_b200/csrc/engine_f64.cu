@@ -8,7 +8,7 @@ const EngineOps<double>* engine_ops<double>(int n) {
     const EngineOps<double>* ops = nullptr;
     with_size<double>(n, [&](auto L) {
         using E = decltype(L);
-        static const EngineOps<double> o{E::S::TC, E::setup, E::col, E::row, E::col_inv, E::fwd, E::row_c2r};
+        static const EngineOps<double> o{E::S::TC, E::S::TC_STAGE, E::setup, E::col, E::row, E::col_inv, E::fwd, E::row_c2r};
         ops = &o;
     });
     return ops;

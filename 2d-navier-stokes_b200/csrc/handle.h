@@ -91,10 +91,12 @@ struct ns2d_handle {
     double dp_err = 0.0;
     // one RK4/RK4CN step captured as a CUDA graph for fixed-dt stepping
     cudaGraphExec_t step_graph = nullptr;
-    // a step within a run of steps, followed by another ([0]) or the last ([1])
-    cudaGraphExec_t run_graph[2] = {nullptr, nullptr};
+    // a step within a run of steps, followed by another ([0]) or the last ([1]), and
+    // several followed by another ([2])
+    cudaGraphExec_t run_graph[3] = {nullptr, nullptr, nullptr};
     double run_dt = 0.0;
     int run_branch = -1;
+    int64_t run_total = 0;     // steps taken in runs of this dt and branch
     int ab_col0 = 0;           // the col0 array that holds the state's column 0 (AB4 runs)
     int graph_kernels = 9;  // kernels in one captured step
     double graph_dt = 0.0;

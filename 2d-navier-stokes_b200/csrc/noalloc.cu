@@ -145,7 +145,7 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
     }
     a.norm2 = std::pow(1.0 / (double)(n * n), 2.0);
     const EngineOps<double>* ops = engine_ops<double>(n);
-    ops->col(COL_P1, SCH_CN, a, st, nullptr);
+    ops->col(COL_P1, SCH_CN, a, st, nullptr, nullptr);
 
     RowArgs<double> r{};
     r.f0 = f[0];
@@ -163,7 +163,7 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
     a.src = nl;
     a.rhs_store = (double2*)d_rhs;  // no state here: the conjugacy side effect is not applied
     a.conj_mode = 0;
-    ops->col(COL_RHS, SCH_CN, a, st, nullptr);
+    ops->col(COL_RHS, SCH_CN, a, st, nullptr, nullptr);
     // no error was pending on entry, so one found now is a launch of this call
     if (cudaGetLastError() != cudaSuccess) return NS2D_ERR_CUDA;
     return NS2D_OK;
