@@ -45,6 +45,8 @@ struct ns2d_handle {
     bool band_known = false;   // dband[0] describes the state
     bool ffield_band = false;  // the listed forcing has modes in the columns dealiasing empties
     bool band_forced = false;  // and the state may hold their trace
+    double2* dio2 = nullptr;   // the same for results (small grids)
+    void* pin_io = nullptr;    // page-locked staging of both (small grids)
     double2* dio = nullptr;    // staging [nx][nyf] complex128
     double* ddiag = nullptr;   // measurables: DG_N totals + 8 * n_spect spectra
     double* dpart = nullptr;   // per-block partial bounds of the final column pass

@@ -49,6 +49,8 @@ template <typename Real>
 struct ResArgs {
     using C = typename Cx<Real>::T;
     const C* src;          // RES_RHS: the evaluation's input
+    const double2* src64;  // where the input or state comes from instead, in the caller's layout [N][nyf] ...
+    double2* out64;        // ... and where the RHS or the new state also goes; both or neither for steps
     C* state;              // w_hat
     C* rhs;                // RES_RHS: the RHS; RES_CN: stage 1's RHS of every step (AB4 start-up), may be null
     C* h[4];               // AB4: RHS of steps n-3, n-2, n-1, and the one to be written
@@ -188,7 +190,12 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
             const size_t g = (size_t)i * a.ldc + ky;
             const int kx = (i <= N / 2) ? i : i - N;
             const int k2 = kx * kx + ky * ky;
-            w = rhs_only ? a.src[g] : a.state[g];
+            if (a.src64) {
+                const double2 d64 = a.src64[(size_t)i * a.nyf + ky];
+                w = cmake<C>((Real)d64.x, (Real)d64.y);
+            } else {
+                w = rhs_only ? a.src[g] : a.state[g];
+            }
             if (k2 != 0) inv = inv_k2<Real>((Real)k2);
             if constexpr (SCHEME == RES_EXPLICIT) {
                 if (a.lin_stage && k2 != 0) {
@@ -217,7 +224,23 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
     }
     wide = __syncthreads_or(wide);
     cluster_sync<CL>();  // every block runs and has cleared its flags
-    if (status0) return;
+    // The state goes back to where the step's result is expected (and over any
+    // earlier content of the columns left out below).
+    auto put_state = [&](int n) {
+        for (int q = threadIdx.x; q < n * N; q += NT) {
+            const int ky = rank + CL * (q / N), i = q % N;
+            if (ky >= a.nyf) continue;
+            const C w = sW[q];
+            a.state[(size_t)i * a.ldc + ky] = w;
+            if (a.out64) a.out64[(size_t)i * a.nyf + ky] = make_double2((double)w.x, (double)w.y);
+        }
+    };
+    if (status0) {
+        if constexpr (!rhs_only) {
+            if (a.src64) put_state(L::SLOTS);
+        }
+        return;
+    }
     if (threadIdx.x < CL) cluster_store(cluster_addr(smem_addr(&s_wide[rank]), threadIdx.x), wide ? 1 : 0);
     cluster_sync<CL>();
     wide = false;
@@ -233,6 +256,12 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
         for (int q = slots * N + threadIdx.x; q < L::SLOTS * N; q += NT) {
             const int ky = rank + CL * (q / N), i = q % N;
             if (ky < a.nyf) fill[(size_t)i * a.ldc + ky] = cmake<C>(0, 0);
+        }
+    }
+    if constexpr (rhs_only) {
+        for (int q = slots * N + threadIdx.x; a.out64 && q < L::SLOTS * N; q += NT) {
+            const int ky = rank + CL * (q / N), i = q % N;
+            if (ky < a.nyf) a.out64[(size_t)i * a.nyf + ky] = make_double2(0.0, 0.0);
         }
     }
     const C* h0 = a.h[0];
@@ -434,6 +463,13 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
 #pragma unroll
                     for (int m = 0; m < E; ++m) store[g0 + (size_t)(T * m) * a.ldc] = v[0][m];
                 }
+                if constexpr (rhs_only) {
+                    if (a.out64) {
+#pragma unroll
+                        for (int m = 0; m < E; ++m)
+                            a.out64[(size_t)(t + T * m) * a.nyf + ky] = make_double2((double)v[0][m].x, (double)v[0][m].y);
+                    }
+                }
                 if constexpr (!rhs_only) {
                     C w[E];
 #pragma unroll
@@ -538,11 +574,8 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
             __syncthreads();  // the stage input is complete before the next derived spectra
         }
     }
-    if (!rhs_only) {
-        for (int q = threadIdx.x; q < slots * N; q += NT) {
-            const int ky = rank + CL * (q / N), i = q % N;
-            a.state[(size_t)i * a.ldc + ky] = sW[q];
-        }
+    if constexpr (!rhs_only) {
+        put_state(a.src64 ? L::SLOTS : slots);
         if (a.status && rank == 0 && threadIdx.x == 0) atomicAdd(a.status + 1, done);
     }
     cluster_sync<CL>();  // no block leaves while another may still store into its shared memory
