@@ -22,9 +22,9 @@
 //   columns: forward x-FFT, dealiasing, forcing, conjugacy, stage combine or
 //            update, all on the block's own columns
 //
-// What bounds it is the chain of latencies: at 64^2 FP64 an evaluation takes about
-// 6,900 cycles, of which the two cluster barriers 1,000-1,300 (a barrier of up to
-// 8 blocks costs about 500 cycles, of 16 about 890), the four transforms on the
+// What bounds it is the chain of latencies: at 64^2 FP64 an evaluation takes 7,000 to
+// 8,000 cycles, of which the two cluster barriers 1,300-2,200 (a barrier of up to
+// 8 blocks costs 500-860 cycles, of 16 about 900), the four transforms on the
 // path about 800 each, and the rest loads, twiddles and the remote stores; at
 // 128^2 FP64 arithmetic and remote-store issue add to it.  Measured per step
 // (RK4CN, 2/3, FP64 / FP32, us): 16^2 28.8 / 28.8 -> 6.4 / 5.3, 32^2 39.0 / 34.9 ->
@@ -278,21 +278,30 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
                 const bool on = u < 4 * slots;
                 const int slot = on ? u >> 2 : 0, f = u & 3;
                 const int ky = rank + CL * slot;
-                // the field's derived spectrum (derived_pair): f & 1 the conj(q) ones
+                // the field's derived spectrum (derived_pair): f & 1 the conj(q) ones,
+                // f >= 2 those of X rather than X/k^2, turned by i.  Selects and exact
+                // signs instead of branches: a warp's teams hold different fields
+                // (an evaluation at 64^2 FP64 9,240 cycles with branches, 8,040 without).
                 const Real tr = (Real)t;
                 const Real kys = (f & 1) ? -(Real)ky : (Real)ky;
+                const bool turn = f >= 2;
+                const Real sx = f == 0 ? (Real)1 : (Real)-1, sy = f == 1 ? (Real)-1 : (Real)1;
                 C v[1][E];
+                Real sc[E];
 #pragma unroll
                 for (int m = 0; m < E; ++m) {
-                    const int q = slot * N + t + T * m;
-                    const Real kx = kx_of<Real, N, T>(m, t, tr);
-                    const Real sc = f < 2 ? sI[q] : (Real)1;
-                    C X = sX[q];
-                    X = cmake<C>(mul_rn(sc, X.x), mul_rn(sc, X.y));
-                    const C d = cmake<C>(fma_rn(kx, X.x, -mul_rn(kys, X.y)), fma_rn(kx, X.y, mul_rn(kys, X.x)));
-                    v[0][m] = f >= 2 ? cmake<C>(-d.y, d.x) : f == 1 ? cmake<C>(-d.x, -d.y) : d;
-                    if (m == 0 && t == 0 && ky == 0) v[0][m] = cmake<C>(0, 0);
+                    v[0][m] = sX[slot * N + t + T * m];
+                    sc[m] = sI[slot * N + t + T * m];
                 }
+#pragma unroll
+                for (int m = 0; m < E; ++m) {
+                    const Real kx = kx_of<Real, N, T>(m, t, tr);
+                    const Real s1 = turn ? (Real)1 : sc[m];
+                    const C X = cmake<C>(mul_rn(s1, v[0][m].x), mul_rn(s1, v[0][m].y));
+                    const C d = cmake<C>(fma_rn(kx, X.x, -mul_rn(kys, X.y)), fma_rn(kx, X.y, mul_rn(kys, X.x)));
+                    v[0][m] = cmake<C>(mul_rn(sx, turn ? d.y : d.x), mul_rn(sy, turn ? d.x : d.y));
+                }
+                if (t == 0 && ky == 0) v[0][0] = cmake<C>(0, 0);
                 fft_batched<N, +1, 1>(v, pol, seed, t);
                 if (on) {
                     const unsigned base = smem_addr(sF + (size_t)ky * L::KS + f * RPC);
