@@ -993,7 +993,7 @@ bool step_settled(const ns2d_handle* h, double dt, int* branch) {
 // the adjoint's record).  The first step with a given dt runs eagerly (it
 // settles the operator branch and its table); the step is then captured
 // once as a CUDA graph of its nine launches and replayed for the following
-// steps.  With kernel timing on, a second graph carries an event pair around
+// steps.  Grids that the resident kernel takes do without: a step is one launch.  With kernel timing on, a second graph carries an event pair around
 // every launch and is read back after each replay.  Stage capture for the
 // adjoint uses the eager form.
 ns2d_status rk4_step_loop(ns2d_handle* h, double dt) {

@@ -27,9 +27,9 @@
 // 8 blocks costs 500-860 cycles, of 16 about 900), the four transforms on the
 // path about 800 each, and the rest loads, twiddles and the remote stores; at
 // 128^2 FP64 arithmetic and remote-store issue add to it.  Measured per step
-// (RK4CN, 2/3, FP64 / FP32, us): 16^2 28.8 / 28.8 -> 6.4 / 5.3, 32^2 39.0 / 34.9 ->
-// 9.5 / 7.6, 64^2 45.3 / 41.1 -> 13.4 / 10.3, 128^2 53.4 / 44.6 -> 20.4 / 16.9 against
-// the pass launches replayed from a graph; explicit RK4 at 64^2 154 -> 14.0 (its
+// (RK4CN, 2/3, FP64 / FP32, us): 16^2 28.8 / 28.8 -> 6.5 / 5.3, 32^2 39.0 / 34.9 ->
+// 9.9 / 7.9, 64^2 45.3 / 41.1 -> 14.0 / 10.3, 128^2 53.4 / 44.6 -> 20.7 / 18.0 against
+// the pass launches replayed from a graph; explicit RK4 at 64^2 154 -> 13.9 (its
 // passes never settled on a graph).
 //
 // Columns that the 2/3 rule empties (ky >= kc, k2 >= kmax_sqr for every kx) hold
