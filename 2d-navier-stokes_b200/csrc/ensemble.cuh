@@ -77,7 +77,8 @@ __device__ __forceinline__ void ens_apply_stage(ColArgs<Real>& a, const EnsMembe
 // Resident blocks per SM the ensemble kernels are compiled for, now that every
 // size's transforms hold eight elements a thread: in FP32 three 256-thread (six
 // 128-thread) blocks, 85 registers a thread (a step of the 64-member ensemble
-// 292 us; two blocks 317, four 314 with spills), in FP64 two of 256, 128 registers
+// 284 us; with the row layout before TeamLayout::slot's 16 292, two blocks 317,
+// four 314 with spills), in FP64 two of 256, 128 registers
 // (453 us; one 547, three 533).
 template <typename Real, int THREADS>
 struct EnsMinBlocks {

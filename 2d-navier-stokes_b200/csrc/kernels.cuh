@@ -1140,7 +1140,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
         const TeamPolicy<NH, C> polh{region, 1 + g};
         fft_batched<NH, -1, 1>(z, polh, twiddle_seeds_strided<NH>(a.tw, t, 2), t);
 #pragma unroll
-        for (int m = 0; m < EH; ++m) region[TLH::slot(t + T * m)] = z[0][m];
+        for (int m = 0; m < EH; ++m) region[TLH::template slot<C>(t + T * m)] = z[0][m];
         polh.sync();
         C* dst = a.nl + (size_t)x * a.ldc;
 #pragma unroll
@@ -1148,7 +1148,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
             const int k = t + T * m;
             if (k >= a.kc) continue;
             const C zk = z[0][m];
-            const C zm = region[TLH::slot((NH - k) & (NH - 1))];
+            const C zm = region[TLH::template slot<C>((NH - k) & (NH - 1))];
             const C ev = cmake<C>((Real)0.5 * (zk.x + zm.x), (Real)0.5 * (zk.y - zm.y));
             const C od = cmake<C>((Real)0.5 * (zk.y + zm.y), (Real)0.5 * (zm.x - zk.x));
             dst[k] = cadd(ev, cmul(__ldg(a.tw + k), od));
@@ -1171,7 +1171,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
     fft_batched<N, -1, 1>(z, pol, seed, t);
     // split: X_a = (Z_k + conj Z_{N-k})/2, X_b = (Z_k - conj Z_{N-k})/(2i)
 #pragma unroll
-    for (int m = 0; m < E; ++m) region[TL::slot(t + T * m)] = z[0][m];
+    for (int m = 0; m < E; ++m) region[TL::template slot<C>(t + T * m)] = z[0][m];
     pol.sync();
     C* dst_a = a.nl + (size_t)(rblock * TC + ga) * a.ldc;
     C* dst_b = dst_a + a.ldc;
@@ -1179,8 +1179,8 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
     for (int m = 0; m < E; ++m) {
         const int k = t + T * m;
         if (k < a.kc) {  // kc <= N/2 + 1
-            const C zk = region[TL::slot(k)];
-            const C zm = region[TL::slot((N - k) & (N - 1))];
+            const C zk = region[TL::template slot<C>(k)];
+            const C zm = region[TL::template slot<C>((N - k) & (N - 1))];
             const C ra = cmake<C>((Real)0.5 * (zk.x + zm.x), (Real)0.5 * (zk.y - zm.y));
             const C rb = cmake<C>((Real)0.5 * (zk.y + zm.y), (Real)0.5 * (zm.x - zk.x));
             if constexpr (T >= 32) {

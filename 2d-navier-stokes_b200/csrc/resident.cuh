@@ -369,15 +369,15 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
                 }
                 fft_batched<N, -1, 1>(z, pol, seed, t);
 #pragma unroll
-                for (int m = 0; m < E; ++m) pol.sm[TeamLayout<N>::slot(t + T * m)] = z[0][m];
+                for (int m = 0; m < E; ++m) pol.sm[TeamLayout<N>::template slot<C>(t + T * m)] = z[0][m];
                 pol.sync();
                 if (on) {
 #pragma unroll
                     for (int m = 0; m < E; ++m) {
                         const int k = t + T * m;
                         if (k < nl_cols) {  // k <= N/2
-                            const C zk = pol.sm[TeamLayout<N>::slot(k)];
-                            const C zm = pol.sm[TeamLayout<N>::slot((N - k) & (N - 1))];
+                            const C zk = pol.sm[TeamLayout<N>::template slot<C>(k)];
+                            const C zm = pol.sm[TeamLayout<N>::template slot<C>((N - k) & (N - 1))];
                             const C ra = cmake<C>((Real)0.5 * (zk.x + zm.x), (Real)0.5 * (zk.y - zm.y));
                             const C rb = cmake<C>((Real)0.5 * (zk.y + zm.y), (Real)0.5 * (zm.x - zk.x));
                             const int at = (k / CL) * N + rank * RPC + 2 * p;
