@@ -667,7 +667,10 @@ def run_gpu(args, rank, world, local_rank):
                         f"checkpoints every {ADJ_EVERY} steps with stage recomputation",
             "adjoint_over_forward": adj[0]["adjoint_over_forward"], "runs": adj,
         }
-    if world == 1 and not args.no_cpu_baseline:
+    from pyoracle import ref_available
+    if world == 1 and not args.no_cpu_baseline and not all(ref_available(v) for v in ("rk4cn", "houli")):
+        line["cpu_baseline"] = {"unavailable": "the reference build (oracle/_ref) is absent"}
+    elif world == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1
         table = cpu_table(threads, runs=5, budget_s=args.cpu_seconds / 6.0)
         main_row = [r for r in table if r["grid"] == f"{N}x{N}" and r["threads"] == threads][0]
