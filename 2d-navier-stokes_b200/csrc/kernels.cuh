@@ -566,7 +566,6 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
     const int kyc = valid ? ky : 0;
     const int ldc = a.ldc;
     const bool dead = tile * TC >= a.kc;
-    const auto seed = twiddle_seeds<N>(a.tw, t);
     constexpr bool XTRA = SCH != SCH_CN;  // Hou-Li factors, a stored RHS
     constexpr bool FIN = MODE == COL_FINAL || MODE == COL_NEXT;
     constexpr bool need_state = MODE == COL_STAGE || FIN;
@@ -608,6 +607,8 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
         pdl_launch();
         pdl_wait();
     }
+    // (the table too: the no-allocation entry point writes it just before)
+    const auto seed = twiddle_seeds<N>(a.tw, t);
     if (!dead) issue();
     const BlockBegin b = begin();
     const bool narrow = b.narrow;

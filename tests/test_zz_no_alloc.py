@@ -87,6 +87,34 @@ def test_noalloc_rhs_recorded_in_a_captured_graph_houli(n):
     s.close()
 
 
+def test_noalloc_sizes_in_turn_without_waits():
+    """Every call writes the twiddle table of its size at the same place, just
+    ahead of its passes: calls of changing size queued back to back, with no wait
+    between them, give each call's own RHS."""
+    import torch
+
+    L = load()
+    sizes = (256, 64, 128, 16, 256, 32, 128, 256, 64, 32, 16, 128) * 4
+    stream = torch.cuda.current_stream().cuda_stream
+    params, ins, expect, outs = {}, {}, {}, []
+    for n in sorted(set(sizes)):
+        params[n] = abi.default_params(nx=n, ny=n, nu=1e-3)
+        w = initial.decaying(n, seed=n, k0=min(6.0, n / 8), dealias="2/3")
+        s = Solver(params[n])
+        expect[n] = s.nonlinear_rhs(w)
+        s.close()
+        ins[n] = torch.from_numpy(w.view(np.float64).copy()).cuda()
+    for n in sizes:
+        outs.append(torch.full_like(ins[n], float("nan")))
+    torch.cuda.synchronize()
+    for n, out in zip(sizes, outs):
+        assert _noalloc(L, params[n], ins[n].data_ptr(), out.data_ptr(), stream) == abi.OK
+    torch.cuda.synchronize()
+    for k, (n, out) in enumerate(zip(sizes, outs)):
+        got = out.cpu().numpy().view(np.complex128).reshape(n, n // 2 + 1)
+        assert np.max(np.abs(got - expect[n])) <= RHS_TOL * np.max(np.abs(expect[n])), (k, n)
+
+
 def test_noalloc_rejects_misaligned_arrays():
     """A float64 view that starts 8 bytes into an allocation is refused
     before anything is launched; the context stays usable."""
