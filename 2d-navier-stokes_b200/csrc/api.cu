@@ -90,7 +90,9 @@ void fill_common(ns2d_handle* h, ColArgs<Real>& a, int branch) {
     a.status = h->dstatus;
     a.final_tail = 1;
     a.force_field = h->ffield_on ? (const C*)h->ffield : nullptr;
-    a.ntiles = (h->nyf + engine_ops<Real>(h->nx)->tc - 1) / engine_ops<Real>(h->nx)->tc;
+    const int tc = engine_ops<Real>(h->nx)->tc;  // the stage pass's width divides it
+    a.ntiles = (h->nyf + tc - 1) / tc;
+    a.kdead = (a.kc + tc - 1) / tc * tc;
     a.lin = make_lin(h, branch);
     a.phase_only = h->p.model == NS2D_MODEL_PHASE_ONLY ? 1 : 0;
 }

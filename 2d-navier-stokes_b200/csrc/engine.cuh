@@ -25,6 +25,7 @@ struct Shape {
     // 47 us, 53 with two; 32-byte rows are two to a line), and so does FP32 (17.7
     // against 19.1: 16-byte rows).
     static constexpr int TC_STAGE = (N == 1024 && sizeof(Real) == 8) ? 2 : TC;
+    static_assert(TC % TC_STAGE == 0, "ColArgs::kdead");
     static constexpr int PAIRS_RAW = (N == 256) ? 1 : (128 / T) / 2 < 1 ? 1 : (128 / T) / 2;
     static constexpr int PAIRS = PAIRS_RAW > N / 2 ? N / 2 : PAIRS_RAW;
 };

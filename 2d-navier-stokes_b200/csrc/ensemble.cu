@@ -266,6 +266,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
         const int km = (int)(n / 3.0);
         a.kmax_sqr = km * km;
         a.kc = kept_columns(n, e->p.dealias, 0);
+        a.kdead = a.kc;  // one tile width for all passes of a step
         a.dealias = e->p.dealias;
         a.houli_int = (e->p.quirks & NS2D_QUIRK_HOU_LI_INT) ? 1 : 0;
         a.kolm = (e->p.forcing == NS2D_FORCING_KOLM) ? 1 : 0;

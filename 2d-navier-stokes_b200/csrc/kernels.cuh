@@ -99,6 +99,8 @@ struct ColArgs {
     int ldc, nyf;
     int kmax_sqr;        // (int)(N/3)^2 for the 2/3 rule
     int kc;              // columns ky >= kc are emptied by the dealiasing (nyf: none)
+    int kdead;           // kc rounded up to the tiles of every pass of a step, which all leave out the
+                         // tiles from here on (one pass would else take up what another left behind)
     const int* band;     // see band_narrow
     int dealias;         // 0: 2/3, 1: Hou-Li
     int houli_int;       // integer k/(N/2) (reference quirk)
@@ -543,7 +545,7 @@ __device__ __forceinline__ void derived_ifft_tma(typename Cx<Real>::T* pre0, typ
 // same shared memory.  A load that does not land within its bound sets status
 // bit 8 and the body returns false (the block must stop); otherwise it returns
 // true.
-// A tile of emptied columns (all ky >= kc) needs no forward transform (its RHS is
+// A tile of emptied columns (all ky >= kdead) needs no forward transform (its RHS is
 // zero) and, when the band is narrow, nothing else either: state and accumulator
 // stay zero there.
 // begin(): the block's flags (BlockBegin) and a block barrier; called once the
@@ -565,7 +567,7 @@ __device__ __forceinline__ bool col_body(const ColArgs<Real>& a, const Begin& be
     const bool valid = ky < a.nyf;
     const int kyc = valid ? ky : 0;
     const int ldc = a.ldc;
-    const bool dead = tile * TC >= a.kc;
+    const bool dead = tile * TC >= a.kdead;
     constexpr bool XTRA = SCH != SCH_CN;  // Hou-Li factors, a stored RHS
     constexpr bool FIN = MODE == COL_FINAL || MODE == COL_NEXT;
     constexpr bool need_state = MODE == COL_STAGE || FIN;

@@ -165,3 +165,28 @@ def test_runs_equal_single_steps(n, dealias, integ, precision):
         assert np.array_equal(a.get_w_hat(), b.get_w_hat()), k
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("run", [True, False])
+@pytest.mark.parametrize("ky", [341, 342, 343])
+def test_forcing_of_an_earlier_state_leaves_nothing_behind(ky, run):
+    """1024^2 FP64, where the stage pass takes two columns a block and the others
+    four, and the emptied columns begin at 341, in the middle of a tile: after
+    steps with a mode forced there, a state set anew steps as on a new handle."""
+    n, dt = 1024, 1e-4
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, dt=dt)
+    w0 = _state(n, "narrow")
+    s, fresh = Solver(p), Solver(p)
+    s.set_w_hat(w0)
+    s.set_forcing_modes([3 * (n // 2 + 1) + ky], [np.abs(w0).max() * (1 + 2j)])
+    s.step_n(2, dt)
+    s.set_forcing_modes([], [])
+    for obj in (s, fresh):
+        obj.set_w_hat(w0)
+        if run:
+            obj.step_n(4, dt)
+        else:
+            obj.rk4_step(dt)
+    assert np.array_equal(s.get_w_hat(), fresh.get_w_hat())
+    s.close()
+    fresh.close()
