@@ -408,9 +408,15 @@ ns2d_status backward_impl(ns2d_handle* h) {
     // the CN table of the recorded dt, before any launch reads it
     ns2d_status s0 = internal::ensure_cn(h, a->dt, a->branch);
     if (s0) return s0;
-    // the state becomes the recorded run's again, which the caller may have
-    // replaced since
-    ACK(h, cudaMemcpyAsync(h->dband, a->band, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+    // The state becomes the recorded run's again, which the caller may have
+    // replaced since; a forcing set since may reach the emptied columns too.  The
+    // word holds for the sweep only: the next step looks at what it left.
+    if (h->band_forced) ACK(h, cudaMemsetAsync(h->dband, 1, sizeof(int), h->stream));
+    else ACK(h, cudaMemcpyAsync(h->dband, a->band, sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+    struct SweepBand {
+        ns2d_handle* h;
+        ~SweepBand() { h->band_known = false; }
+    } sweep_band{h};
     h->band_known = true;
     ACK(h, cudaEventRecord(a->t[2], h->stream));
     ACK(h, cudaStreamWaitEvent(a->stream, a->t[2], 0));  // lambda(T) is written on the handle's stream

@@ -190,3 +190,26 @@ def test_forcing_of_an_earlier_state_leaves_nothing_behind(ky, run):
     assert np.array_equal(s.get_w_hat(), fresh.get_w_hat())
     s.close()
     fresh.close()
+
+
+def test_forcing_set_before_the_reverse_sweep():
+    """A mode in the emptied columns, forced from after the recorded run on: the
+    steps that follow the sweep take it up."""
+    n, dt = 256, 1e-3
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, quirks=0, dt=dt)
+    idx, val = [3 * (n // 2 + 1) + n // 2 - 9, 2 * (n // 2 + 1) + 1], [30.0 * n, 5.0 * n]
+    s, ref = Solver(p), Solver(p)
+    s.set_w_hat(_state(n, "narrow"))
+    s.adjoint_record(6, dt, 3)
+    w6 = s.get_w_hat()
+    s.set_forcing_modes(idx, val)
+    s.adjoint_backward(initial.decaying(n, 8, k0=5.0, dealias="2/3"))
+    assert np.array_equal(s.get_w_hat(), w6)
+    ref.set_w_hat(w6)
+    ref.set_forcing_modes(idx, val)
+    for obj in (s, ref):
+        obj.step_n(4, dt)
+    assert np.abs(ref.get_w_hat()[3, n // 2 - 9]) > 0
+    assert rel_err(s.get_w_hat(), ref.get_w_hat()) <= 1e-12
+    s.close()
+    ref.close()
