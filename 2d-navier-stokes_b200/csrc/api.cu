@@ -314,10 +314,12 @@ ns2d_status ensure_band(ns2d_handle* h) {
     return NS2D_OK;
 }
 
-// The state was written from outside (set_w_hat and the host-resident step).
-void state_replaced(ns2d_handle* h) {
+// The state was written from outside (set_w_hat, which also ends AB4's history, and
+// the host-resident step, which keeps it: right-hand sides of forced steps in there
+// hold the forcing).
+void state_replaced(ns2d_handle* h, bool keep_history = false) {
     h->band_known = false;
-    h->band_forced = h->ffield_on && h->ffield_band;
+    h->band_forced = (h->ffield_on && h->ffield_band) || (keep_history && h->ab_count > 0 && h->band_forced);
 }
 
 // Rebuild the Crank-Nicolson factor table when dt or the operator branch changed.
@@ -1757,7 +1759,7 @@ ns2d_status ns2d_mean_flow(ns2d_handle* h, double* mean_x, double* mean_y) {
 ns2d_status ns2d_rk4_step_host(ns2d_handle* h, double* w_hat, double dt) {
     if (!h || !w_hat) return NS2D_ERR_INVALID;
     cudaSetDevice(h->p.device);
-    state_replaced(h);
+    state_replaced(h, true);
     if (resident_ok(h)) {
         bool direct = false;
         if (ns2d_status su = upload_spec(h, w_hat)) return su;

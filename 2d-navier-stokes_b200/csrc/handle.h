@@ -44,7 +44,7 @@ struct ns2d_handle {
     int* dband = nullptr;      // band_narrow words: [0] the state, [1] the update factors, [2] the explicit linear ones
     bool band_known = false;   // dband[0] describes the state
     bool ffield_band = false;  // the listed forcing has modes in the columns dealiasing empties
-    bool band_forced = false;  // and the state may hold their trace
+    bool band_forced = false;  // and the state or AB4's history may hold their trace
     double2* dio2 = nullptr;   // the same for results (small grids)
     void* pin_io = nullptr;    // page-locked staging of both (small grids)
     double2* dio = nullptr;    // staging [nx][nyf] complex128

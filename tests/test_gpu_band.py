@@ -213,3 +213,27 @@ def test_forcing_set_before_the_reverse_sweep():
     assert rel_err(s.get_w_hat(), ref.get_w_hat()) <= 1e-12
     s.close()
     ref.close()
+
+
+def test_history_of_forced_steps_after_a_host_step():
+    """The host-resident step replaces the state and keeps AB4's history, whose
+    right-hand sides hold an earlier forcing of the emptied columns.  Reference:
+    the same calls with 1e-280 in an emptied column of the host's array, which
+    keeps those columns in use whatever the history holds."""
+    n, dt = 256, 1e-3
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, integrator=abi.AB4, dt=dt)
+    out = []
+    for trace in (0.0, 1e-280):
+        s = Solver(p)
+        s.set_w_hat(_state(n, "narrow"))
+        s.set_forcing_modes([3 * (n // 2 + 1) + n // 2 - 9], [30.0 * n])
+        s.step_n(5, dt)
+        s.set_forcing_modes([], [])
+        w = _state(n, "narrow", seed=5)
+        w[7, n // 2 - 4] = trace
+        s.rk4_step_host(w, dt)
+        s.ab4_step(dt, 6)
+        out.append(s.get_w_hat())
+        s.close()
+    assert np.abs(out[1][3, n // 2 - 9]) > 0
+    assert rel_err(out[0], out[1]) <= 1e-12
