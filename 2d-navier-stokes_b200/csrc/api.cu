@@ -88,6 +88,7 @@ void fill_common(ns2d_handle* h, ColArgs<Real>& a, int branch) {
     a.norm2 = (Real)std::pow(norm_fac, 2.0);
     a.inv_nxny = norm_fac;
     a.status = h->dstatus;
+    a.stop = h->dstatus;
     a.final_tail = 1;
     a.force_field = h->ffield_on ? (const C*)h->ffield : nullptr;
     const int tc = engine_ops<Real>(h->nx)->tc;  // the stage pass's width divides it
@@ -111,7 +112,7 @@ RowArgs<Real> row_args(ns2d_handle* h) {
     r.nrows = h->nx;
     r.kc = kept_columns(h->nx, h->p.dealias, h->p.dealias_edge);
     r.band = h->dband;
-    r.status = h->dstatus;
+    r.stop = h->dstatus;
     return r;
 }
 
@@ -216,9 +217,10 @@ void launch_col(ns2d_handle* h, int mode, const ColArgs<Real>& a, int scheme = S
 // Row pass of stage `stage` (1..4); with a capture target set, the stage's real
 // fields go to planes 2(stage-1) and 2(stage-1)+1 of it.
 template <typename Real>
-void launch_row(ns2d_handle* h, int stage = 0, bool use_band = true) {
+void launch_row(ns2d_handle* h, int stage = 0, bool in_step = true, bool use_band = true) {
     TimedLaunch t(h, 3);
     RowArgs<Real> r = row_args<Real>(h);
+    if (!in_step) r.stop = nullptr;
     if (!use_band) r.band = nullptr;
     if (h->cap_step && stage >= 1) {
         const size_t plane = (size_t)h->nx * h->ny;
@@ -550,6 +552,7 @@ ns2d_status rhs_impl(ns2d_handle* h, const void* src, bool src_is_state) {
         ResArgs<Real> r;
         fill_resident<Real>(h, r, 4);
         r.src = (const C*)src;
+        r.status = nullptr;
         r.rhs = (C*)h->rhsbuf;
         r.nsteps = 1;
         r.conj_quirk = (quirk(h, NS2D_QUIRK_CONJ_STATE) || src_is_state) ? 1 : 0;
@@ -562,10 +565,12 @@ ns2d_status rhs_impl(ns2d_handle* h, const void* src, bool src_is_state) {
     ColArgs<Real> a;
     fill_common<Real>(h, a, 4);
     a.src = (const C*)src;
+    a.stop = nullptr;
     if (!src_is_state) a.band = nullptr;
     launch_col<Real>(h, COL_P1, a);
-    launch_row<Real>(h, 0, src_is_state);
+    launch_row<Real>(h, 0, false, src_is_state);
     fill_common<Real>(h, a, 4);
+    a.stop = nullptr;
     a.src = (const C*)h->nl;
     a.rhs_store = (C*)h->rhsbuf;
     a.conj_mode = (quirk(h, NS2D_QUIRK_CONJ_STATE) || src_is_state) ? 1 : 0;
@@ -1194,6 +1199,7 @@ ns2d_status resident_rhs_host(ns2d_handle* h, const double* in, double* out) {
     fill_resident<Real>(h, r, 4);
     r.src = (const Cplx<Real>*)h->state;
     r.src64 = in ? h->dio : nullptr;
+    r.status = nullptr;
     r.out64 = h->dio2;
     r.rhs = nullptr;
     r.nsteps = 1;

@@ -293,7 +293,7 @@ ns2d_status create_t(ns2d_ensemble* e) {
         mb.row.nrows = n;
         mb.row.kc = a.kc;
         mb.row.band = a.band;
-        mb.row.status = nullptr;
+        mb.row.stop = nullptr;
         mb.col0[0] = (C*)c0[0];
         mb.col0[1] = (C*)c0[1];
         mb.n = n;

@@ -131,7 +131,9 @@ struct ColArgs {
     int final_tail;      // COL_FINAL: 1 = SystemCheck bound over ntiles tiles, 0 = non-finite check only
     int phase_only;      // COL_FINAL: rescale each updated mode k != 0 to the amplitude it had before
     int ntiles;          // number of column tiles of this field
-    int* status;         // [0] status bits (kernels return early when set), [1] completed steps
+    int* status;         // [0] status bits, [1] completed steps
+    const int* stop;     // a set word ends the pass before it begins: status[0] in steps; null for an
+                         // evaluation by itself, which owes its caller a result whatever came before
 };
 
 // Whether the evaluation's input is known to be zero in the columns ky >= kc
@@ -993,7 +995,7 @@ constexpr bool pass_pdl(int n) { return n <= 512; }
 template <typename Real, int N, int TC, int MODE, int SCH>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_kernel(ColArgs<Real> a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    col_body<Real, N, TC, MODE, SCH, true, false, false, pass_pdl(N)>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, smraw);
+    col_body<Real, N, TC, MODE, SCH, true, false, false, pass_pdl(N)>(a, [&] { return block_begin(a.stop, a.band); }, blockIdx.x, smraw);
 }
 
 // Column pass with TMA tile loads and stores, without the rarely used parts (see
@@ -1003,7 +1005,7 @@ template <typename Real, int N, int TC, int MODE, int SCH>
 __global__ void __launch_bounds__(Plan<N>::T * TC) col_tma_kernel(ColArgs<Real> a, const __grid_constant__ ColMaps maps) {
     extern __shared__ __align__(16) unsigned char smraw[];
     unsigned char* sm = smraw + ((1024u - ((unsigned)__cvta_generic_to_shared(smraw) & 1023u)) & 1023u);
-    col_body<Real, N, TC, MODE, SCH, false, true, true, pass_pdl(N)>(a, [&] { return block_begin(a.status, a.band); }, blockIdx.x, sm, &maps);
+    col_body<Real, N, TC, MODE, SCH, false, true, true, pass_pdl(N)>(a, [&] { return block_begin(a.stop, a.band); }, blockIdx.x, sm, &maps);
 }
 
 // Whether a column pass can run without its GEN parts.
@@ -1025,7 +1027,7 @@ struct RowArgs {
     int nrows;
     int kc;           // columns of the product that survive dealiasing (only they are stored)
     const int* band;  // see band_narrow
-    int* status;
+    const int* stop;  // as ColArgs
     C* cap_uv;    // optional capture of the real fields: (u, v) and (w_x, w_y) as
     C* cap_w;     // complex pairs, [x][y] (adjoint stage recomputation); null = off
 };
@@ -1209,7 +1211,7 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) row_kernel(RowArgs<Rea
         pdl_launch();
         pdl_wait();
     }
-    const BlockBegin b = block_begin(a.status, a.band);
+    const BlockBegin b = block_begin(a.stop, a.band);
     if (b.exit) return;
     row_body<Real, N, PAIRS, CAP>(a, b.narrow, blockIdx.x, smraw);
 }

@@ -158,7 +158,7 @@ extern "C" ns2d_status ns2d_nonlinear_rhs_noalloc(const ns2d_params* p, const do
     r.ldc = nyf;
     r.nrows = n;
     r.kc = a.kc;
-    r.status = nullptr;
+    r.stop = nullptr;
     ops->row(r, st);
 
     a.src = nl;

@@ -71,7 +71,7 @@ struct ResArgs {
     Real norm2;
     double dt, inv_nxny;
     LinOp lin;
-    int* status;
+    int* status;           // as ColArgs; a set word ends the launch before its first step.  RES_RHS: null
 };
 
 // Cluster and block shapes.  CL blocks of NT threads; a unit is one transform by
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
     // Load the block's columns.  A set status word (an earlier step's failed
     // SystemCheck) ends the launch, as it does every pass launch; it is read
     // before the cluster's first barrier, so every block sees the same value.
-    const int status0 = a.status ? *(volatile const int*)a.status : 0;
+    const int status0 = !rhs_only && a.status ? *(volatile const int*)a.status : 0;
     if (threadIdx.x < CL) s_stop[threadIdx.x] = 0;
     bool wide = a.wide != 0;
     for (int q = threadIdx.x; q < L::SLOTS * N; q += NT) {
@@ -235,11 +235,11 @@ __global__ void __launch_bounds__(ResShape<N>::NT) resident_kernel(const __grid_
             if (a.out64) a.out64[(size_t)i * a.nyf + ky] = make_double2((double)w.x, (double)w.y);
         }
     };
-    if (status0) {
-        if constexpr (!rhs_only) {
+    if constexpr (!rhs_only) {
+        if (status0) {
             if (a.src64) put_state(L::SLOTS);
+            return;
         }
-        return;
     }
     if (threadIdx.x < CL) cluster_store(cluster_addr(smem_addr(&s_wide[rank]), threadIdx.x), wide ? 1 : 0);
     cluster_sync<CL>();

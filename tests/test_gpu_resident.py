@@ -98,3 +98,22 @@ def test_blowup_stops_the_launch():
     s.set_w_hat(_state(n, False, 3))
     s.step_n(3, 1e-3)
     assert np.all(np.isfinite(s.get_w_hat()))
+
+
+@pytest.mark.parametrize("n", [64, 256])
+def test_rhs_after_a_blowup(n):
+    """The RHS of a given field does not depend on the handle's state: after a
+    failed step it is still that of a new handle."""
+    p = abi.default_params(nx=n, ny=n, nu=1e-3)
+    w = initial.decaying(n, seed=3, k0=n / 16.0, dealias="2/3")
+    fresh, s = Solver(p), Solver(p)
+    other = initial.decaying(n, seed=4, k0=n / 16.0, dealias="2/3")
+    s.nonlinear_rhs(other)
+    s.rk4_step_host(other, 1e-3)
+    bad = w.copy()
+    bad[2, 2] = np.nan
+    s.set_w_hat(bad)
+    with pytest.raises(Exception, match="BLOWUP"):
+        s.step_n(3, 1e-3)
+    assert np.array_equal(s.nonlinear_rhs(w), fresh.nonlinear_rhs(w))
+    assert not np.all(np.isfinite(s.nonlinear_rhs()))  # the failed state's own
