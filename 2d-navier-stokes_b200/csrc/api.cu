@@ -1160,29 +1160,32 @@ ns2d_status state_to_host(ns2d_handle* h, const void* src, double* host, bool wa
 // memory, and the resident kernel reads and writes that layout: at these sizes a
 // strided or pageable copy costs more than the kernel (64^2 FP64, page-locked
 // arrays: RHS call 66 -> 39 us, host-resident step 93 -> 47).
-bool is_pinned(const void* p) {
+// Page-locked memory, and anything else that CUDA knows (managed or device memory
+// in the place of a host array), is left to the driver; only pageable memory, which
+// the CPU can read, goes through the handle's buffer.
+bool known_to_cuda(const void* p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return at.type == cudaMemoryTypeHost;
+    return at.type != cudaMemoryTypeUnregistered;
 }
 size_t spec_bytes(const ns2d_handle* h) { return sizeof(double2) * (size_t)h->nx * h->nyf; }
 ns2d_status upload_spec(ns2d_handle* h, const double* host) {
     const void* from = host;
-    if (!is_pinned(host)) {
+    if (!known_to_cuda(host)) {
         std::memcpy(h->pin_io, host, spec_bytes(h));
         from = h->pin_io;
     }
-    CK(h, cudaMemcpyAsync(h->dio, from, spec_bytes(h), cudaMemcpyHostToDevice, h->stream));
+    CK(h, cudaMemcpyAsync(h->dio, from, spec_bytes(h), cudaMemcpyDefault, h->stream));
     return NS2D_OK;
 }
 // Queues the copy of h->dio2; finish_spec completes it after a wait.
 ns2d_status download_spec(ns2d_handle* h, double* host, bool* direct) {
-    *direct = is_pinned(host);
+    *direct = known_to_cuda(host);
     CK(h, cudaMemcpyAsync(*direct ? (void*)host : (void*)((char*)h->pin_io + spec_bytes(h)), h->dio2, spec_bytes(h),
-                          cudaMemcpyDeviceToHost, h->stream));
+                          cudaMemcpyDefault, h->stream));
     return NS2D_OK;
 }
 void finish_spec(ns2d_handle* h, double* host, bool direct) {

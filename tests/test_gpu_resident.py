@@ -117,3 +117,25 @@ def test_rhs_after_a_blowup(n):
         s.step_n(3, 1e-3)
     assert np.array_equal(s.nonlinear_rhs(w), fresh.nonlinear_rhs(w))
     assert not np.all(np.isfinite(s.nonlinear_rhs()))  # the failed state's own
+
+
+@pytest.mark.parametrize("precision", [abi.FP64, abi.FP32])
+def test_device_memory_in_the_place_of_host_arrays(precision):
+    """Arrays that CUDA knows are copied by the driver, wherever they are."""
+    import ctypes as C
+
+    import torch
+
+    n = 64
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, precision=precision)
+    w = initial.decaying(n, seed=3, k0=4.0, dealias="2/3")
+    s = Solver(p)
+    d_in = torch.from_numpy(w.view(np.float64).copy()).cuda()
+    d_out = torch.zeros_like(d_in)
+    ptr = [C.cast(t.data_ptr(), C.POINTER(C.c_double)) for t in (d_in, d_out)]
+    torch.cuda.synchronize()
+    s._ck(s.L.ns2d_nonlinear_rhs(s.h, ptr[0], ptr[1]))
+    assert np.array_equal(d_out.cpu().numpy().view(np.complex128), s.nonlinear_rhs(w))
+    s._ck(s.L.ns2d_rk4_step_host(s.h, ptr[0], 1e-3))
+    s.rk4_step_host(w, 1e-3)
+    assert np.array_equal(d_in.cpu().numpy().view(np.complex128), w)
