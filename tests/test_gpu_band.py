@@ -237,3 +237,22 @@ def test_history_of_forced_steps_after_a_host_step():
         s.close()
     assert np.abs(out[1][3, n // 2 - 9]) > 0
     assert rel_err(out[0], out[1]) <= 1e-12
+
+
+@pytest.mark.parametrize("integ", [abi.RK4CN, abi.RK4])
+@pytest.mark.parametrize("steps", [64, 83])
+def test_long_runs_equal_single_steps(steps, integ):
+    """Long runs replay graphs of several steps and end with single ones."""
+    n, dt = 256, 1e-4
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, integrator=integ)
+    w0 = initial.decaying(n, seed=12, k0=n / 16.0, dealias="2/3")
+    a, b = Solver(p), Solver(p)
+    for s in (a, b):
+        s.set_w_hat(w0)
+    for run in (steps, 21, 9):
+        a.step_n(run, dt)
+        for _ in range(run):
+            b.rk4_step(dt)
+        assert np.array_equal(a.get_w_hat(), b.get_w_hat()), run
+    a.close()
+    b.close()
