@@ -46,7 +46,7 @@ struct ns2d_handle {
     bool ffield_band = false;  // the listed forcing has modes in the columns dealiasing empties
     bool band_forced = false;  // and the state or AB4's history may hold their trace
     double2* dio2 = nullptr;   // the same for results (small grids)
-    void* pin_io = nullptr;    // page-locked staging of both (small grids)
+    void* pin_io = nullptr;    // page-locked staging of both (small grids), in the block of pin
     double2* dio = nullptr;    // staging [nx][nyf] complex128
     double* ddiag = nullptr;   // measurables: DG_N totals + 8 * n_spect spectra
     double* dpart = nullptr;   // per-block partial bounds of the final column pass
