@@ -24,7 +24,8 @@ struct ns2d_handle {
     int64_t launches = 0;
     size_t elem = 0;         // bytes per complex element
     size_t field_bytes = 0;  // nx * ldc * elem
-    // device buffers
+    // device buffers, all but those of later calls (dp, dp_last, lint, the listed forcing's) in one allocation
+    void* slab = nullptr;
     void* state = nullptr;
     void* acc = nullptr;
     void* nl = nullptr;
