@@ -188,8 +188,9 @@ inline bool with_size(int n, F&& f) {
     }
 }
 
-// The launch functions of one grid size in one precision, compiled in
-// engine_f32.cu and engine_f64.cu.
+// The launch functions of one grid size in one precision.  Each size and precision
+// is a module of its own (engine_size.cu): the first handle of a program loads the
+// kernels of its size and no others.
 template <typename Real>
 struct EngineOps {
     int tc, tc_stage;  // column-tile widths: of the passes, of the common step's stage pass
@@ -201,8 +202,14 @@ struct EngineOps {
                 int ldc, const typename Cx<Real>::T* tw, cudaStream_t s);
     void (*row_c2r)(int op, const RowC2RArgs<Real>& a, cudaStream_t s);
 };
+template <typename Real, int N>
+const EngineOps<Real>* engine_ops_of();
 // Null for a size that has none.
 template <typename Real>
-const EngineOps<Real>* engine_ops(int n);
+inline const EngineOps<Real>* engine_ops(int n) {
+    const EngineOps<Real>* ops = nullptr;
+    with_size<Real>(n, [&](auto L) { ops = engine_ops_of<Real, decltype(L)::SIZE>(); });
+    return ops;
+}
 
 }  // namespace ns2d
