@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(Plan<N>::T * 2 * PAIRS) adj_row_kernel(AdjRowA
     const int t = threadIdx.x % T;
     const int x = blockIdx.x * TC + g;
     C* region = reinterpret_cast<C*>(smraw) + (size_t)g * RS::TEAM;
-    const auto seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N, row_extra(N)>(a.tw, t);
     const TeamPolicy<N, C> pol{region, 1 + g};
     // mu = c2r(mu_x) along y: Hermitian extension, real parts at ky = 0 and N/2
     C z[1][E];

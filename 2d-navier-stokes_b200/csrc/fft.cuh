@@ -179,33 +179,43 @@ struct SmemLayout {
 // stage's Ns, so a thread's middle-stage butterflies all share k = t mod Ns and
 // its twiddles are powers of one value; the last stage's twiddles are powers of
 // exp(-2 pi i t / N).  The seeds are loaded once per kernel and the powers
-// w^r (r < R) are formed by a multiplication tree of depth log2 R, so the
-// transform issues no table loads of its own.
-template <typename C>
+// w^r (r < R) are formed by a multiplication tree, so the transform issues no
+// table loads of its own.  A power carries r times the rounding of its seed, most of
+// a transform's error; with EXTRA the fourth power (the second of radix 4) comes from
+// the table too (an RHS at 1024^2 errs by 0.84e-15 with it in all transforms, by
+// 1.10e-15 without).  It costs the column passes nothing; the row passes of the
+// radix-16 plans, whose registers are full, go without (row_extra).
+template <typename C, bool EXTRA = true>
 struct TwSeed {
     C mid;   // exp(-2 pi i (t mod Ns1) (N / (Ns1 R1)) / N)
     C last;  // exp(-2 pi i t / N)
 };
+template <typename C>
+struct TwSeed<C, true> {
+    C mid, last;
+    C lastk;  // last^extra_power(last radix)
+};
+constexpr int extra_power(int radix) { return radix > 4 ? 4 : 2; }
 
-template <int N, typename C>
-__device__ __forceinline__ TwSeed<C> twiddle_seeds(const C* __restrict__ tw, int t) {
-    using P = Plan<N>;
-    TwSeed<C> s;
-    constexpr int NS1 = P::R0;
-    s.mid = __ldg(tw + (t % NS1) * (N / (NS1 * P::R1)));
-    s.last = __ldg(tw + t);
-    return s;
-}
+// Whether the row passes of an N grid load the extra power: at 1024 it takes 30
+// registers and the third block off an SM in FP64 (17.8 -> 19.5 us), and its reads, a
+// sector per lane, show where the rows are short (2048 FP32 32.1 -> 33.2 us).
+constexpr bool row_extra(int n) { return n <= 512; }
 
 // Seeds of the N-point plan read from the table of a multiple of N points:
 // tw[stride * j] = exp(-2 pi i j / N).
-template <int N, typename C>
-__device__ __forceinline__ TwSeed<C> twiddle_seeds_strided(const C* __restrict__ tw, int t, int stride) {
+template <int N, bool EXTRA = true, typename C>
+__device__ __forceinline__ TwSeed<C, EXTRA> twiddle_seeds(const C* __restrict__ tw, int t, int stride = 1) {
     using P = Plan<N>;
-    TwSeed<C> s;
+    TwSeed<C, EXTRA> s;
     constexpr int NS1 = P::R0;
     s.mid = __ldg(tw + stride * ((t % NS1) * (N / (NS1 * P::R1))));
     s.last = __ldg(tw + stride * t);
+    if constexpr (EXTRA) {
+        constexpr int K = extra_power(P::R0);
+        static_assert(K * P::T <= N, "the powers are in the table");
+        s.lastk = __ldg(tw + stride * (K * t));
+    }
     return s;
 }
 
@@ -216,6 +226,19 @@ __device__ __forceinline__ void tw_powers(C w, C* out) {
     out[1] = w;
 #pragma unroll
     for (int r = 2; r < R; ++r) out[r] = (r & 1) ? cmul(out[r - 1], w) : cmul(out[r / 2], out[r / 2]);
+}
+// The same for the last stage.
+template <int R, int SIGN, typename C, bool EXTRA>
+__device__ __forceinline__ void last_powers(const TwSeed<C, EXTRA>& seed, C* out) {
+    if constexpr (EXTRA) {
+        constexpr int K = extra_power(R);
+        tw_powers<K, SIGN>(seed.last, out);
+        out[K] = SIGN > 0 ? cconj(seed.lastk) : seed.lastk;
+#pragma unroll
+        for (int r = K + 1; r < R; ++r) out[r] = r % K == 0 ? cmul(out[r - K], out[K]) : cmul(out[r / K * K], out[r % K]);
+    } else {
+        tw_powers<R, SIGN>(seed.last, out);
+    }
 }
 
 // Middle stage: reads smem (pattern of the previous stage's writes), writes smem.
@@ -275,7 +298,7 @@ __device__ __forceinline__ void fft(C* v, C* sm, const TwSeed<C>& seed, int t, i
 #pragma unroll
     for (int r = 0; r < RL; ++r) v[r] = sm[L::slot(t + r * (N / RL), c)];
     C w[RL];
-    tw_powers<RL, SIGN>(seed.last, w);
+    last_powers<RL, SIGN>(seed, w);
 #pragma unroll
     for (int r = 1; r < RL; ++r) v[r] = cmul(v[r], w[r]);
     small_dft<RL, SIGN>(v);
@@ -353,8 +376,8 @@ struct TeamPolicy {
 // B transforms of length N in lockstep.  v[b][m] = x_b[t + T m] in and out.
 // The twiddle powers are shared by the B transforms; one barrier phase serves
 // all of them.
-template <int N, int SIGN, int B, typename C, typename Pol>
-__device__ __forceinline__ void fft_batched(C (&v)[B][N / Plan<N>::T], const Pol& pol, const TwSeed<C>& seed, int t) {
+template <int N, int SIGN, int B, typename C, typename Pol, bool EXTRA>
+__device__ __forceinline__ void fft_batched(C (&v)[B][N / Plan<N>::T], const Pol& pol, const TwSeed<C, EXTRA>& seed, int t) {
     using P = Plan<N>;
     constexpr int T = P::T;
     constexpr int E = N / T;
@@ -400,7 +423,7 @@ __device__ __forceinline__ void fft_batched(C (&v)[B][N / Plan<N>::T], const Pol
     constexpr int RL = (P::S == 3) ? P::R2 : P::R1;
     static_assert(RL == P::R0, "last radix must equal the first");
     C w[RL];
-    tw_powers<RL, SIGN>(seed.last, w);
+    last_powers<RL, SIGN>(seed, w);
 #pragma unroll
     for (int b = 0; b < B; ++b) {
 #pragma unroll

@@ -1069,7 +1069,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
     const int t = threadIdx.x % T;
     const int x = rblock * TC + g;
     C* region = reinterpret_cast<C*>(smraw) + (size_t)g * RS::TEAM;
-    const auto seed = twiddle_seeds<N>(a.tw, t);
+    const auto seed = twiddle_seeds<N, row_extra(N)>(a.tw, t);
     const TeamPolicy<N, C> pol{region, 1 + g};
 
     // Z1 = U + i V and Z2 = WX + i WY over the full y range; at DC and Nyquist
@@ -1143,7 +1143,7 @@ __device__ __forceinline__ void row_body(const RowArgs<Real>& a, bool narrow, in
 #pragma unroll
         for (int m = 0; m < EH; ++m) z[0][m] = zin[t + T * m];
         const TeamPolicy<NH, C> polh{region, 1 + g};
-        fft_batched<NH, -1, 1>(z, polh, twiddle_seeds_strided<NH>(a.tw, t, 2), t);
+        fft_batched<NH, -1, 1>(z, polh, twiddle_seeds<NH, row_extra(N)>(a.tw, t, 2), t);
 #pragma unroll
         for (int m = 0; m < EH; ++m) region[TLH::template slot<C>(t + T * m)] = z[0][m];
         polh.sync();
