@@ -135,23 +135,24 @@ __global__ void __launch_bounds__(Plan<N>::T * TC * adj_groups<N>()) adj_col_ker
                 v[1][m] = Ps[2 * pair + 1][q];
             }
             fft_batched<N, -1, 2>(v, pol, seed, t);
-            // With q = kx + i ky the four terms conj(m) P are
-            //   pair 0: (conj(q) Q+ - q Q-) / (2 k^2),  pair 1: -i (conj(q) R+ + q R-) / 2
+            // The four terms conj(m) P, of Q+- = P0 +- i P1 and R+- = P2 +- i P3:
+            //   pair 0: (kx (Q+ - Q-) - i ky (Q+ + Q-)) / (2 k^2)
+            //   pair 1: (-i kx (R+ + R-) - ky (R+ - R-)) / 2
+            // The factors with 1/k^2 are formed in FP64 and rounded once.
 #pragma unroll
             for (int m = 0; m < E; ++m) {
                 const Real kx = kx_of<Real, N, T>(m, t, tr);
-                const C p = v[0][m], n = v[1][m];
-                const C cp = cmake<C>(kx * p.x + kyr * p.y, kx * p.y - kyr * p.x);
-                const C qn = cmake<C>(kx * n.x - kyr * n.y, kx * n.y + kyr * n.x);
+                const C d = csub(v[0][m], v[1][m]), e = cadd(v[0][m], v[1][m]);
                 C L;
                 if (m == 0 && t == 0 && ky == 0) {
                     L = cmake<C>(0, 0);
                 } else if (pair == 0) {
-                    const Real s = (Real)0.5 * inv_k2<Real>(kx * kx + kyr * kyr);
-                    L = cscale(csub(cp, qn), s);
+                    const double kd = (double)kx, h = 0.5 * inv_k2<double>(kd * kd + (double)ky * (double)ky);
+                    const Real sx = (Real)(kd * h), sy = (Real)((double)ky * h);
+                    L = cmake<C>(sx * d.x + sy * e.y, sx * d.y - sy * e.x);
                 } else {
-                    const C sum = cadd(cp, qn);
-                    L = cmake<C>((Real)0.5 * sum.y, (Real)-0.5 * sum.x);
+                    const Real sx = (Real)0.5 * kx, sy = (Real)0.5 * kyr;
+                    L = cmake<C>(sx * e.y - sy * d.x, -(sx * e.x) - sy * d.y);
                 }
                 C* const to = Lbuf + (G > 1 ? g * N * TC : 0) + (t + T * m) * TC + c;
                 if (G == 1 && pair > 0) L = cadd(*to, L);

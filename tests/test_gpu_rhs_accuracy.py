@@ -1,4 +1,4 @@
-"""Accuracy of one FP32 evaluation of the nonlinear term."""
+"""Accuracy of one FP32 evaluation of the nonlinear term, and of its adjoint."""
 import numpy as np
 import pytest
 
@@ -22,4 +22,24 @@ def test_fp32_rhs_error_against_fp64(n, k0, seeds, bound):
         err.append(np.linalg.norm(a.nonlinear_rhs(w) - want) / np.linalg.norm(want))
     a.close()
     b.close()
+    assert np.mean(err) <= bound
+
+
+@pytest.mark.parametrize("n,k0,bound", [(32, 2.0, 5.85e-8), (64, 4.0, 6.1e-8), (256, 6.0, 1.18e-7)])
+def test_fp32_gradient_error_against_fp64(n, k0, bound):
+    """The same for a reverse sweep over one step whose nonlinear part is as large
+    as the linear one: the bounds are the errors with every multiplier (kx/k^2,
+    ky/k^2) formed in FP64 and rounded once, term by term."""
+    err = []
+    for seed in range(6):
+        w, lam = (initial.decaying(n, seed=s0 + seed, k0=k, dealias="2/3").astype(np.complex64).astype(np.complex128)
+                  for s0, k in ((50, k0), (90, n / 8.0)))
+        g = []
+        for q in (abi.FP32, abi.FP64):
+            s = Solver(abi.default_params(nx=n, ny=n, nu=1e-3, quirks=0, precision=q))
+            s.set_w_hat(w)
+            s.adjoint_record(1, 0.02, 1)
+            g.append(s.adjoint_backward(lam))
+            s.close()
+        err.append(np.linalg.norm(g[0] - g[1]) / np.linalg.norm(g[1]))
     assert np.mean(err) <= bound
