@@ -111,18 +111,25 @@ __global__ void __launch_bounds__(Plan<N>::T * TC * adj_groups<N>()) adj_col_ker
     const IlvGroupPolicy<N, TC, C> pol{sm + 2 * g * SM::FFT, c, 1 + g};
     const Real tr = (Real)t, kyr = (Real)ky;
 
-    // operands of the epilogue, on their way under the transforms
+    // Operands of the epilogue: on their way under the transforms where a thread
+    // holds few elements; with sixteen (1024 and 2048) they would spill there, 600
+    // bytes a thread in FP64, and are read after (a reverse step at 1024^2 FP64 414 us
+    // against 440, at 2048^2 1,782 against 1,930).
+    constexpr bool AHEAD = EG <= 8;
     C lx[EG], lp[MODE == ADJ_END ? 1 : EG];
     double2 f[MODE == ADJ_END ? 1 : EG];
+    const auto operands = [&] {
 #pragma unroll
-    for (int m = 0; m < EG; ++m) {
-        const size_t q = (size_t)(t + T * (m + g * EG)) * ldc + kyc;
-        if constexpr (MODE != ADJ_START) lx[m] = a.lam_x[q];
-        if constexpr (MODE != ADJ_END) {
-            lp[m] = a.lam_p[q];
-            f[m] = a.cn[q];
+        for (int m = 0; m < EG; ++m) {
+            const size_t q = (size_t)(t + T * (m + g * EG)) * ldc + kyc;
+            if constexpr (MODE != ADJ_START) lx[m] = a.lam_x[q];
+            if constexpr (MODE != ADJ_END) {
+                lp[m] = a.lam_p[q];
+                f[m] = a.cn[q];
+            }
         }
-    }
+    };
+    if constexpr (AHEAD) operands();
     if constexpr (MODE != ADJ_START) {
         const C* const Ps[4] = {a.P0, a.P1, a.P2, a.P3};
 #pragma unroll 1
@@ -161,6 +168,7 @@ __global__ void __launch_bounds__(Plan<N>::T * TC * adj_groups<N>()) adj_col_ker
         }
         if constexpr (G > 1) __syncthreads();
     }
+    if constexpr (!AHEAD) operands();
 #pragma unroll
     for (int m = 0; m < EG; ++m) {
         const int i = t + T * (m + g * EG);
