@@ -74,15 +74,22 @@ __device__ __forceinline__ void ens_apply_stage(ColArgs<Real>& a, const EnsMembe
     }
 }
 
-// Resident blocks per SM the ensemble kernels are compiled for, now that every
-// size's transforms hold eight elements a thread: in FP32 three 256-thread (six
-// 128-thread) blocks, 85 registers a thread (a step of the 64-member ensemble
-// 284 us; with the row layout before TeamLayout::slot's 16 292, two blocks 317,
-// four 314 with spills), in FP64 two of 256, 128 registers
-// (453 us; one 547, three 533).
-template <typename Real, int THREADS>
+// Resident blocks per SM the ensemble kernels are compiled for, with eight elements
+// of a transform a thread at every size.  FP32: three 256-thread (six 128-thread)
+// blocks, 80 registers a thread; FP64: two, 128 registers.  The row kernels fit
+// (80 and 128 registers); the column kernels spill, the common stage pass 290 bytes a
+// thread in FP32 and 660 in FP64, the general forms up to 1,950, and are faster all
+// the same.  A step of 64 members (32 x 128^2, 24 x 256^2, 8 x 512^2), us,
+// this bound / two blocks in FP32 and one in FP64: common step FP32 284 / 317, FP64
+// 453 / 547 (both tuned); untuned, general kernels only: explicit RK4 362 / 373 and
+// 621 / 650, Hou-Li 487 / 471 and 761 / 832, phase-only 366 / 364 and 621 / 615,
+// explicit with Hou-Li 496 / 504 and 781 / 907.  STAGE, the per-stage launch: in FP32
+// two blocks (common step 434 against 467 with three, explicit 470 against 491, Hou-Li
+// 577 against 607), in FP64 two (645 against 794 with one, 678 against 841, 838
+// against 1,081).
+template <typename Real, int THREADS, bool STAGE = false>
 struct EnsMinBlocks {
-    static constexpr int value = sizeof(Real) == 4 ? 768 / THREADS : 512 / THREADS;
+    static constexpr int value = sizeof(Real) == 4 && !STAGE ? 768 / THREADS : 512 / THREADS;
 };
 
 // SCH, GEN: as col_body.  TMA: the tiles move by TMA copies through maps[2 m + v], the
@@ -183,7 +190,7 @@ __device__ __forceinline__ bool ens_wait_count(const int* cnt, int need, int* st
 }
 
 template <typename Real, int MODE, int THREADS, int SCH>
-__global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS>::value))
+__global__ void __launch_bounds__(THREADS, (EnsMinBlocks<Real, THREADS, true>::value))
     ens_stage_kernel(const EnsMember<Real>* __restrict__ members, const EnsTask* __restrict__ tasks, int ntasks,
                      EnsStage st, EnsSync sy) {
     extern __shared__ __align__(16) unsigned char smraw[];
