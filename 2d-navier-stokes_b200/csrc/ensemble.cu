@@ -659,12 +659,15 @@ ns2d_status meas_t(ns2d_ensemble* e, int m, ns2d_measures* out) {
     return NS2D_OK;
 }
 
+// Device ms of a step, in the form that a run of steps takes.
 double time_steps(ns2d_ensemble* e, double dt, int steps) {
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
+    const bool run = ens_can_run(e);
+    if (run) EDISPATCH(e, first_pass, e);
     cudaEventRecord(a, e->stream);
-    for (int k = 0; k < steps; ++k) EDISPATCH(e, step_t, e, dt);
+    for (int k = 0; k < steps; ++k) EDISPATCH(e, step_t, e, dt, !run, run);
     cudaEventRecord(b, e->stream);
     cudaEventSynchronize(b);
     float ms = 0.f;
@@ -813,7 +816,7 @@ ns2d_status ns2d_ensemble_tune(ns2d_ensemble* e, double dt, int32_t* col_grid, i
     // launches of a step), the block size -- which sets the tile shape: ky
     // columns per column tile and row pairs per row block of every member --
     // and the persistent grid as a multiple of the SM count (1..8 blocks per
-    // SM, capped by the item count), chosen by timing full steps.  Steps taken
+    // SM, capped by the item count), chosen by timing steps of a run.  Steps taken
     // here advance the members; callers re-set their states.
     const int saved_hyper = e->hyper_flag;
     e->fused = false;

@@ -153,3 +153,18 @@ def test_one_launch_per_stage_equals_nine_launches(precision):
         assert rel_err(e.get_w_hat(m), ref.get_w_hat(m)) <= tol, m
     e.close()
     ref.close()
+
+
+def test_tuner_times_steps_of_a_run():
+    """A step of a run is eight launches, after one that starts the run; the
+    tuner's 25 timings of three steps each take that form (its per-stage timings
+    add four launches a step, so multiples of twelve)."""
+    sizes = [64, 128, 64]
+    e = Ensemble(abi.default_params(nu=1e-3, dt=1e-3), sizes)
+    for m, n in enumerate(sizes):
+        e.set_w_hat(m, initial.decaying(n, m, k0=6.0, dealias="2/3"))
+    before = e.launch_count
+    e.tune(1e-3)
+    rest = e.launch_count - before - (len(sizes) + 9) - 25 * (1 + 3 * 8)
+    assert rest > 0 and rest % 12 == 0
+    e.close()
