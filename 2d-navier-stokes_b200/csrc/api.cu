@@ -584,6 +584,23 @@ ns2d_status rhs_impl(ns2d_handle* h, const void* src, bool src_is_state) {
     return NS2D_OK;
 }
 
+// The Dormand-Prince arrays, on first use, in one allocation.
+ns2d_status ensure_dp(ns2d_handle* h) {
+    if (h->dp_kptr) return NS2D_OK;
+    constexpr int n = (int)(sizeof(h->dp) / sizeof(h->dp[0]));
+    if (!h->dp[0]) {
+        void* base = nullptr;
+        CK(h, cudaMalloc(&base, n * h->field_bytes));
+        for (int k = 0; k < n; ++k) h->dp[k] = (char*)base + k * h->field_bytes;
+    }
+    CK(h, cudaMemsetAsync(h->dp[0], 0, n * h->field_bytes, h->stream));
+    const void** kptr = nullptr;
+    CK(h, cudaMalloc((void**)&kptr, sizeof(void*) * 7));
+    h->dp_kptr = kptr;
+    CK(h, cudaMemcpy((void*)kptr, h->dp, sizeof(void*) * 7, cudaMemcpyHostToDevice));
+    return NS2D_OK;
+}
+
 // RK5DPStep (Solver/src/solver.c:360-570) as the reference intends it: seven
 // stages k_s = N(X_s) - D X_s with X_s = y0 + dt sum_r a_sr k_r (Butcher table
 // of solver.c:33-42), y5 into the state, and the RMS of the embedded error
@@ -600,14 +617,7 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
         {19372.0 / 6561.0, -25360.0 / 2187.0, 64448.0 / 6561.0, -212.0 / 729.0, 0, 0},
         {9017.0 / 3168.0, -355.0 / 33.0, 46732.0 / 5247.0, 49.0 / 176.0, -5103.0 / 18656.0, 0},
         {35.0 / 384.0, 0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0}};
-    if (!h->dp[0]) {
-        for (void*& p : h->dp) {
-            CK(h, cudaMalloc(&p, h->field_bytes));
-            CK(h, cudaMemsetAsync(p, 0, h->field_bytes, h->stream));
-        }
-        CK(h, cudaMalloc((void**)&h->dp_kptr, sizeof(void*) * 7));
-        CK(h, cudaMemcpy((void*)h->dp_kptr, h->dp, sizeof(void*) * 7, cudaMemcpyHostToDevice));
-    }
+    if (ns2d_status sd = ensure_dp(h)) return sd;
     if (ns2d_status sb = ensure_band(h)) return sb;
     compute_forcing(h, dt);
     const bool euler = h->p.system == NS2D_EULER;
@@ -617,7 +627,7 @@ ns2d_status dp5_step_impl(ns2d_handle* h, double dt, double* err) {
     }
     // Each stage's column pass forms its derivative k_s and, from the state (y0
     // until the end) and k_0..k_s, the next stage input with its derived spectra.
-    void* x = h->dp[8];
+    void* x = h->dp[7];
     ColArgs<Real> a;
     fill_common<Real>(h, a, branch);
     a.src = (const C*)h->state;
@@ -684,14 +694,7 @@ ns2d_status rk5dp_step_impl(ns2d_handle* h, double dt, int iters, double* err) {
         {19372.0 / 6561.0, -25360.0 / 2187.0, 64448.0 / 6561.0, -212.0 / 729.0, 0, 0},
         {9017.0 / 3168.0, -355.0 / 33.0, 46732.0 / 5247.0, 49.0 / 176.0, -5103.0 / 18656.0, 0},
         {35.0 / 384.0, 0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0}};
-    if (!h->dp[0]) {
-        for (void*& p : h->dp) {
-            CK(h, cudaMalloc(&p, h->field_bytes));
-            CK(h, cudaMemsetAsync(p, 0, h->field_bytes, h->stream));
-        }
-        CK(h, cudaMalloc((void**)&h->dp_kptr, sizeof(void*) * 7));
-        CK(h, cudaMemcpy((void*)h->dp_kptr, h->dp, sizeof(void*) * 7, cudaMemcpyHostToDevice));
-    }
+    if (ns2d_status sd = ensure_dp(h)) return sd;
     if (!h->dp_last) {
         CK(h, cudaMalloc(&h->dp_last, h->field_bytes));
         CK(h, cudaMemsetAsync(h->dp_last, 0, h->field_bytes, h->stream));
@@ -701,7 +704,7 @@ ns2d_status rk5dp_step_impl(ns2d_handle* h, double dt, int iters, double* err) {
     const bool euler = h->p.system == NS2D_EULER;
     const int branch = euler ? 4 : resolve_branch(h, false);
     const bool conj_quirk = quirk(h, NS2D_QUIRK_CONJ_STATE);
-    void* x = h->dp[8];
+    void* x = h->dp[7];
     for (int s = 0; s < 7; ++s) {
         const void* xs = h->state;
         if (s > 0) {
@@ -862,10 +865,8 @@ void fill_twiddles(std::vector<Cplx<Real>>& tw, int n) {
 }
 
 void free_all(ns2d_handle* h) {
-    void* ptrs[] = {h->slab, h->dp_last, h->lint};
+    void* ptrs[] = {h->slab, h->dp[0], h->dp_last, h->lint};
     for (void* p : ptrs)
-        if (p) cudaFree(p);
-    for (void* p : h->dp)
         if (p) cudaFree(p);
     void* fp[] = {h->ffield, h->fidx, h->fval};
     for (void* p : fp)

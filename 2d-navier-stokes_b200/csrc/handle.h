@@ -85,8 +85,8 @@ struct ns2d_handle {
     int32_t* fidx = nullptr;
     double2* fval = nullptr;
     int fcap = 0;
-    // Dormand-Prince stages k0..k6, y0 and the stage input (allocated on first use)
-    void* dp[9] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    // Dormand-Prince stages k0..k6 and the stage input (one allocation, on first use)
+    void* dp[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     const void** dp_kptr = nullptr;  // device array of the seven stage pointers
     // RK5DPStep as written: the state of the last error step (Int_data->w_hat_last,
     // zero until then) and the last error (Int_data->DP_err)
