@@ -427,8 +427,8 @@ ns2d_status rk4_step_impl(ns2d_handle* h, double dt, void* rk1_out, bool first =
 }
 
 // Steps per launch of the resident kernel: the launch and the load and store of
-// the state cost about one step, and a launch stays well under a millisecond or
-// two, so other work on the device gets its turn.
+// the state cost about one step, and a launch ends in 0.8 ms at 16^2 to 2.7 ms at
+// 128^2 FP64, so other work on the device gets its turn.
 constexpr int kResidentSteps = 128;
 
 // nsteps RK4 / RK4CN steps of a small grid in the resident kernel; rk1_out as in

@@ -28,8 +28,8 @@
 // path about 800 each, and the rest loads, twiddles and the remote stores; at
 // 128^2 FP64 arithmetic and remote-store issue add to it.  Measured per step
 // (RK4CN, 2/3, FP64 / FP32, us): 16^2 28.8 / 28.8 -> 6.5 / 5.3, 32^2 39.0 / 34.9 ->
-// 9.9 / 7.9, 64^2 45.3 / 41.1 -> 14.0 / 10.3, 128^2 53.4 / 44.6 -> 20.7 / 18.0 against
-// the pass launches replayed from a graph; explicit RK4 at 64^2 154 -> 13.9 (its
+// 9.9 / 8.0, 64^2 45.3 / 41.1 -> 13.8 / 10.2, 128^2 53.4 / 44.6 -> 20.6 / 17.2 against
+// the pass launches replayed from a graph; explicit RK4 at 64^2 154 -> 13.6 (its
 // passes never settled on a graph).
 //
 // Columns that the 2/3 rule empties (ky >= kc, k2 >= kmax_sqr for every kx) hold

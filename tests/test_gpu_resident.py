@@ -139,3 +139,21 @@ def test_device_memory_in_the_place_of_host_arrays(precision):
     s._ck(s.L.ns2d_rk4_step_host(s.h, ptr[0], 1e-3))
     s.rk4_step_host(w, 1e-3)
     assert np.array_equal(d_in.cpu().numpy().view(np.complex128), w)
+
+
+@pytest.mark.parametrize("integ", [abi.RK4CN, abi.RK4])
+@pytest.mark.parametrize("n", [16, 32, 64, 128])
+def test_passes_give_the_same_states(n, integ):
+    """Per-pass timing takes the pass kernels: the same bits, except at 64, whose
+    row pass transforms each row by itself in half the length."""
+    p = abi.default_params(nx=n, ny=n, nu=1e-3, integrator=integ)
+    w0 = _state(n, False, 8)
+    a, b = Solver(p), Solver(p)
+    b.set_kernel_timing(True)
+    for s in (a, b):
+        s.set_w_hat(w0)
+        s.step_n(5, 1e-3)
+    if n == 64:
+        assert rel_err(a.get_w_hat(), b.get_w_hat()) <= TOL[abi.FP64]
+    else:
+        assert np.array_equal(a.get_w_hat(), b.get_w_hat())
